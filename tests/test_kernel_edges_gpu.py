@@ -1,0 +1,74 @@
+"""Kernels at the sizes where their tiling can go wrong: edges of tiles, remainders, the smallest and largest of a rule's range."""
+import math
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from verl_b200.ops import native
+
+    return native.ops()
+
+
+def rel(a, b):
+    return float((a.double() - b.double()).norm() / b.double().norm().clamp_min(1e-30))
+
+
+# ------------------------------------------------------------------------------------------------ advantages
+@pytest.mark.parametrize("B,L", [(1, 1), (3, 17), (5, 128), (2, 1024), (2, 1025), (1300, 33), (7, 4099)])
+@pytest.mark.parametrize("gamma,lam", [(1.0, 0.95), (0.9, 0.0)])
+def test_gae_tiles(ops, B, L, gamma, lam):
+    from verl_b200.ops import functional as F
+
+    g = torch.Generator().manual_seed(B * 31 + L)
+    r, v = torch.randn(B, L, generator=g) * 0.1, torch.randn(B, L, generator=g)
+    m = (torch.rand(B, L, generator=g) > 0.3).float()
+    m[:, 0] = 1
+    adv, ret = F.gae_advantage(r.to(DEV), v.to(DEV), m.to(DEV), gamma, lam, whiten=False)
+    want, nextv, last = torch.zeros(B, L, dtype=torch.float64), torch.zeros(B, dtype=torch.float64), torch.zeros(B, dtype=torch.float64)
+    rd, vd = r.double(), v.double()
+    for t in reversed(range(L)):
+        step = rd[:, t] + gamma * nextv - vd[:, t] + gamma * lam * last
+        nextv = torch.where(m[:, t] > 0, vd[:, t], nextv)
+        last = torch.where(m[:, t] > 0, step, last)
+        want[:, t] = last
+    # 24 significant bits per step of a chain that forgets with gamma * lam: 1e-5 leaves room for some tens of roundings
+    assert rel(adv.cpu(), want) < 1e-5 and rel(ret.cpu(), want + vd) < 1e-5
+    white, _ = F.gae_advantage(r.to(DEV), v.to(DEV), m.to(DEV), gamma, lam, whiten=True)
+    md, n = m.double(), m.double().sum()
+    mean = (want * md).sum() / n
+    var = ((want - mean).square() * md).sum() / (n - 1).clamp(min=1)
+    if n > 1:
+        assert rel(white.cpu(), (want - mean) * torch.rsqrt(var + 1e-8)) < 2e-5
+    again, _ = F.gae_advantage(r.to(DEV), v.to(DEV), m.to(DEV), gamma, lam, whiten=True)
+    assert torch.equal(again, white)
+
+
+@pytest.mark.parametrize("B,L,dtype", [(1, 1, torch.int64), (6, 129, torch.int32), (1024, 7, torch.int64), (1025, 7, torch.int32), (1025, 7, torch.int64)])
+def test_group_advantage_rows(ops, B, L, dtype):
+    from verl_b200.ops import functional as F
+
+    g = torch.Generator().manual_seed(B)
+    groups = max(1, B // 5)
+    ids = torch.randint(groups, (B,), generator=g)
+    r, m = torch.rand(B, L, generator=g), (torch.rand(B, L, generator=g) > 0.2).float()
+    for by_std in (True, False):
+        adv, score = F.grpo_advantage(r.to(DEV), m.to(DEV), ids.to(DEV).to(dtype), groups, 1e-6, by_std)
+        s = r.double().sum(-1)
+        want = torch.zeros(B, dtype=torch.float64)
+        for k in range(groups):
+            sel = ids == k
+            if sel.sum() == 1:
+                want[sel] = s[sel] / (1 + 1e-6) if by_std else s[sel]
+            elif sel.any():
+                want[sel] = s[sel] - s[sel].mean()
+                if by_std:
+                    want[sel] /= s[sel].std() + 1e-6
+        # the sums of squares of the atomic form cancel about two digits of the 7 that fp32 has
+        assert rel(score.cpu(), s) < 1e-6 and rel(adv.cpu(), want[:, None] * m.double()) < (1e-5 if B <= 1024 else 2e-4)

@@ -6,101 +6,207 @@
 
 namespace vb {
 
-// scores[b] = sum_t rewards[b,t]; group statistics accumulated with atomics: stats[g] = {sum, sumsq, count}.
-__global__ void grpo_scores_kernel(const float* __restrict__ rewards, const int* __restrict__ group, int B, int L,
-                                   float* __restrict__ scores, float* __restrict__ stats) {
-  const int b = blockIdx.x;
-  __shared__ float red[32];
+// scores[b] = sum_t rewards[b,t]; one block per row. With `stats` (zeroed by the caller) also stats[g] += {sum, sumsq, count}.
+template <typename I>
+__global__ void __launch_bounds__(128)
+grpo_scores_kernel(const float* __restrict__ rewards, const I* __restrict__ group, int L, float* __restrict__ scores,
+                   float* __restrict__ stats) {
+  __shared__ float red[4];
+  const float* row = rewards + static_cast<long long>(blockIdx.x) * L;
   float s = 0.f;
-  for (int t = threadIdx.x; t < L; t += blockDim.x) s += rewards[static_cast<long long>(b) * L + t];
+  for (int t = threadIdx.x; t < L; t += 128) s += row[t];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
-    float tot = 0.f;
-    for (int w = 0; w < (blockDim.x + 31) / 32; ++w) tot += red[w];
-    scores[b] = tot;
-    const int g = group[b];
-    atomicAdd(&stats[3 * g], tot);
-    atomicAdd(&stats[3 * g + 1], tot * tot);
-    atomicAdd(&stats[3 * g + 2], 1.f);
+    const float tot = red[0] + red[1] + red[2] + red[3];
+    scores[blockIdx.x] = tot;
+    if (stats) {
+      float* st = stats + 3 * static_cast<long long>(group[blockIdx.x]);
+      atomicAdd(st, tot);
+      atomicAdd(st + 1, tot * tot);
+      atomicAdd(st + 2, 1.f);
+    }
   }
 }
 
-// adv[b,t] = (score - mean_g) / (std_g + eps) * mask[b,t]   (unbiased std; singleton group: mean 0, std 1)
-__global__ void grpo_adv_kernel(const float* __restrict__ scores, const int* __restrict__ group,
-                                const float* __restrict__ stats, const float* __restrict__ mask, int B, int L,
-                                float eps, int norm_by_std, float* __restrict__ adv) {
+__device__ __forceinline__ float grpo_block_sum(float v, float* red) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return red[0] + red[1] + red[2] + red[3];
+}
+
+// adv[b,t] = (score - mean_g) / (std_g + eps) * mask[b,t]   (unbiased std; singleton group: mean 0, std 1). Without `stats` a row's
+// block finds the members of its group among the B scores itself: the mean first, then the squares around it (no cancellation), with
+// neither a zeroed scratch nor atomics. That scan is quadratic in B over the whole grid, so it is taken up to GRPO_SCAN_ROWS.
+template <typename I>
+__global__ void __launch_bounds__(128)
+grpo_adv_kernel(const float* __restrict__ scores, const I* __restrict__ group, const float* __restrict__ stats,
+                const float* __restrict__ mask, int B, int L, float eps, int norm_by_std, float* __restrict__ adv) {
+  __shared__ float red[4];
   const int b = blockIdx.x;
-  const int g = group[b];
-  const float n = stats[3 * g + 2];
+  const I g = group[b];
+  float n = 0.f, sum = 0.f;
+  if (stats) {
+    n = stats[3 * static_cast<long long>(g) + 2];
+    sum = stats[3 * static_cast<long long>(g)];
+  } else {
+    for (int i = threadIdx.x; i < B; i += 128)
+      if (group[i] == g) {
+        n += 1.f;
+        sum += scores[i];
+      }
+    n = grpo_block_sum(n, red);
+    sum = grpo_block_sum(sum, red);
+  }
   float mean = 0.f, sd = 1.f;
-  if (n > 1.5f) {
-    mean = stats[3 * g] / n;
-    const float var = fmaxf((stats[3 * g + 1] - n * mean * mean) / (n - 1.f), 0.f);
-    sd = sqrtf(var);
+  if (n > 1.5f && stats) {
+    mean = sum / n;
+    sd = sqrtf(fmaxf((stats[3 * static_cast<long long>(g) + 1] - n * mean * mean) / (n - 1.f), 0.f));
+  } else if (n > 1.5f) {
+    mean = sum / n;
+    float sq = 0.f;
+    for (int i = threadIdx.x; i < B; i += 128)
+      if (group[i] == g) sq += (scores[i] - mean) * (scores[i] - mean);
+    sd = sqrtf(grpo_block_sum(sq, red) / (n - 1.f));
   }
   const float a = norm_by_std ? (scores[b] - mean) / (sd + eps) : (scores[b] - mean);
-  for (int t = threadIdx.x; t < L; t += blockDim.x) {
-    const long long i = static_cast<long long>(b) * L + t;
-    adv[i] = a * mask[i];
-  }
+  const long long row = static_cast<long long>(b) * L;
+  for (int t = threadIdx.x; t < L; t += 128) adv[row + t] = a * mask[row + t];
 }
 
-// GAE: one thread per sequence, reverse scan. On masked tokens next-value and last-gae carry through.
-__global__ void gae_kernel(const float* __restrict__ rewards, const float* __restrict__ values,
-                           const float* __restrict__ mask, int B, int L, float gamma, float lam,
-                           float* __restrict__ adv, float* __restrict__ ret) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  float nextv = 0.f, last = 0.f;
-  for (int t = L - 1; t >= 0; --t) {
-    const long long i = static_cast<long long>(b) * L + t;
-    const float v = values[i], mk = mask[i];
-    const float delta = rewards[i] + gamma * nextv - v;
-    const float cand = delta + gamma * lam * last;
-    nextv = v * mk + (1.f - mk) * nextv;
-    last = cand * mk + (1.f - mk) * last;
-    adv[i] = last;
-    ret[i] = last + v;
-  }
+// One step of GAE, from the later state (value and advantage of the next unmasked token) to the earlier one, is an affine map
+//   n' = p n + u,   l' = q n + s l + w
+// with p = 1 - mask, u = mask * v, q = mask * gamma, s = mask * gamma * lambda + 1 - mask, w = mask * (r - v). Such maps compose to
+// maps of the same form, so the reverse scan over time is a prefix scan.
+struct GaeMap {
+  float p, u, q, s, w;
+};
+__device__ __forceinline__ GaeMap gae_after(const GaeMap& e, const GaeMap& l) {  // the map `l` (later tokens) first, then `e`
+  return {e.p * l.p, e.p * l.u + e.u, e.q * l.p + e.s * l.q, e.s * l.s, e.q * l.u + e.s * l.w + e.w};
+}
+__device__ __forceinline__ GaeMap gae_shfl_down(const GaeMap& m, int o) {
+  return {__shfl_down_sync(0xffffffffu, m.p, o), __shfl_down_sync(0xffffffffu, m.u, o), __shfl_down_sync(0xffffffffu, m.q, o),
+          __shfl_down_sync(0xffffffffu, m.s, o), __shfl_down_sync(0xffffffffu, m.w, o)};
 }
 
-// acc = {sum(x*m), sum(x*x*m), sum(m)}
-__global__ void masked_moments_kernel(const float* __restrict__ x, const float* __restrict__ mask, long long n,
-                                      float* __restrict__ acc) {
-  float s = 0.f, ss = 0.f, c = 0.f;
-  for (long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; i < n;
-       i += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const float m = mask[i], v = x[i];
-    s += v * m;
-    ss += v * v * m;
-    c += m;
-  }
+constexpr int GAE_PER = 4;           // consecutive tokens per thread
+constexpr int GAE_MAX_BLOCKS = 148 * 8;
+
+// A block takes whole rows and walks a row from its end in tiles of blockDim * 4 tokens: every thread composes the maps of its four
+// tokens, a scan over the block gives the state behind them, and the four tokens are then stepped through. 512 x 1024 tokens: 267 us with
+// one thread per row (serial loads of the whole row, uncoalesced) -> 8 us for the scan and the whitening (13.8 us the whole call, 284 before); the bytes alone are 1.6 us, what is left is one
+// row's chain of load, scan and store. `part` (null: no whitening) gets the block's masked sums of the advantages: sum, sum of
+// squares, count.
+__global__ void __launch_bounds__(256)
+gae_kernel(const float* __restrict__ rewards, const float* __restrict__ values, const float* __restrict__ mask, int B, int L, float gamma,
+           float lam, float* __restrict__ adv, float* __restrict__ ret, double* __restrict__ part) {
+  __shared__ GaeMap warp_map[8];
+  __shared__ float carry[2];
+  __shared__ double red[8][3];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int tile = blockDim.x * GAE_PER;
+  float s1 = 0.f, s2 = 0.f, s0 = 0.f;
+  for (int b = blockIdx.x; b < B; b += gridDim.x) {
+    const long long row = static_cast<long long>(b) * L;
+    float n_in = 0.f, l_in = 0.f;  // the state behind the tile
+    for (int t1 = ((L + tile - 1) / tile) * tile; t1 > 0; t1 -= tile) {
+      const int t0 = t1 - tile + threadIdx.x * GAE_PER;
+      float r[GAE_PER], v[GAE_PER], m[GAE_PER];
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    s += __shfl_xor_sync(0xffffffffu, s, o);
-    ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    c += __shfl_xor_sync(0xffffffffu, c, o);
+      for (int j = 0; j < GAE_PER; ++j) {
+        const bool in = t0 + j < L;
+        r[j] = in ? rewards[row + t0 + j] : 0.f;
+        v[j] = in ? values[row + t0 + j] : 0.f;
+        m[j] = in ? mask[row + t0 + j] : 0.f;  // a masked token hands the state through
+      }
+      GaeMap acc{1.f, 0.f, 0.f, 1.f, 0.f};
+#pragma unroll
+      for (int j = GAE_PER - 1; j >= 0; --j)
+        acc = gae_after({1.f - m[j], m[j] * v[j], m[j] * gamma, m[j] * gamma * lam + 1.f - m[j], m[j] * (r[j] - v[j])}, acc);
+      // inclusive scan from the warp's last lane backwards, then over the warps
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const GaeMap later = gae_shfl_down(acc, o);
+        if (lane + o < 32) acc = gae_after(acc, later);
+      }
+      if (lane == 0) warp_map[warp] = acc;
+      GaeMap behind = gae_shfl_down(acc, 1);  // of the lanes behind this one
+      if (lane == 31) behind = {1.f, 0.f, 0.f, 1.f, 0.f};
+      __syncthreads();
+      for (int k = warp + 1; k < warps; ++k) behind = gae_after(behind, warp_map[k]);
+      float nextv = behind.p * n_in + behind.u, last = behind.q * n_in + behind.s * l_in + behind.w;
+#pragma unroll
+      for (int j = GAE_PER - 1; j >= 0; --j) {
+        const float cand = r[j] + gamma * nextv - v[j] + gamma * lam * last;
+        nextv = v[j] * m[j] + (1.f - m[j]) * nextv;
+        last = cand * m[j] + (1.f - m[j]) * last;
+        if (t0 + j < L) {
+          adv[row + t0 + j] = last;
+          ret[row + t0 + j] = last + v[j];
+          s1 += last * m[j];
+          s2 += last * last * m[j];
+          s0 += m[j];
+        }
+      }
+      if (threadIdx.x == 0) {
+        carry[0] = nextv;
+        carry[1] = last;
+      }
+      __syncthreads();
+      n_in = carry[0];
+      l_in = carry[1];
+    }
   }
-  if ((threadIdx.x & 31) == 0) {
-    atomicAdd(&acc[0], s);
-    atomicAdd(&acc[1], ss);
-    atomicAdd(&acc[2], c);
+  if (!part) return;
+  double d[3] = {s1, s2, s0};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) d[k] += __shfl_xor_sync(0xffffffffu, d[k], o);
+    if (lane == 0) red[warp][k] = d[k];
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double t = 0;
+    for (int k = 0; k < warps; ++k) t += red[k][threadIdx.x];
+    part[blockIdx.x * 3 + threadIdx.x] = t;
   }
 }
-// x <- (x - mean) * rsqrt(var + 1e-8) * (apply_mask ? mask : 1), unbiased variance
-__global__ void whiten_kernel(float* __restrict__ x, const float* __restrict__ mask, long long n,
-                              const float* __restrict__ acc, int apply_mask) {
-  const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  if (i >= n) return;
-  const float c = acc[2];
-  const float mean = acc[0] / (c + 1e-8f);
-  float var = acc[1] / (c + 1e-8f) - mean * mean;
-  var = fmaxf(var, 0.f) * (c / fmaxf(c - 1.f, 1.f));
-  const float w = (x[i] - mean) * rsqrtf(var + 1e-8f);
-  x[i] = apply_mask ? w * mask[i] : w;
+
+// x <- (x - mean) * rsqrt(var + 1e-8), unbiased variance over the unmasked tokens. Every block folds the partial sums of the scan
+// (at most 1184 x 3) itself, in one order: no memset, no atomics, the same bits every time.
+__global__ void __launch_bounds__(256)
+whiten_kernel(float* __restrict__ x, long long n, const double* __restrict__ part, int nparts) {
+  __shared__ double red[8][3];
+  __shared__ float mw[2];
+  double d[3] = {0, 0, 0};
+  for (int i = threadIdx.x; i < nparts; i += blockDim.x)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) d[k] += part[i * 3 + k];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) d[k] += __shfl_xor_sync(0xffffffffu, d[k], o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] = d[k];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t[3] = {0, 0, 0};
+    for (int k = 0; k < 8; ++k)
+      for (int j = 0; j < 3; ++j) t[j] += red[k][j];
+    const double c = t[2], mean = t[0] / (c + 1e-8);
+    const double var = fmax(t[1] / (c + 1e-8) - mean * mean, 0.0) * (c / fmax(c - 1.0, 1.0));
+    mw[0] = static_cast<float>(mean);
+    mw[1] = static_cast<float>(1.0 / sqrt(var + 1e-8));
+  }
+  __syncthreads();
+  const float mean = mw[0], scale = mw[1];
+  for (long long i = blockIdx.x * 256LL + threadIdx.x; i < n; i += gridDim.x * 256LL) x[i] = (x[i] - mean) * scale;
 }
 
 }  // namespace vb
@@ -109,27 +215,47 @@ using namespace vb;
 
 extern "C" {
 
-// stats: scratch of 3 * num_groups floats, zeroed by this call.
-int vb_grpo_advantage(const float* rewards, const float* mask, const int* group, int B, int L, int num_groups,
-                      float eps, int norm_by_std, float* scores, float* stats, float* adv, cudaStream_t s) {
+// Up to this many rows the scan of grpo_adv_kernel is the cheaper way (320 x 2048: 21.5 us for the call with memset, conversion of the
+// ids and atomics, 12.6 us with the scan; at 2560 rows the scan's 157 MB of L2 reads take longer than the atomics).
+constexpr int GRPO_SCAN_ROWS = 1024;
+int vb_grpo_needs_stats(int B) { return B > GRPO_SCAN_ROWS; }
+
+// group: int32 or int64 ids (group64); ids in [0, num_groups). stats: 3 * num_groups floats (zeroed here) when vb_grpo_needs_stats.
+int vb_grpo_advantage(const float* rewards, const float* mask, const void* group, int group64, int B, int L, int num_groups, float eps,
+                      int norm_by_std, float* scores, float* stats, float* adv, cudaStream_t s) {
   if (B == 0) return 0;
-  cudaMemsetAsync(stats, 0, sizeof(float) * 3 * num_groups, s);
-  grpo_scores_kernel<<<B, 128, 0, s>>>(rewards, group, B, L, scores, stats);
-  grpo_adv_kernel<<<B, 128, 0, s>>>(scores, group, stats, mask, B, L, eps, norm_by_std, adv);
+  if (vb_grpo_needs_stats(B))
+    cudaMemsetAsync(stats, 0, sizeof(float) * 3 * num_groups, s);
+  else
+    stats = nullptr;
+  if (group64) {
+    const long long* g = static_cast<const long long*>(group);
+    grpo_scores_kernel<<<B, 128, 0, s>>>(rewards, g, L, scores, stats);
+    grpo_adv_kernel<<<B, 128, 0, s>>>(scores, g, stats, mask, B, L, eps, norm_by_std, adv);
+  } else {
+    const int* g = static_cast<const int*>(group);
+    grpo_scores_kernel<<<B, 128, 0, s>>>(rewards, g, L, scores, stats);
+    grpo_adv_kernel<<<B, 128, 0, s>>>(scores, g, stats, mask, B, L, eps, norm_by_std, adv);
+  }
   return static_cast<int>(cudaGetLastError());
 }
 
-// acc: scratch of 4 floats, zeroed by this call. Whitening of the advantages over the whole batch (statistics
-// over unmasked tokens, result not re-masked) is applied when `whiten` is non-zero.
-int vb_gae(const float* rewards, const float* values, const float* mask, int B, int L, float gamma, float lam,
-           int whiten, float* adv, float* ret, float* acc, cudaStream_t s) {
-  if (B == 0) return 0;
-  gae_kernel<<<(B + 63) / 64, 64, 0, s>>>(rewards, values, mask, B, L, gamma, lam, adv, ret);
-  if (whiten) {
+// Blocks of the scan = rows of `part` (3 doubles each). A row's tiles follow one another, so rows are what fills the machine; a block
+// is as wide as the row needs, up to 256 threads (1024 tokens per tile).
+int vb_gae_blocks(int B) { return B < GAE_MAX_BLOCKS ? B : GAE_MAX_BLOCKS; }
+
+// Whitening of the advantages over the whole batch (statistics over unmasked tokens, result not re-masked) is applied when `part` is
+// given.
+int vb_gae(const float* rewards, const float* values, const float* mask, int B, int L, float gamma, float lam, float* adv, float* ret,
+           double* part, cudaStream_t s) {
+  if (B == 0 || L == 0) return 0;
+  const int want = (L + GAE_PER - 1) / GAE_PER;
+  const int threads = want >= 256 ? 256 : (want + 31) / 32 * 32;
+  gae_kernel<<<vb_gae_blocks(B), threads, 0, s>>>(rewards, values, mask, B, L, gamma, lam, adv, ret, part);
+  if (part) {
     const long long n = static_cast<long long>(B) * L;
-    cudaMemsetAsync(acc, 0, sizeof(float) * 4, s);
-    masked_moments_kernel<<<148 * 2, 256, 0, s>>>(adv, mask, n, acc);
-    whiten_kernel<<<static_cast<int>((n + 255) / 256), 256, 0, s>>>(adv, mask, n, acc, 0);
+    const long long want_blocks = (n + 1023) / 1024;
+    whiten_kernel<<<static_cast<int>(want_blocks < 148 * 4 ? want_blocks : 148 * 4), 256, 0, s>>>(adv, n, part, vb_gae_blocks(B));
   }
   return static_cast<int>(cudaGetLastError());
 }

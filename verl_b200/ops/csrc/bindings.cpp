@@ -539,16 +539,18 @@ std::tuple<Tensor, Tensor> grpo_advantage(const Tensor& rewards, const Tensor& m
                                           int64_t num_groups, double eps, bool norm_by_std) {
   CHECK_F32(rewards);
   CHECK_F32(mask);
-  TORCH_CHECK(group.scalar_type() == at::kInt && rewards.is_contiguous() && mask.is_contiguous());
+  TORCH_CHECK((group.scalar_type() == at::kInt || group.scalar_type() == at::kLong) && group.is_contiguous() && rewards.is_contiguous() &&
+              mask.is_contiguous());
+  TORCH_CHECK(group.is_cuda() && group.numel() == rewards.size(0) && mask.sizes() == rewards.sizes());
   const c10::cuda::CUDAGuard guard(rewards.device());
   const int64_t B = rewards.size(0), L = rewards.size(1);
   Tensor adv = at::empty_like(rewards);
   Tensor scores = at::empty({B}, rewards.options());
-  Tensor stats = at::empty({num_groups, 3}, rewards.options());
+  Tensor stats = vb_grpo_needs_stats((int)B) ? at::empty({num_groups, 3}, rewards.options()) : Tensor();
   count(2);
-  CHECK_RC(vb_grpo_advantage(rewards.data_ptr<float>(), mask.data_ptr<float>(), group.data_ptr<int>(), (int)B, (int)L,
-                             (int)num_groups, (float)eps, norm_by_std, scores.data_ptr<float>(),
-                             stats.data_ptr<float>(), adv.data_ptr<float>(), cur_stream()),
+  CHECK_RC(vb_grpo_advantage(rewards.data_ptr<float>(), mask.data_ptr<float>(), group.data_ptr(), group.scalar_type() == at::kLong, (int)B,
+                             (int)L, (int)num_groups, (float)eps, norm_by_std, scores.data_ptr<float>(),
+                             stats.defined() ? stats.data_ptr<float>() : nullptr, adv.data_ptr<float>(), cur_stream()),
            "vb_grpo_advantage");
   return {adv, scores};
 }
@@ -561,11 +563,12 @@ std::tuple<Tensor, Tensor> gae(const Tensor& rewards, const Tensor& values, cons
   TORCH_CHECK(rewards.is_contiguous() && values.is_contiguous() && mask.is_contiguous());
   const c10::cuda::CUDAGuard guard(rewards.device());
   Tensor adv = at::empty_like(rewards), ret = at::empty_like(rewards);
-  Tensor acc = at::empty({4}, rewards.options());
-  count(3);
+  const int64_t blocks = vb_gae_blocks((int)rewards.size(0));
+  Tensor part = whiten ? at::empty({blocks, 3}, rewards.options().dtype(at::kDouble)) : Tensor();
+  count(whiten ? 2 : 1);
   CHECK_RC(vb_gae(rewards.data_ptr<float>(), values.data_ptr<float>(), mask.data_ptr<float>(), (int)rewards.size(0),
-                  (int)rewards.size(1), (float)gamma, (float)lam, whiten, adv.data_ptr<float>(), ret.data_ptr<float>(),
-                  acc.data_ptr<float>(), cur_stream()),
+                  (int)rewards.size(1), (float)gamma, (float)lam, adv.data_ptr<float>(), ret.data_ptr<float>(),
+                  whiten ? part.data_ptr<double>() : nullptr, cur_stream()),
            "vb_gae");
   return {adv, ret};
 }

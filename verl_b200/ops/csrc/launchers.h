@@ -146,8 +146,10 @@ int vb_moe_combine_peer(const unsigned long long* y_ptrs_dev, const int* src_ran
                         long long ldo, int T, int H, int k, cudaStream_t s);
 int vb_moe_publish_counts(const int* counts, const unsigned long long* table_ptrs_dev, int W, int rank, int E, cudaStream_t s);
 // advantage.cu
-int vb_grpo_advantage(const float* rewards, const float* mask, const int* group, int B, int L, int num_groups,
-                      float eps, int norm_by_std, float* scores, float* stats, float* adv, cudaStream_t s);
-int vb_gae(const float* rewards, const float* values, const float* mask, int B, int L, float gamma, float lam,
-           int whiten, float* adv, float* ret, float* acc, cudaStream_t s);
+int vb_grpo_needs_stats(int B);
+int vb_grpo_advantage(const float* rewards, const float* mask, const void* group, int group64, int B, int L, int num_groups, float eps,
+                      int norm_by_std, float* scores, float* stats, float* adv, cudaStream_t s);
+int vb_gae_blocks(int B);
+int vb_gae(const float* rewards, const float* values, const float* mask, int B, int L, float gamma, float lam, float* adv, float* ret,
+           double* part, cudaStream_t s);
 }

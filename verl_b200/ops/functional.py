@@ -637,8 +637,8 @@ def grpo_advantage(rewards: torch.Tensor, mask: torch.Tensor, group: torch.Tenso
                    eps: float = 1e-6, norm_by_std: bool = True):
     """Device GRPO outcome advantage. ``group`` is an int tensor of group ids in [0, num_groups)."""
     if rewards.is_cuda:
-        return _ops().grpo_advantage(rewards.float().contiguous(), mask.float().contiguous(),
-                                     group.to(torch.int32).contiguous(), num_groups, eps, norm_by_std)
+        ids = group if group.dtype in (torch.int32, torch.int64) else group.to(torch.int32)
+        return _ops().grpo_advantage(rewards.float().contiguous(), mask.float().contiguous(), ids.contiguous(), num_groups, eps, norm_by_std)
     scores = rewards.float().sum(-1)
     adv = torch.zeros_like(scores)
     for g in range(num_groups):
