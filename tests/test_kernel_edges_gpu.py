@@ -72,3 +72,51 @@ def test_group_advantage_rows(ops, B, L, dtype):
                     want[sel] /= s[sel].std() + 1e-6
         # the sums of squares of the atomic form cancel about two digits of the 7 that fp32 has
         assert rel(score.cpu(), s) < 1e-6 and rel(adv.cpu(), want[:, None] * m.double()) < (1e-5 if B <= 1024 else 2e-4)
+
+
+# ------------------------------------------------------------------------------------------------ sampler
+def _uniforms(seeds, V, step):
+    """The sampler's stream of uniforms: splitmix64's finaliser on uint64, the upper 24 bits, halfway between the grid points."""
+    def mix(z):
+        z = z + np.uint64(0x9E3779B97F4A7C15)
+        z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+        z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+        return z ^ (z >> np.uint64(31))
+
+    with np.errstate(over="ignore"):
+        key = mix(seeds.astype(np.uint64) ^ (np.uint64(step) * np.uint64(0xD1342543DE82EF95)))
+        h = (mix(key[:, None] + np.arange(V, dtype=np.uint64)[None]) >> np.uint64(40)).astype(np.int64)
+    return h, (h.astype(np.float32) + np.float32(0.5)).astype(np.float64) / 2.0**24
+
+
+@pytest.mark.parametrize("B,V,ld,valid", [(1, 8, 8, 8), (3, 4096, 4096, 4095), (5, 4104, 4104, 4104), (2, 16392, 16400, 0), (2, 33001, 33003, 0),
+                                          (170, 9000, 9000, 8999), (1200, 1000, 1000, 0)])
+@pytest.mark.parametrize("scale", [0.3, 2.5, 40.0])
+def test_sampler_takes_the_token_of_the_whole_row(ops, B, V, ld, valid, scale):
+    from verl_b200.ops import functional as F
+
+    g = torch.Generator().manual_seed(V + B)
+    lg = (torch.randn(B, ld, generator=g) * scale).bfloat16()
+    lg[:, ::97] = -math.inf  # masked logits
+    if B > 1:
+        lg[0] = -math.inf  # a row with one token left
+        lg[0, (valid or V) // 2] = -300.0
+    seeds = torch.randint(1 << 40, (B,), generator=g)
+    row = lg.to(DEV)[:, :V]
+    n = valid or V
+    x = lg[:, :n].double()
+    for T in (1.0, 0.7, 0.0):
+        tok, lp = F.sample_tokens(row, T, seeds.to(DEV), 3, valid)
+        tok, lp = tok.cpu(), lp.cpu()
+        xt = (lg[:, :n].float() * torch.tensor(1.0 / T if T else 1.0, dtype=torch.float32)).double()
+        if T:
+            h, u = _uniforms(seeds.numpy(), n, 3)
+            score = xt - torch.log(-torch.log(torch.from_numpy(u)))
+            plain = torch.from_numpy((h < 2**24 - 512).all(-1))  # near u = 1 the device's logarithm is coarser than the spacing of u
+        else:
+            score, plain = x, torch.ones(B, dtype=torch.bool)
+            assert torch.equal(tok, x.argmax(-1))
+        got = score.gather(1, tok[:, None])[:, 0]
+        assert ((score.max(-1).values - got)[plain] <= 1e-4 * (1 + score.max(-1).values.abs()[plain])).all()
+        want = xt.gather(1, tok[:, None])[:, 0] - xt.logsumexp(-1)
+        assert (lp.double() - want).abs().max() < 1e-4 * (1 + xt[xt > -math.inf].abs().max())

@@ -1,6 +1,7 @@
 // Rollout-engine kernels: paged KV-cache append, paged decode attention (GQA-aware, one pass over the
 // cache per KV head), and the token sampler (temperature + Gumbel-max with the sampled token's log-prob).
 // All are bandwidth-bound: the design goal is one coalesced read of every cache byte per decode step.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -234,71 +235,161 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
   return z ^ (z >> 31);
 }
 
-// One block per row. logits [B, V] bf16 (row stride ld). Columns >= valid_vocab are masked out.
-// Greedy when inv_temp <= 0 (the log-prob is then reported at temperature 1).
-__global__ void sample_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int V, int valid_vocab,
-                              float inv_temp, const long long* __restrict__ seeds, long long step,
-                              long long* __restrict__ tokens, float* __restrict__ logprobs) {
-  const int row = blockIdx.x;
-  const bool greedy = inv_temp <= 0.f;
-  const float it = greedy ? 1.f : inv_temp;
+// Token and log-prob of every row of logits [B, V] bf16 (row stride ld). Columns >= valid_vocab are masked out.
+// Greedy when inv_temp <= 0 (the log-prob is then reported at temperature 1), else Gumbel-max over x + g(u_i) with
+// u_i = ((mix64(key + i) >> 40) + 0.5) / 2^24 and g(u) = -log(-log(u)).
+//
+// A row is spread over a cluster of CTAs whose partial results meet in distributed shared memory, so that few rows still use the whole
+// chip and many rows end together (a CTA per row: 320 rows were two waves of 148 x 2). A thread takes 8 neighbouring logits
+// at a time: one rescaling of the running sum and one exponential per logit. That exponential also decides which logits need their two
+// logarithms at all: x + g(u) can beat the warp's best score s only if u >= exp(-exp(x - s)), and exp(-t) >= 1 - t, so a logit with
+// u < 1 - t, t = e^(x - m) e^(m - s), cannot win. The bound is widened by 66 / 2^24 and a factor 1 + 2^-10 on t, far above the rounding
+// of its terms and of the logarithms, and the 64 uppermost values of u always count as candidates, so the token is the one that
+// evaluating every logit gives (of equal scores the first). What is left is the 64-bit hash: 44 instructions a logit in all, issued in
+// two of three cycles; loading a turn ahead and collecting the candidates of a turn in a mask were both slower (98 and 105 us).
+// 320 x 152064 at temperature 1: 160 us -> 96 us; greedy, where the row is what counts: 37 us (15 us for the bytes).
+constexpr int SAMPLE_THREADS = 256;
+
+struct SamplePart {
+  float m, l, best, best_x;
+  int best_i;
+};
+__device__ __forceinline__ void sample_fold(SamplePart& a, const SamplePart& b) {
+  const float mn = fmaxf(a.m, b.m);
+  a.l = (mn == -INFINITY) ? a.l + b.l : a.l * __expf(a.m - mn) + b.l * __expf(b.m - mn);
+  a.m = mn;
+  if (b.best > a.best || (b.best == a.best && b.best_i < a.best_i)) {
+    a.best = b.best;
+    a.best_i = b.best_i;
+    a.best_x = b.best_x;
+  }
+}
+
+// mix64(key + i) >> 40: the last step of mix64, z ^ (z >> 31), touches only the lowest of the upper 32 bits, which the shift drops
+__device__ __forceinline__ uint32_t sample_bits(uint64_t key, int i) {
+  uint64_t z = key + static_cast<uint64_t>(i) + 0x9E3779B97F4A7C15ull;
+  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+  return static_cast<uint32_t>(z >> 40);
+}
+__device__ __forceinline__ float exp2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float sample_score(float x, uint32_t h) {
+  const float u = (static_cast<float>(h) + 0.5f) * (1.0f / 16777216.0f);  // (0,1)
+  return x - __logf(-__logf(u));
+}
+// the largest value of a warp (not NaN), through the order-preserving map of floats to unsigned integers
+__device__ __forceinline__ float warp_max(float v) {
+  const uint32_t f = __float_as_uint(v);
+  const uint32_t k = __reduce_max_sync(0xffffffffu, (f & 0x80000000u) ? ~f : (f | 0x80000000u));
+  return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k);
+}
+
+template <bool VEC, bool GREEDY>
+__global__ void __launch_bounds__(SAMPLE_THREADS, 6)
+sample_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int valid_vocab, float inv_temp,
+              const long long* __restrict__ seeds, long long step, long long* __restrict__ tokens, float* __restrict__ logprobs) {
+  namespace cg = cooperative_groups;
+  const cg::cluster_group cluster = cg::this_cluster();
+  const int parts = static_cast<int>(cluster.num_blocks()), part = static_cast<int>(cluster.block_rank());
+  const int row = blockIdx.x / parts;
+  constexpr float LOG2E = 1.4426950408889634f;
+  const float it = GREEDY ? 1.f : inv_temp, it2 = it * LOG2E;
   const __nv_bfloat16* lr = logits + row * ld;
   const uint64_t key = mix64(static_cast<uint64_t>(seeds[row]) ^ (static_cast<uint64_t>(step) * 0xD1342543DE82EF95ull));
-  float m = -INFINITY, l = 0.f, best = -INFINITY, best_x = 0.f;
-  int best_i = 0;
-  for (int i = threadIdx.x; i < valid_vocab; i += blockDim.x) {
-    const float x = __bfloat162float(lr[i]) * it;
-    const float mn = fmaxf(m, x);
-    l = l * __expf(m - mn) + __expf(x - mn);
-    m = mn;
-    float score = x;
-    if (!greedy) {
-      const uint64_t h = mix64(key + static_cast<uint64_t>(i));
-      const float u = (static_cast<float>(h >> 40) + 0.5f) * (1.0f / 16777216.0f);  // (0,1)
-      score = x - __logf(-__logf(u));
-    }
-    if (score > best) {
-      best = score;
-      best_i = i;
-      best_x = x;
-    }
-  }
-  __shared__ float sm[32], sl[32], sb[32], sx[32];
-  __shared__ int si[32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  SamplePart a{-INFINITY, 0.f, -INFINITY, 0.f, 0x7fffffff};
+  float warp_best = -INFINITY;
+  const int stride = parts * SAMPLE_THREADS * 8;
+  const int lane = threadIdx.x & 31;
+  // every lane of a warp makes the same number of turns (the loop holds warp-wide exchanges): the bound is the warp's first logit
+  for (int w0 = (part * SAMPLE_THREADS + static_cast<int>(threadIdx.x) - lane) * 8; w0 < valid_vocab; w0 += stride) {
+    const int i0 = w0 + lane * 8;
+    float x[8];  // as stored: the temperature comes in with the exponential's scale, and where a logit is a candidate
+    if (VEC && i0 + 8 <= valid_vocab) {
+      const uint4 raw = *reinterpret_cast<const uint4*>(lr + i0);
+      const uint32_t u[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float m2 = __shfl_xor_sync(0xffffffffu, m, o), l2 = __shfl_xor_sync(0xffffffffu, l, o);
-    const float b2 = __shfl_xor_sync(0xffffffffu, best, o), x2 = __shfl_xor_sync(0xffffffffu, best_x, o);
-    const int i2 = __shfl_xor_sync(0xffffffffu, best_i, o);
-    const float mn = fmaxf(m, m2);
-    l = (mn == -INFINITY) ? 0.f : l * __expf(m - mn) + l2 * __expf(m2 - mn);
-    m = mn;
-    if (b2 > best || (b2 == best && i2 < best_i)) {
-      best = b2;
-      best_i = i2;
-      best_x = x2;
+      for (int j = 0; j < 4; ++j) {
+        x[2 * j] = __uint_as_float(u[j] << 16);
+        x[2 * j + 1] = __uint_as_float(u[j] & 0xffff0000u);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = i0 + j < valid_vocab ? __bfloat162float(lr[i0 + j]) : -INFINITY;
     }
-  }
-  if (lane == 0) {
-    sm[w] = m; sl[w] = l; sb[w] = best; sx[w] = best_x; si[w] = best_i;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = blockDim.x >> 5;
-    for (int k = 1; k < nw; ++k) {
-      const float mn = fmaxf(m, sm[k]);
-      l = (mn == -INFINITY) ? 0.f : l * __expf(m - mn) + sl[k] * __expf(sm[k] - mn);
-      m = mn;
-      if (sb[k] > best || (sb[k] == best && si[k] < best_i)) {
-        best = sb[k];
-        best_i = si[k];
-        best_x = sx[k];
+    float mx = x[0];
+#pragma unroll
+    for (int j = 1; j < 8; ++j) mx = fmaxf(mx, x[j]);
+    const float mn = fmaxf(a.m, mx * it);
+    const float ref = mn == -INFINITY ? 0.f : mn;  // nothing but masked logits so far: their exponentials are 0
+    float sum = a.l * __expf(a.m - ref);
+    const float ref2 = ref * LOG2E;
+    if (!GREEDY && warp_best == -INFINITY) {
+      // a first score to beat: every lane's largest logit
+      int jm = 0;
+#pragma unroll
+      for (int j = 7; j >= 0; --j) jm = x[j] == mx ? j : jm;
+      a.best = sample_score(mx * it, sample_bits(key, i0 + jm));
+      if (!(a.best > -INFINITY)) a.best = -INFINITY;  // masked or NaN: nothing to beat yet
+      else {
+        a.best_i = i0 + jm;
+        a.best_x = mx * it;
+      }
+      warp_best = warp_max(a.best);
+    }
+    const float t_scale = 8388608.f * 1.0009765625f * __expf(ref - warp_best);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float e = exp2_approx(fmaf(x[j], it2, -ref2));
+      sum += e;
+      if (GREEDY) {
+        if (x[j] > a.best) {
+          a.best = x[j];
+          a.best_i = i0 + j;
+          a.best_x = x[j];
+        }
+      } else {
+        // h / 2 as a float without a conversion (those run at the rate of the exponentials): 2^23 + h / 2
+        const float bound = fmaf(-e, t_scale, 16777216.f - 33.f);
+        const uint32_t h = sample_bits(key, i0 + j);
+        if (!(__uint_as_float(0x4B000000u | (h >> 1)) < bound)) {  // a NaN bound counts as a candidate
+          const float score = sample_score(x[j] * it, h);
+          if (score > a.best || (score == a.best && i0 + j < a.best_i)) {
+            a.best = score;
+            a.best_i = i0 + j;
+            a.best_x = x[j] * it;
+          }
+        }
       }
     }
-    tokens[row] = best_i;
-    if (logprobs) logprobs[row] = best_x - (m + __logf(l));
+    a.m = mn;
+    a.l = sum;
+    if (!GREEDY) warp_best = warp_max(a.best);
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const SamplePart b{__shfl_xor_sync(0xffffffffu, a.m, o), __shfl_xor_sync(0xffffffffu, a.l, o), __shfl_xor_sync(0xffffffffu, a.best, o),
+                       __shfl_xor_sync(0xffffffffu, a.best_x, o), __shfl_xor_sync(0xffffffffu, a.best_i, o)};
+    sample_fold(a, b);
+  }
+  __shared__ SamplePart warp_part[SAMPLE_THREADS / 32];
+  __shared__ SamplePart cta_part;
+  if (lane == 0) warp_part[threadIdx.x >> 5] = a;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < SAMPLE_THREADS / 32; ++k) sample_fold(a, warp_part[k]);
+    cta_part = a;
+  }
+  cluster.sync();
+  if (part == 0 && threadIdx.x == 0) {
+    for (int k = 1; k < parts; ++k) sample_fold(a, *cluster.map_shared_rank(&cta_part, k));
+    tokens[row] = a.best_i == 0x7fffffff ? 0 : a.best_i;
+    if (logprobs) logprobs[row] = a.best_x - (a.m + __logf(a.l));
+  }
+  cluster.sync();  // a CTA's shared memory is read by its cluster until here
 }
 
 // ---- top-k / top-p (nucleus) sampling without a sort.
@@ -554,9 +645,25 @@ int vb_sample(const void* logits, long long ld, int B, int V, int valid_vocab, f
               long long step, long long* tokens, float* logprobs, cudaStream_t s) {
   if (B == 0) return 0;
   if (valid_vocab <= 0 || valid_vocab > V) valid_vocab = V;
-  sample_kernel<<<B, 1024, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(logits), ld, V, valid_vocab, inv_temp, seeds,
-                                   step, tokens, logprobs);
-  return static_cast<int>(cudaGetLastError());
+  // 16-byte loads where every row starts on a 16-byte boundary. CTAs per row: as many as have a full turn of logits, up to the portable
+  // cluster size, no more than about two waves of the chip need (148 SMs x 4 CTAs).
+  const bool vec = reinterpret_cast<uintptr_t>(logits) % 16 == 0 && ld % 8 == 0;
+  int parts = 1;
+  while (parts < 8 && parts * SAMPLE_THREADS * 8 < valid_vocab && static_cast<long long>(B) * parts < 148 * 16) parts *= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(B) * parts);
+  cfg.blockDim = dim3(SAMPLE_THREADS);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = parts;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const auto kernel = inv_temp <= 0.f ? (vec ? sample_kernel<true, true> : sample_kernel<false, true>)
+                                      : (vec ? sample_kernel<true, false> : sample_kernel<false, false>);
+  return static_cast<int>(cudaLaunchKernelEx(&cfg, kernel, reinterpret_cast<const __nv_bfloat16*>(logits), ld, valid_vocab, inv_temp, seeds,
+                                             step, tokens, logprobs));
 }
 
 }  // extern "C"
