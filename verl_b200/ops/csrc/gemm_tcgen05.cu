@@ -1521,21 +1521,44 @@ extern "C" int vb_gemm_status() {
 
 namespace vb {
 
-// logprob / entropy from the per-tile partials written by EPI_LSE.
-__global__ void lmhead_merge_kernel(const float* __restrict__ partial, const float* __restrict__ label_logit,
-                                    float* __restrict__ logprob, float* __restrict__ entropy,
-                                    float* __restrict__ lse_out, int T, int num_n) {
-  const int row = blockIdx.x * blockDim.x + threadIdx.x;
-  if (row >= T) return;
+// logprob / entropy from the per-tile partials written by EPI_LSE. 32 rows to a block (a warp reads whole lines of a plane), the tiles
+// dealt over its 16 warps, each of which keeps a running maximum so that every plane is read once. A thread per row, walking the 594
+// tiles of a vocabulary of 152064 one after the other and twice, took 130 us at 23 rows and 237 us at 12,800; now 21 us at 23 rows (a block of one warp per tile group: latency).
+constexpr int MERGE_WARPS = 16;
+__global__ void __launch_bounds__(MERGE_WARPS * 32)
+lmhead_merge_kernel(const float* __restrict__ partial, const float* __restrict__ label_logit, float* __restrict__ logprob,
+                    float* __restrict__ entropy, float* __restrict__ lse_out, int T, int num_n) {
+  __shared__ float sm[MERGE_WARPS][32], sl[MERGE_WARPS][32], ss[MERGE_WARPS][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = blockIdx.x * 32 + lane;
   const long long plane = static_cast<long long>(num_n) * T;
-  float M = -INFINITY;
-  for (int n = 0; n < num_n; ++n) M = fmaxf(M, partial[static_cast<long long>(n) * T + row]);
-  float L = 0.f, S = 0.f;
-  for (int n = 0; n < num_n; ++n) {
-    const long long o = static_cast<long long>(n) * T + row;
-    const float w = __expf(partial[o] - M);
-    L += partial[plane + o] * w;
-    S += partial[2 * plane + o] * w;
+  float M = -INFINITY, L = 0.f, S = 0.f;
+  if (row < T) {
+#pragma unroll 4
+    for (int n = warp; n < num_n; n += MERGE_WARPS) {
+      const long long o = static_cast<long long>(n) * T + row;
+      const float m = partial[o], l = partial[plane + o], x = partial[2 * plane + o];
+      const float mn = fmaxf(M, m);
+      const float a = M == -INFINITY ? 0.f : __expf(M - mn), w = m == -INFINITY ? 0.f : __expf(m - mn);
+      L = L * a + l * w;
+      S = S * a + x * w;
+      M = mn;
+    }
+  }
+  sm[warp][lane] = M;
+  sl[warp][lane] = L;
+  ss[warp][lane] = S;
+  __syncthreads();
+  if (warp != 0 || row >= T) return;
+#pragma unroll
+  for (int k = 1; k < MERGE_WARPS; ++k) M = fmaxf(M, sm[k][lane]);
+  L = 0.f;
+  S = 0.f;
+#pragma unroll
+  for (int k = 0; k < MERGE_WARPS; ++k) {
+    const float w = __expf(sm[k][lane] - M);  // a warp without a tile: exp(-inf) = 0
+    L += sl[k][lane] * w;
+    S += ss[k][lane] * w;
   }
   const float lse = M + __logf(L);
   if (logprob) logprob[row] = label_logit[row] - lse;
@@ -1564,8 +1587,8 @@ extern "C" int vb_lmhead_fwd(const void* hidden, const void* weight, const long 
   p.labels = labels; p.label_offset = 0; p.inv_temp = inv_temp; p.partial = partial; p.label_logit = label_logit;
   cudaError_t e = launch_variant<256, false, false, 4, EPI_LSE>(ta, tb, p, num_sms(), stream);
   if (e != cudaSuccess) return static_cast<int>(e);
-  lmhead_merge_kernel<<<(T + 127) / 128, 128, 0, stream>>>(partial, label_logit, logprob, entropy, lse, T,
-                                                         vb_lmhead_num_tiles(V));
+  lmhead_merge_kernel<<<(T + 31) / 32, MERGE_WARPS * 32, 0, stream>>>(partial, label_logit, logprob, entropy, lse, T,
+                                                                     vb_lmhead_num_tiles(V));
   return static_cast<int>(cudaGetLastError());
 }
 
