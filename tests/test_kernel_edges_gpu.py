@@ -120,3 +120,34 @@ def test_sampler_takes_the_token_of_the_whole_row(ops, B, V, ld, valid, scale):
         assert ((score.max(-1).values - got)[plain] <= 1e-4 * (1 + score.max(-1).values.abs()[plain])).all()
         want = xt.gather(1, tok[:, None])[:, 0] - xt.logsumexp(-1)
         assert (lp.double() - want).abs().max() < 1e-4 * (1 + xt[xt > -math.inf].abs().max())
+
+
+# ------------------------------------------------------------------------------------------------ head and optimizer
+@pytest.mark.parametrize("T,V", [(1, 8), (31, 4096), (33, 4360), (130, 264)])
+def test_head_merges_its_tiles(ops, T, V):
+    from verl_b200.ops import functional as F
+
+    g = torch.Generator(device=DEV).manual_seed(T)
+    h = torch.randn(T, 64, device=DEV, generator=g).bfloat16()
+    w = (torch.randn(V, 64, device=DEV, generator=g) * 0.5).bfloat16()
+    lab = torch.randint(V, (T,), device=DEV, generator=g)
+    lp, ent, lse = F.lmhead_logprob_entropy(h, w, lab, 0.8)
+    logp = (h.double() @ w.double().T / 0.8).log_softmax(-1)
+    # fp32 logits of magnitude up to about 20: 1e-5 absolute; the kernel's exponentials are the fast ones
+    assert (lp - logp.gather(1, lab[:, None])[:, 0]).abs().max() < 1e-4
+    assert (ent + (logp.exp() * logp).sum(-1)).abs().max() < 2e-4
+
+
+@pytest.mark.parametrize("n,shift", [(1, 0), (3, 0), (4, 0), (1027, 0), (1030, 1)])
+def test_adamw_remainders_and_alignment(ops, n, shift):
+    g = torch.Generator(device=DEV).manual_seed(n)
+    rnd = lambda: torch.randn(n + shift, device=DEV, generator=g)[shift:]
+    p, gr, m, v = rnd(), rnd(), rnd() * 0.1, rnd().square()
+    out = torch.zeros(n + shift, device=DEV, dtype=torch.bfloat16)[shift:]
+    ctrl = torch.tensor([0.0, 0.5, 0.0, 0.0], device=DEV)
+    pd, gd, md, vd = (t.double() for t in (p, gr, m, v))
+    gd = gd * 0.5
+    md, vd = 0.9 * md + 0.1 * gd, 0.999 * vd + 0.001 * gd.square()
+    pd = pd * (1 - 1e-3 * 0.01) - 1e-3 * (md / (1 - 0.9**3)) / ((vd / (1 - 0.999**3)).sqrt() + 1e-8)
+    ops.adamw_(p, gr, m, v, out, ctrl, 1e-3, 0.9, 0.999, 1e-8, 0.01, 3, 1.0, True)
+    assert rel(p, pd) < 1e-6 and rel(m, md) < 1e-6 and rel(v, vd) < 1e-6 and torch.equal(out, p.bfloat16()) and not gr.any()

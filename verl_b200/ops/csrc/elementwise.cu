@@ -295,28 +295,59 @@ __global__ void clip_coef_kernel(float* __restrict__ ctrl, float max_norm) {
 
 // AdamW on a flat shard.  master (fp32) is updated in place; the bf16 working copy is refreshed in the
 // same pass; the gradient is optionally zeroed for the next accumulation round.
-__global__ void adamw_kernel(float* __restrict__ master, float* __restrict__ grad, float* __restrict__ m,
-                             float* __restrict__ v, __nv_bfloat16* __restrict__ out_bf16, long long n,
-                             const float* __restrict__ ctrl, float lr, float beta1, float beta2, float eps,
-                             float wd, float bc1, float bc2_sqrt, float grad_scale, int zero_grad) {
+struct AdamArgs {
+  float lr, beta1, beta2, eps, wd, bc1, bc2_sqrt;
+};
+__device__ __forceinline__ void adamw_one(float& p, float g, float& m, float& v, const AdamArgs& a) {
+  m = a.beta1 * m + (1.f - a.beta1) * g;
+  v = a.beta2 * v + (1.f - a.beta2) * g * g;
+  p *= (1.f - a.lr * a.wd);
+  const float denom = sqrtf(v) / a.bc2_sqrt + a.eps;
+  p -= (a.lr / a.bc1) * (m / denom);
+}
+// 30 bytes an element. VEC: 4 elements a thread in 16-byte accesses (every pointer 16-byte aligned, the bf16 copy 8; the remainder of n
+// goes to the last threads one by one): 2^28 elements in 1.18 ms (6.8 TB/s) instead of 1386 us with 4-byte accesses (5.8 TB/s).
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+adamw_kernel(float* __restrict__ master, float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v,
+             __nv_bfloat16* __restrict__ out_bf16, long long n, const float* __restrict__ ctrl, AdamArgs a, float grad_scale, int zero_grad) {
   const long long i = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  if (i >= n) return;
   const bool skip = ctrl && ctrl[2] != 0.f;
   const float coef = (ctrl ? ctrl[1] : 1.f) * grad_scale;
-  if (!skip) {
-    const float g = grad[i] * coef;
-    float p = master[i];
-    const float mi = beta1 * m[i] + (1.f - beta1) * g;
-    const float vi = beta2 * v[i] + (1.f - beta2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    p *= (1.f - lr * wd);
-    const float denom = sqrtf(vi) / bc2_sqrt + eps;
-    p -= (lr / bc1) * (mi / denom);
-    master[i] = p;
-    if (out_bf16) out_bf16[i] = __float2bfloat16(p);
+  const long long n4 = VEC ? n >> 2 : 0;
+  if (VEC && i < n4) {
+    if (!skip) {
+      const float4 g = reinterpret_cast<const float4*>(grad)[i];
+      float4 p = reinterpret_cast<const float4*>(master)[i], mi = reinterpret_cast<const float4*>(m)[i], vi = reinterpret_cast<const float4*>(v)[i];
+      adamw_one(p.x, g.x * coef, mi.x, vi.x, a);
+      adamw_one(p.y, g.y * coef, mi.y, vi.y, a);
+      adamw_one(p.z, g.z * coef, mi.z, vi.z, a);
+      adamw_one(p.w, g.w * coef, mi.w, vi.w, a);
+      reinterpret_cast<float4*>(m)[i] = mi;
+      reinterpret_cast<float4*>(v)[i] = vi;
+      reinterpret_cast<float4*>(master)[i] = p;
+      if (out_bf16) {
+        __nv_bfloat162 lo = __floats2bfloat162_rn(p.x, p.y), hi = __floats2bfloat162_rn(p.z, p.w);
+        uint2 o;
+        o.x = *reinterpret_cast<unsigned int*>(&lo);
+        o.y = *reinterpret_cast<unsigned int*>(&hi);
+        reinterpret_cast<uint2*>(out_bf16)[i] = o;
+      }
+    }
+    if (zero_grad) reinterpret_cast<float4*>(grad)[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    return;
   }
-  if (zero_grad) grad[i] = 0.f;
+  const long long e = VEC ? (n4 << 2) + (i - n4) : i;
+  if (e >= n) return;
+  if (!skip) {
+    float p = master[e], mi = m[e], vi = v[e];
+    adamw_one(p, grad[e] * coef, mi, vi, a);
+    m[e] = mi;
+    v[e] = vi;
+    master[e] = p;
+    if (out_bf16) out_bf16[e] = __float2bfloat16(p);
+  }
+  if (zero_grad) grad[e] = 0.f;
 }
 
 __global__ void cast_f32_bf16_kernel(const float* __restrict__ in, __nv_bfloat16* __restrict__ out, long long n,
@@ -441,8 +472,15 @@ int vb_adamw(float* master, float* grad, float* m, float* v, void* out_bf16, lon
   if (n == 0) return 0;
   const float bc1 = 1.f - powf(beta1, static_cast<float>(step));
   const float bc2s = sqrtf(1.f - powf(beta2, static_cast<float>(step)));
-  adamw_kernel<<<cdiv_ll(n, 256), 256, 0, s>>>(master, grad, m, v, reinterpret_cast<__nv_bfloat16*>(out_bf16), n, ctrl,
-                                               lr, beta1, beta2, eps, wd, bc1, bc2s, grad_scale, zero_grad);
+  const AdamArgs args{lr, beta1, beta2, eps, wd, bc1, bc2s};
+  const uintptr_t at = reinterpret_cast<uintptr_t>(master) | reinterpret_cast<uintptr_t>(grad) | reinterpret_cast<uintptr_t>(m) |
+                       reinterpret_cast<uintptr_t>(v) | (reinterpret_cast<uintptr_t>(out_bf16) << 1);
+  if (at % 16 == 0)
+    adamw_kernel<true><<<cdiv_ll((n >> 2) + (n & 3), 256), 256, 0, s>>>(master, grad, m, v, reinterpret_cast<__nv_bfloat16*>(out_bf16), n,
+                                                                       ctrl, args, grad_scale, zero_grad);
+  else
+    adamw_kernel<false><<<cdiv_ll(n, 256), 256, 0, s>>>(master, grad, m, v, reinterpret_cast<__nv_bfloat16*>(out_bf16), n, ctrl, args,
+                                                        grad_scale, zero_grad);
   return static_cast<int>(cudaGetLastError());
 }
 int vb_cast_f32_bf16(const float* in, void* out, long long n, float scale, cudaStream_t s) {
