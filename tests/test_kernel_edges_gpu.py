@@ -151,3 +151,128 @@ def test_adamw_remainders_and_alignment(ops, n, shift):
     pd = pd * (1 - 1e-3 * 0.01) - 1e-3 * (md / (1 - 0.9**3)) / ((vd / (1 - 0.999**3)).sqrt() + 1e-8)
     ops.adamw_(p, gr, m, v, out, ctrl, 1e-3, 0.9, 0.999, 1e-8, 0.01, 3, 1.0, True)
     assert rel(p, pd) < 1e-6 and rel(m, md) < 1e-6 and rel(v, vd) < 1e-6 and torch.equal(out, p.bfloat16()) and not gr.any()
+
+
+# ------------------------------------------------------------------------------------------------ attention
+def _attention64(q, k, v, keys_of, scale):
+    """fp64 attention of a packed stream; ``keys_of(t)`` = stream rows that query row t sees."""
+    T, nh, hd = q.shape
+    per = nh // k.shape[1]
+    see = torch.zeros(T, T, dtype=torch.bool, device=q.device)
+    for t in range(T):
+        see[t, keys_of[t]] = True
+    out = []
+    for h in range(nh):
+        s = (q[:, h] @ k[:, h // per].T * scale).masked_fill(~see, -math.inf)
+        out.append(s.softmax(-1) @ v[:, h // per])
+    return torch.stack(out, 1)
+
+
+@pytest.mark.parametrize("hd,nh,nkv", [(64, 14, 2), (128, 4, 4), (128, 7, 1)])
+@pytest.mark.parametrize("groups", [[(0, [1])], [(0, [63, 64, 65, 1, 200])], [(1, [1, 129]), (130, [128, 5, 64]), (0, [33])],
+                                    [(64, [1, 127]), (65, [2, 2]), (128, [130])]])
+def test_attention_of_prompts_and_their_continuations(ops, hd, nh, nkv, groups):
+    """(prompt length, response lengths) per group; a prompt of 0 stands for separate sequences. Both directions, rotary tables folded
+    into the backward pass, against fp64 over the same stream."""
+    from verl_b200.ops import functional as F
+
+    cu, parent, keys, pos = [0], [], [], []
+    for p, rs in groups:
+        if p:
+            base, prompt_seg = cu[-1], len(parent)
+            cu.append(base + p)
+            parent.append(-1)
+            keys += [list(range(base, base + i + 1)) for i in range(p)]
+            pos += list(range(p))
+        for r in rs:
+            a = cu[-1]
+            cu.append(a + r)
+            parent.append(prompt_seg if p else -1)
+            pre = list(range(base, base + p)) if p else []
+            keys += [pre + list(range(a, a + i + 1)) for i in range(r)]
+            pos += list(range(p, p + r))
+    T = cu[-1]
+    g = torch.Generator(device=DEV).manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    qkv, dout = rnd(T, (nh + 2 * nkv) * hd), rnd(T, nh, hd)
+    heads = lambda x: (x[:, : nh * hd].view(T, nh, hd), x[:, nh * hd : (nh + nkv) * hd].view(T, nkv, hd), x[:, (nh + nkv) * hd :].view(T, nkv, hd))
+    q, k, v = heads(qkv)
+    cu_t, par_t = torch.tensor(cu, dtype=torch.int32, device=DEV), torch.tensor(parent, dtype=torch.int32, device=DEV)
+    scale = hd**-0.5
+    longest = max(b - a for a, b in zip(cu, cu[1:]))
+    cos, sin = F.rope_table(512, hd, 1e4, DEV)
+    pos_t = torch.tensor(pos, dtype=torch.int32, device=DEV)
+    out, lse = F.attention_shared_prefix(q, k, v, cu_t, par_t)
+    ref = [t.double().requires_grad_(True) for t in (q, k, v)]
+    want = _attention64(*ref, keys, scale)
+    # bf16 inputs, bf16 probabilities (2^-9 each) and a bf16 result
+    assert rel(out, want.detach()) < 6e-3
+    want.backward(dout.double())
+    c, s = cos[pos_t.long()].double()[:, None], sin[pos_t.long()].double()[:, None]
+
+    def back(x):  # inverse rotation
+        a, b = x.chunk(2, -1)
+        return torch.cat([a * c + b * s, b * c - a * s], -1)
+
+    grads = torch.full_like(qkv, float("nan"))
+    dq, dk, dv = heads(grads)
+    F.attention_bwd_into_(dout, q, k, v, out, lse, cu_t, longest, dq, dk, dv, parent=par_t, rope=(pos_t, cos, sin))
+    # dS is rounded to bf16 and its terms cancel: about 1e-2
+    small = 1e-6 * float(dout.double().norm())  # (a single key: dQ and dK are zero)
+    for got, w in ((dq, back(ref[0].grad)), (dk, back(ref[1].grad)), (dv, ref[2].grad)):
+        assert float((got.double() - w).norm()) < 1.5e-2 * float(w.norm()) + small
+    if max(parent) < 0:
+        plain, plain_lse = F.attention_varlen(q, k, v, cu_t, longest)
+        assert torch.equal(plain, out) and torch.equal(plain_lse, lse)
+        for got, w in zip(F.attention_varlen_bwd(dout, q, k, v, out, lse, cu_t, longest), (r.grad for r in ref)):
+            assert float((got.double() - w).norm()) < 1.5e-2 * float(w.norm()) + small
+
+
+@pytest.mark.parametrize("preset,layers", [("qwen2.5-0.5b", 2), ("tiny-shared", 2)])
+def test_update_with_shared_prompts_equals_separate_rows(ops, preset, layers):
+    from verl_b200.models import DecoderModel, FlatParams
+    from verl_b200.models.config import ModelConfig, get_preset
+    from verl_b200.trainer.ppo.prefix_grouper_utils import pack_shared_prefix_batch
+    from verl_b200.workers.engine.native.engine import pack_padded_batch
+
+    cfg = get_preset(preset) if preset != "tiny-shared" else ModelConfig(
+        model_type="qwen3", vocab_size=512, hidden_size=256, intermediate_size=512, num_attention_heads=4, num_key_value_heads=2, head_dim=128)
+    cfg.num_hidden_layers = layers
+    plen, rlen, P, R = [70, 70, 70, 33, 5, 5], [1, 130, 64, 9, 77, 40], 80, 130
+    gids = [0, 0, 0, 1, 2, 2]
+    g = torch.Generator().manual_seed(1)
+    ids = torch.randint(3, 500, (6, P + R), generator=g)
+    for i in range(1, 6):
+        if gids[i] == gids[i - 1]:
+            ids[i, :P] = ids[i - 1, :P]
+    at = torch.arange(P + R)[None]
+    mask = ((at >= P - torch.tensor(plen)[:, None]) & (at < P + torch.tensor(rlen)[:, None])).long()
+    ids, mask = (ids * mask).to(DEV), mask.to(DEV)
+    w = torch.randn(sum(rlen), generator=g).to(DEV)
+    got = []
+    for shared in (True, False):
+        params = FlatParams(cfg, dtype=torch.bfloat16, device=DEV, with_main_grad=True)
+        params.init_weights(seed=3, std=0.05)
+        model = DecoderModel(cfg, params)
+        if shared:
+            batch, pos, lab, _ = pack_shared_prefix_batch(ids, mask, None, R, gids, plen, rlen)
+            lp, _ = model.forward_logprobs(batch, None, 1.0, positions=pos, position_labels=lab)
+        else:
+            batch, lab, index, valid = pack_padded_batch(ids, mask, None, R)
+            lp, _ = model.forward_logprobs(batch, lab, 1.0, positions=index[valid])
+        (lp * w).sum().backward()
+        got.append((lp.detach(), params.main_grad))
+    # the same numbers in another order of summation, rounded to bf16 in between; std 0.05 weights magnify it a little
+    assert (got[0][0] - got[1][0]).abs().max() < 0.1 and rel(got[0][1], got[1][1]) < 3e-2
+
+
+@pytest.mark.parametrize("T,N,ld", [(1, 1, 1), (63, 511, 511), (65, 513, 520), (130, 1026, 1031), (1000, 4608, 4608)])
+def test_column_sums(ops, T, N, ld):
+    from verl_b200.ops import functional as F
+
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x = torch.randn(T, ld, device=DEV, generator=g).bfloat16()[:, :N]
+    out = torch.randn(N, device=DEV, generator=g)
+    want = out.double() + x.double().sum(0)
+    F.colsum_add_(x, out)
+    assert (out - want).abs().max() < 1e-6 * (10 + T)

@@ -51,6 +51,12 @@ class PackedBatch:
     # every stream token back out of it.
     expand_index: Optional[torch.Tensor] = None
     collapse_index: Optional[torch.Tensor] = None
+    # The same structure as sequences of the stream itself: ``seg_cu`` [S+1] cuts it into prompts and responses, ``seg_parent`` [S] is
+    # the prompt that a response continues (-1: none), ``seg_max`` the longest piece. The native attention kernels run on this form
+    # and expand nothing.
+    seg_cu: Optional[torch.Tensor] = None
+    seg_parent: Optional[torch.Tensor] = None
+    seg_max: int = 0
 
     @property
     def num_tokens(self) -> int:
@@ -509,8 +515,7 @@ class DecoderModel:
             if S is not None:
                 S.update(q_pre=qp, k_pre=kp, rstd_q=rq, rstd_k=rk)
         pos = batch.positions if self.sp is None else batch.positions[self.sp.local_rows(batch.num_tokens, batch.positions.device)]
-        F.apply_rope_(q, pos, self._cos, self._sin)
-        F.apply_rope_(k, pos, self._cos, self._sin)
+        F.apply_rope_(qkv[:, : Q + KV].view(T, nh + nkv, hd), pos, self._cos, self._sin)  # q and k heads lie side by side
         if self.kv_hook is not None:
             self.kv_hook(layer_idx, k, v)
         native_ok = q.is_cuda and F._ATTN_IMPL["fwd"] is not None and hd in (64, 128)
@@ -533,6 +538,11 @@ class DecoderModel:
             attn2 = self.sp.heads_to_seq(attn_f.contiguous()).reshape(T, Q)
             if S is not None:
                 S.update(qkv=qkv, attn=attn2, lse=lse, sp_full=(qf, kf, vf, attn_f))
+        elif batch.seg_parent is not None and F.native_attention(q):
+            attn, lse = F.attention_shared_prefix(q, k, v, batch.seg_cu, batch.seg_parent)
+            attn2 = attn.reshape(T, Q)
+            if S is not None:
+                S.update(qkv=qkv, attn=attn2, lse=lse, segments=True)
         elif batch.expand_index is not None:
             ex = batch.expand_index
             qe, ke, ve = q.index_select(0, ex), k.index_select(0, ex), v.index_select(0, ex)
@@ -583,6 +593,15 @@ class DecoderModel:
         q = qkv[:, :Q].view(T, nh, hd)
         k = qkv[:, Q : Q + KV].view(T, nkv, hd)
         v = qkv[:, Q + KV :].view(T, nkv, hd)
+        if S.get("segments") or (self.sp is None and batch.expand_index is None and lse is not None and F.native_attention(q)):
+            # the kernels write the projection's gradient in place, rotated back
+            g_qkv = torch.empty_like(qkv)
+            seg = bool(S.get("segments"))
+            F.attention_bwd_into_(g_attn.view(T, nh, hd), q, k, v, attn2.view(T, nh, hd), lse, batch.seg_cu if seg else batch.cu_seqlens,
+                                  batch.seg_max if seg else batch.max_seqlen, g_qkv[:, :Q].view(T, nh, hd),
+                                  g_qkv[:, Q : Q + KV].view(T, nkv, hd), g_qkv[:, Q + KV :].view(T, nkv, hd),
+                                  parent=batch.seg_parent if seg else None, rope=(batch.positions, self._cos, self._sin))
+            return self._qkv_bwd(W, g_qkv, h1, S)
         cu = batch.cu_seqlens if q.is_cuda and F._ATTN_IMPL["bwd"] is not None and lse is not None else self._cu_cpu(batch)
         if isinstance(self.sp, ContextParallel):
             kf, vf, spans = S["cp_full"]
@@ -623,8 +642,15 @@ class DecoderModel:
         gk.copy_(dk)
         g_qkv[:, Q + KV :].view(T, nkv, hd).copy_(dv)
         pos = batch.positions if self.sp is None else batch.positions[self.sp.local_rows(batch.num_tokens, batch.positions.device)]
-        F.apply_rope_(gq, pos, self._cos, self._sin, backward=True)
-        F.apply_rope_(gk, pos, self._cos, self._sin, backward=True)
+        F.apply_rope_(g_qkv[:, : Q + KV].view(T, nh + nkv, hd), pos, self._cos, self._sin, backward=True)
+        return self._qkv_bwd(W, g_qkv, h1, S)
+
+    def _qkv_bwd(self, W, g_qkv, h1, S: dict):
+        """From the gradient of the rotated-back q, k and v to the gradient of the projection's input."""
+        cfg = self.cfg
+        T = g_qkv.shape[0]
+        nh, nkv, hd, Q, KV = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, cfg.q_size, cfg.kv_size
+        gq, gk = g_qkv[:, :Q].view(T, nh, hd), g_qkv[:, Q : Q + KV].view(T, nkv, hd)
         if cfg.qk_norm:
             wq, wk = W["self_attn.q_norm.weight"], W["self_attn.k_norm.weight"]
             dqp = F.rms_norm_bwd(gq.reshape(T * nh, hd).contiguous(), S["q_pre"], wq, S["rstd_q"], None,
@@ -642,7 +668,7 @@ class DecoderModel:
         self._wgrad(W["self_attn.qkv_proj.weight"], g_qkv, h1)
         b = W.get("self_attn.qkv_proj.bias")
         if b is not None and getattr(b, "main_grad", None) is not None:
-            b.main_grad.add_(g_qkv.float().sum(0))
+            F.colsum_add_(g_qkv, b.main_grad)
         return g_h1
 
     def _lin(self, W, name: str, x: torch.Tensor, S: Optional[dict] = None) -> torch.Tensor:

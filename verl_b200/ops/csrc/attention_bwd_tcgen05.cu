@@ -1,4 +1,4 @@
-// Causal GQA attention backward over packed (varlen) sequences on tcgen05 tensor cores (head_dim 128).
+// Causal GQA attention backward over packed (varlen) sequences on tcgen05 tensor cores (head_dim 64 and 128).
 //
 // One CTA = one (sequence, block of 128 keys, KV head). K and V of the block stay in shared memory and dK, dV stay in
 // TMEM for the whole CTA, which walks over every query head of the GQA group and every block of 64 queries at or
@@ -23,7 +23,17 @@
 //   warps 2..9  two threads per key row (32 of the step's 64 queries each): tcgen05.ld S^T / dP^T -> P^T, dS^T ->
 //               swizzled shared memory; drain dQ^T with coalesced red.add (lanes = 32 consecutive head-dim elements of
 //               one query); final dV (warps 2..5) / dK (warps 6..9) store
-// D[q] = sum_d dO[q,d] O[q,d] comes from a small pre-pass; dQ is accumulated in fp32 and converted afterwards.
+// D[q] = sum_d dO[q,d] O[q,d] comes from a small pre-pass; dQ, dK and dV leave in fp32 and a last pass turns them into the bf16 gradient
+// of the projection output, undoing the rotary embedding on the way (attn_bwd_finish_kernel).
+//
+// Head_dim 64: dQ^T has 64 rows, but the tensor core's M stays 128 (with M = 64 the rows would sit on half of the lanes of every warp):
+// A's second panel of 64 rows is the V tile, which lies right behind K in shared memory with the stride of a K panel, and the lanes
+// 64..127 of the result are never read. 4 of 24 MMAs of a step are spent on them.
+//
+// With `parent` (see attention_fwd_tcgen05.cu) a key block of a prompt has queries in several sequences. They are dealt to one CTA per
+// (key block, query sequence): blockIdx.y = s is sequence s against its own keys, num_seqs + s is sequence s against those of parent[s],
+// unmasked. dK / dV of a prompt, and only of a prompt, are then summed with fp32 atomics. One CTA per key block for all members would
+// need no atomics but leave the launch waiting for the few prompt blocks: 434 steps against 174 on average for two groups of five.
 #include "tcgen05_common.cuh"
 
 #include <math.h>
@@ -36,13 +46,13 @@ constexpr int AB_THREADS = 320;  // TMA warp, MMA warp, eight softmax warps
 
 struct AttnBwdParams {
   const int* cu_seqlens;
+  const int* parent;   // [num_seqs] or null
   int num_seqs, nh, nkv, total_tokens, max_tiles;  // max_tiles: key blocks of the longest sequence
   const float* lse;    // [nh, T] natural log
   const float* delta;  // [nh, T]
   float* dq32;         // [T, nh*hd] fp32, zero on entry
-  __nv_bfloat16* dk;   // [T, nkv*hd] (row stride lddk)
-  __nv_bfloat16* dv;
-  long long lddk, lddv;
+  float* dk32;         // [T, nkv*hd] fp32; zero on entry with `parent`
+  float* dv32;
   float scale, scale_log2;
   int* status;
 };
@@ -91,12 +101,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.x;
   const int G = p.nh / p.nkv;
-  const int seq_start = p.cu_seqlens[blockIdx.y];
-  const int seqlen = p.cu_seqlens[blockIdx.y + 1] - seq_start;
+  // query sequence, and the sequence of its keys: itself, or its parent
+  const bool cross = static_cast<int>(blockIdx.y) >= p.num_seqs;
+  const int qs = static_cast<int>(blockIdx.y) - (cross ? p.num_seqs : 0);
+  const int ks = cross ? p.parent[qs] : qs;
+  if (ks < 0 || ks >= p.num_seqs) return;  // no parent: uniform over the CTA, nothing allocated yet
+  const int seq_start = p.cu_seqlens[qs], seqlen = p.cu_seqlens[qs + 1] - seq_start;
+  const int key_start = p.cu_seqlens[ks], keylen = p.cu_seqlens[ks + 1] - key_start;
   const int from_end = p.max_tiles - 1 - static_cast<int>(blockIdx.z);
-  const int ntiles = (seqlen + AB_BK - 1) / AB_BK;
-  if (from_end >= ntiles) return;  // shorter sequence: uniform over the CTA, nothing allocated yet
+  const int ntiles = (keylen + AB_BK - 1) / AB_BK;
   if (ntiles > p.max_tiles && blockIdx.z == 0 && threadIdx.x == 0) atomicExch(p.status, ST_BAD_ARGS);  // max_seqlen too small
+  if (from_end >= ntiles || seqlen <= 0) return;  // shorter sequence
+  // dK / dV of this block are also written by CTAs of other query sequences
+  const bool shared_keys = cross || (p.parent != nullptr && ks + 1 < p.num_seqs && p.parent[ks + 1] == ks);
   const int k0 = (ntiles - 1 - from_end) * AB_BK;
 
   if (threadIdx.x == 0) {
@@ -122,7 +139,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  const int i0 = k0 / AB_BQ;                                    // first query block at or below the diagonal
+  const int i0 = cross ? 0 : k0 / AB_BQ;                        // first query block at or below the diagonal
   const int nqb = (seqlen + AB_BQ - 1) / AB_BQ;
   const int per_head = nqb - i0;
   const int n_it = per_head * G;
@@ -134,8 +151,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       mbar_expect_tx(kv_full, 2 * L::KV_BYTES);
 #pragma unroll
       for (int c = 0; c < PANELS; ++c) {
-        tma_load_2d(sK + c * (AB_BK * 128), &tm_k, kv_full, kvh * HD + 64 * c, seq_start + k0);
-        tma_load_2d(sV + c * (AB_BK * 128), &tm_v, kv_full, kvh * HD + 64 * c, seq_start + k0);
+        tma_load_2d(sK + c * (AB_BK * 128), &tm_k, kv_full, kvh * HD + 64 * c, key_start + k0);
+        tma_load_2d(sV + c * (AB_BK * 128), &tm_v, kv_full, kvh * HD + 64 * c, key_start + k0);
       }
       for (int it = 0; it < n_it; ++it) {
         const int st = it & 1;
@@ -158,7 +175,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (lane == 0 && n_it > 0) {
       constexpr uint32_t idesc_s = make_idesc_f16(AB_BK, AB_BQ, false, false);   // S^T, dP^T
       constexpr uint32_t idesc_kv = make_idesc_f16(AB_BK, HD, false, true);      // dV, dK
-      constexpr uint32_t idesc_dq = make_idesc_f16(HD, AB_BQ, true, true);       // dQ^T (M = hd = 128)
+      constexpr uint32_t idesc_dq = make_idesc_f16(128, AB_BQ, true, true);      // dQ^T (M = hd, padded to 128)
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aP = smem_u32(sP), aDS = smem_u32(sDS);
       auto issue_sdp = [&](int it) {
         const int st = it & 1;
@@ -223,6 +240,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     constexpr float LOG2E = 1.4426950408889634f;
 
     auto drain_dq = [&](int it) {
+      if (HD < 128 && q * 32 >= HD) return;  // lanes of the padding rows
       const int head = kvh * G + it / per_head;
       const int q0 = (i0 + it % per_head) * AB_BQ + cbase;
       const long long row_stride = static_cast<long long>(p.nh) * HD;
@@ -268,7 +286,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tmem_ld_32x32(tmem_base + TM_DP + cbase + lane_off, dp);
         tmem_ld_wait();
         // only the blocks on the diagonal and the last (partial) query block of the sequence need the mask
-        const bool masked = (q0 < k0 + AB_BK) || (q0 + AB_BQ > seqlen);
+        const bool masked = (!cross && q0 < k0 + AB_BK) || (q0 + AB_BQ > seqlen) || (cross && k0 + AB_BK > keylen);
         const float4* vL4 = reinterpret_cast<const float4*>(vL);
         const float4* vD4 = reinterpret_cast<const float4*>(vD);
 #pragma unroll
@@ -281,7 +299,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             float pe = exp2f(fmaf(__uint_as_float(s[c + u]), p.scale_log2, -lv[u]));
             if (masked) {
               const int qi = q0 + cbase + c + u;
-              if (!((key <= qi) && (qi < seqlen))) pe = 0.f;
+              if (!((cross ? key < keylen : key <= qi) && (qi < seqlen))) pe = 0.f;
             }
             pv[u] = pe;
             dsv[u] = pe * fmaf(__uint_as_float(dp[c + u]), p.scale, -dv_[u]);  // delta is stored pre-multiplied by scale
@@ -323,26 +341,23 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     } else {
       tc_fence_after();
       drain_dq(n_it - 1);
-      // dV (first four warps) and dK (last four) of this key block: exclusive to this CTA, plain stores; the TMEM loads
-      // are warp-wide, the stores are predicated on the key being inside the sequence
-      const bool key_ok = key < seqlen;
-      const long long tok = static_cast<long long>(seq_start) + key;
-      __nv_bfloat16* dst = (half == 0 ? p.dv + tok * p.lddv : p.dk + tok * p.lddk) + static_cast<long long>(kvh) * HD;
+      // dV (first four warps) and dK (last four) of this key block: exclusive to this CTA (plain stores) unless other sequences share
+      // the keys; the TMEM loads are warp-wide, the stores are predicated on the key being inside the sequence
+      const bool key_ok = key < keylen;
+      const long long tok = static_cast<long long>(key_start) + key;
+      float* dst = (half == 0 ? p.dv32 : p.dk32) + (tok * p.nkv + kvh) * HD;
 #pragma unroll 1
       for (int c = 0; c < HD / 32; ++c) {
         uint32_t o[32];
         tmem_ld_32x32(tmem_base + (half == 0 ? TM_DV : TM_DK) + c * 32 + lane_off, o);
         tmem_ld_wait();
-        if (key_ok) {
+        if (!key_ok) continue;
+        if (shared_keys) {
 #pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            uint4 v;
-            v.x = pack_bf16x2(__uint_as_float(o[i]), __uint_as_float(o[i + 1]));
-            v.y = pack_bf16x2(__uint_as_float(o[i + 2]), __uint_as_float(o[i + 3]));
-            v.z = pack_bf16x2(__uint_as_float(o[i + 4]), __uint_as_float(o[i + 5]));
-            v.w = pack_bf16x2(__uint_as_float(o[i + 6]), __uint_as_float(o[i + 7]));
-            *reinterpret_cast<uint4*>(dst + c * 32 + i) = v;
-          }
+          for (int i = 0; i < 32; ++i) atomicAdd(dst + c * 32 + i, __uint_as_float(o[i]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) *reinterpret_cast<uint4*>(dst + c * 32 + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
         }
       }
     }
@@ -356,39 +371,68 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   }
 }
 
-// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]; one warp per (token, head)
-__global__ void attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ dout, long long lddo,
-                                      const __nv_bfloat16* __restrict__ out, long long ldo, float* __restrict__ delta,
-                                      int T, int nh, int hd) {
-  const long long w = (blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (w >= static_cast<long long>(T) * nh) return;
-  const int t = static_cast<int>(w / nh), h = static_cast<int>(w % nh);
-  const __nv_bfloat16* a = dout + static_cast<long long>(t) * lddo + static_cast<long long>(h) * hd;
-  const __nv_bfloat16* b = out + static_cast<long long>(t) * ldo + static_cast<long long>(h) * hd;
+// delta[h, t] = sum_d dO[t, h, d] * O[t, h, d]; hd / 8 lanes per (token, head), 16 bytes each, so that a warp has 1 KB in flight
+__global__ void __launch_bounds__(256)
+attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ dout, long long lddo, const __nv_bfloat16* __restrict__ out, long long ldo,
+                      float* __restrict__ delta, int T, int nh, int hd) {
+  const int lanes = hd >> 3;
+  const long long i = blockIdx.x * 256LL + threadIdx.x;
+  const long long w = i / lanes;
+  const int l = static_cast<int>(i - w * lanes);
   float s = 0.f;
-  for (int d = lane * 2; d < hd; d += 64) {
-    const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(a + d));
-    const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(b + d));
-    s += x.x * y.x + x.y * y.y;
-  }
+  const bool ok = w < static_cast<long long>(T) * nh;
+  const int t = static_cast<int>(w / nh), h = static_cast<int>(w % nh);
+  if (ok) {
+    const uint4 a = *reinterpret_cast<const uint4*>(dout + static_cast<long long>(t) * lddo + h * hd + l * 8);
+    const uint4 b = *reinterpret_cast<const uint4*>(out + static_cast<long long>(t) * ldo + h * hd + l * 8);
+    const uint32_t av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (lane == 0) delta[static_cast<long long>(h) * T + t] = s;
+    for (int j = 0; j < 4; ++j) {
+      s = fmaf(__uint_as_float(av[j] << 16), __uint_as_float(bv[j] << 16), s);
+      s = fmaf(__uint_as_float(av[j] & 0xffff0000u), __uint_as_float(bv[j] & 0xffff0000u), s);
+    }
+  }
+  for (int o = lanes >> 1; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (ok && l == 0) delta[static_cast<long long>(h) * T + t] = s;
 }
 
-// dq (bf16, row stride lddq) = dq32 (fp32 [T, nh*hd])
-__global__ void attn_bwd_dq_cast_kernel(const float* __restrict__ dq32, __nv_bfloat16* __restrict__ dq, long long lddq,
-                                        int T, int width) {
-  const long long i4 = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-  const long long per_row = width / 4;
-  if (i4 >= static_cast<long long>(T) * per_row) return;
-  const long long t = i4 / per_row, c = (i4 % per_row) * 4;
-  const float4 v = *reinterpret_cast<const float4*>(dq32 + t * width + c);
-  uint2 o;
-  o.x = pack_bf16x2(v.x, v.y);
-  o.y = pack_bf16x2(v.z, v.w);
-  *reinterpret_cast<uint2*>(dq + t * lddq + c) = o;
+// bf16 gradients from the fp32 sums: heads 0 .. nh of dq32, then nkv heads of dk32, then of dv32. With cos_t the q and k heads are
+// rotated back by their token's position before they are rounded. Four pairs (d, d + hd / 2) per thread. One pass where the
+// projection output's gradient used to take seven (cast of dq, copies of dq, dk and dv, rotations of q and k in place).
+__global__ void __launch_bounds__(256)
+attn_bwd_finish_kernel(const float* __restrict__ dq32, const float* __restrict__ dk32, const float* __restrict__ dv32,
+                       __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv, long long lddq,
+                       long long lddk, long long lddv, const int* __restrict__ pos, const float* __restrict__ cos_t,
+                       const float* __restrict__ sin_t, int T, int nh, int nkv, int hd) {
+  const int half = hd >> 1, per_head = half >> 2, heads = nh + 2 * nkv;
+  const long long i = blockIdx.x * 256LL + threadIdx.x;
+  const long long item = i / per_head;
+  if (item >= static_cast<long long>(T) * heads) return;
+  const int d = static_cast<int>(i - item * per_head) * 4;
+  const long long t = item / heads;
+  const int h = static_cast<int>(item - t * heads);
+  const float* src;
+  __nv_bfloat16* dst;
+  if (h < nh) {
+    src = dq32 + (t * nh + h) * hd;
+    dst = dq + t * lddq + h * hd;
+  } else if (h < nh + nkv) {
+    src = dk32 + (t * nkv + h - nh) * hd;
+    dst = dk + t * lddk + (h - nh) * hd;
+  } else {
+    src = dv32 + (t * nkv + h - nh - nkv) * hd;
+    dst = dv + t * lddv + (h - nh - nkv) * hd;
+  }
+  float4 a = *reinterpret_cast<const float4*>(src + d), b = *reinterpret_cast<const float4*>(src + half + d);
+  if (cos_t != nullptr && h < nh + nkv) {
+    const long long o = static_cast<long long>(pos[t]) * half + d;
+    const float4 c = *reinterpret_cast<const float4*>(cos_t + o), sn = *reinterpret_cast<const float4*>(sin_t + o);
+    const float4 x = a, y = b;
+    a = make_float4(x.x * c.x + y.x * sn.x, x.y * c.y + y.y * sn.y, x.z * c.z + y.z * sn.z, x.w * c.w + y.w * sn.w);
+    b = make_float4(y.x * c.x - x.x * sn.x, y.y * c.y - x.y * sn.y, y.z * c.z - x.z * sn.z, y.w * c.w - x.w * sn.w);
+  }
+  *reinterpret_cast<uint2*>(dst + d) = make_uint2(pack_bf16x2(a.x, a.y), pack_bf16x2(a.z, a.w));
+  *reinterpret_cast<uint2*>(dst + half + d) = make_uint2(pack_bf16x2(b.x, b.y), pack_bf16x2(b.z, b.w));
 }
 
 __device__ int g_attn_bwd_status[4];
@@ -397,16 +441,36 @@ __device__ int g_attn_bwd_status[4];
 
 using namespace vb;
 
-// Workspace (caller-provided, any content): delta [nh*T] fp32 and dq32 [T*nh*hd] fp32 (zeroed here).
-// q/dout/out: [T, nh, hd] views, k/v: [T, nkv, hd] views; dq/dk/dv are written with their own row strides.
+namespace vb {
+template <int HD>
+static cudaError_t launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
+                                   const AttnBwdParams& p, cudaStream_t stream) {
+  auto kern = attn_bwd_kernel<HD>;
+  constexpr int smem = AttnBwdSmem<HD>::TOTAL;
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  const dim3 grid(p.nkv, p.num_seqs * (p.parent != nullptr ? 2 : 1), p.max_tiles);
+  kern<<<grid, AB_THREADS, smem, stream>>>(tq, tk, tv, tdo, p);
+  return cudaGetLastError();
+}
+}  // namespace vb
+
+// Workspaces (caller-provided, any content): delta [nh*T], dq32 [T*nh*hd], dkv32 [2*T*nkv*hd], all fp32.
+// q/dout/out: [T, nh, hd] views, k/v: [T, nkv, hd] views; dq/dk/dv are written with their own row strides. With pos / cos_t / sin_t
+// (tables [*, hd/2]) the gradients are those in front of the rotary embedding. max_seqlen: of the sequences as cu_seqlens cuts them.
 extern "C" int vb_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout, long long ldq,
                            long long ldk, long long ldv, long long ldo, long long lddo, const float* lse,
-                           const int* cu_seqlens, int num_seqs, int total_tokens, int nh, int nkv, int hd, float scale,
-                           void* dq, void* dk, void* dv, long long lddq, long long lddk, long long lddv, float* delta_ws,
-                           float* dq32_ws, int max_seqlen, cudaStream_t stream) {
+                           const int* cu_seqlens, const int* parent, int num_seqs, int total_tokens, int nh, int nkv, int hd, float scale,
+                           void* dq, void* dk, void* dv, long long lddq, long long lddk, long long lddv, const int* pos,
+                           const float* cos_t, const float* sin_t, float* delta_ws, float* dq32_ws, float* dkv32_ws, int max_seqlen,
+                           cudaStream_t stream) {
   if (total_tokens <= 0 || num_seqs <= 0) return 0;
-  if (max_seqlen <= 0 || num_seqs > 65535) return -4;
-  if (hd != 128) return -2;
+  if (max_seqlen <= 0 || num_seqs > (parent != nullptr ? 32767 : 65535)) return -4;
+  if (hd != 64 && hd != 128) return -2;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (ldo % 8) || (lddo % 8) || (lddq % 8) || (lddk % 8) || (lddv % 8) || (nh % nkv)) return -1;
   CUtensorMap tq, tk, tv, tdo;
   const auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -416,34 +480,27 @@ extern "C" int vb_attn_bwd(const void* q, const void* k, const void* v, const vo
   if (!make_tmap_2d(&tv, v, bf, 2, total_tokens, (uint64_t)nkv * hd, ldv, 64, AB_BK, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
   static int* status = nullptr;
   if (status == nullptr) cudaGetSymbolAddress(reinterpret_cast<void**>(&status), g_attn_bwd_status);
-  const long long warps = static_cast<long long>(total_tokens) * nh;
-  attn_bwd_delta_kernel<<<static_cast<int>((warps * 32 + 255) / 256), 256, 0, stream>>>(
+  const long long T = total_tokens, lanes = T * nh * (hd / 8);
+  attn_bwd_delta_kernel<<<static_cast<int>((lanes + 255) / 256), 256, 0, stream>>>(
       reinterpret_cast<const __nv_bfloat16*>(dout), lddo, reinterpret_cast<const __nv_bfloat16*>(out), ldo, delta_ws,
       total_tokens, nh, hd);
-  cudaError_t e = cudaMemsetAsync(dq32_ws, 0, sizeof(float) * static_cast<size_t>(total_tokens) * nh * hd, stream);
+  float* dk32 = dkv32_ws;
+  float* dv32 = dkv32_ws + T * nkv * hd;
+  cudaError_t e = cudaMemsetAsync(dq32_ws, 0, sizeof(float) * static_cast<size_t>(T) * nh * hd, stream);
+  if (e == cudaSuccess && parent != nullptr) e = cudaMemsetAsync(dkv32_ws, 0, sizeof(float) * 2 * static_cast<size_t>(T) * nkv * hd, stream);
   if (e != cudaSuccess) return static_cast<int>(e);
   AttnBwdParams p{};
-  p.cu_seqlens = cu_seqlens; p.num_seqs = num_seqs; p.nh = nh; p.nkv = nkv; p.total_tokens = total_tokens;
-  p.lse = lse; p.delta = delta_ws; p.dq32 = dq32_ws;
-  p.dk = reinterpret_cast<__nv_bfloat16*>(dk); p.dv = reinterpret_cast<__nv_bfloat16*>(dv);
-  p.lddk = lddk; p.lddv = lddv; p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
-  auto kern = attn_bwd_kernel<128>;
-  constexpr int smem = AttnBwdSmem<128>::TOTAL;
-  static bool configured = false;
-  if (!configured) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  p.cu_seqlens = cu_seqlens; p.parent = parent; p.num_seqs = num_seqs; p.nh = nh; p.nkv = nkv; p.total_tokens = total_tokens;
+  p.lse = lse; p.delta = delta_ws; p.dq32 = dq32_ws; p.dk32 = dk32; p.dv32 = dv32;
+  p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   p.max_tiles = (max_seqlen + AB_BK - 1) / AB_BK;
   if (p.max_tiles > 65535) return -4;
-  dim3 grid(nkv, num_seqs, p.max_tiles);
-  kern<<<grid, AB_THREADS, smem, stream>>>(tq, tk, tv, tdo, p);
-  e = cudaGetLastError();
+  e = hd == 128 ? launch_attn_bwd<128>(tq, tk, tv, tdo, p, stream) : launch_attn_bwd<64>(tq, tk, tv, tdo, p, stream);
   if (e != cudaSuccess) return static_cast<int>(e);
-  const long long n4 = static_cast<long long>(total_tokens) * nh * hd / 4;
-  attn_bwd_dq_cast_kernel<<<static_cast<int>((n4 + 255) / 256), 256, 0, stream>>>(
-      dq32_ws, reinterpret_cast<__nv_bfloat16*>(dq), lddq, total_tokens, nh * hd);
+  const long long n = T * (nh + 2 * nkv) * (hd / 8);
+  attn_bwd_finish_kernel<<<static_cast<int>((n + 255) / 256), 256, 0, stream>>>(
+      dq32_ws, dk32, dv32, reinterpret_cast<__nv_bfloat16*>(dq), reinterpret_cast<__nv_bfloat16*>(dk), reinterpret_cast<__nv_bfloat16*>(dv),
+      lddq, lddk, lddv, pos, cos_t, sin_t, total_tokens, nh, nkv, hd);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -9,6 +9,10 @@
 //               domain -> P (bf16) written to shared memory in the K-major 128B-swizzle layout the MMA reads;
 //               O in TMEM is rescaled (tcgen05.ld / tcgen05.st) only when some row maximum of the warp moved.
 // Epilogue: O / l -> bf16 [T, nh, hd]; LSE (natural log) -> [nh, T] for the backward pass.
+//
+// With `parent`, a sequence may be the continuation of another one (the responses of a group behind their shared prompt): its queries
+// see all keys of sequence parent[s] and then their own, causally. The key tiles of the prompt come straight from the prompt's rows of the
+// stream, so nothing is expanded to one copy per member and the prompt's own queries are computed once.
 #include "tcgen05_common.cuh"
 
 #include <math.h>
@@ -21,6 +25,7 @@ constexpr int ATT_THREADS = 192;
 
 struct AttnFwdParams {
   const int* cu_seqlens;  // [B+1]
+  const int* parent;      // [B] sequence whose keys come first, -1: none; null: none anywhere
   int num_seqs;
   int nh, nkv;
   __nv_bfloat16* out;  // [T, nh, hd]
@@ -69,7 +74,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint64_t* bar_p = bars + 7;      // 1
   uint64_t* bar_o = bars + 8;      // 1
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 9);
-  int* s_tile = reinterpret_cast<int*>(bars + 10);  // seq start token, q0, seqlen, valid
+  int* s_tile = reinterpret_cast<int*>(bars + 10);  // seq start token, q0, seqlen, valid, parent's start, parent's length
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.y;
@@ -77,18 +82,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   if (threadIdx.x == 0) {
     // locate (sequence, query block) of this CTA: tiles are enumerated sequence by sequence
-    int t = blockIdx.x, found = 0, start = 0, q0 = 0, len = 0;
+    int t = blockIdx.x, found = 0, start = 0, q0 = 0, len = 0, pstart = 0, plen = 0;
     for (int s = 0; s < p.num_seqs; ++s) {
       const int a = p.cu_seqlens[s], b = p.cu_seqlens[s + 1];
       const int nt = (b - a + ATT_BQ - 1) / ATT_BQ;
       if (t < nt) {
         // heavy (late) query blocks first: they have the most key blocks
         start = a; len = b - a; q0 = (nt - 1 - t) * ATT_BQ; found = 1;
+        const int pr = p.parent != nullptr ? p.parent[s] : -1;
+        if (pr >= 0 && pr < p.num_seqs) {
+          pstart = p.cu_seqlens[pr];
+          plen = p.cu_seqlens[pr + 1] - pstart;
+        }
         break;
       }
       t -= nt;
     }
-    s_tile[0] = start; s_tile[1] = q0; s_tile[2] = len; s_tile[3] = found;
+    s_tile[0] = start; s_tile[1] = q0; s_tile[2] = len; s_tile[3] = found; s_tile[4] = pstart; s_tile[5] = plen;
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
@@ -113,7 +123,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int seq_start = s_tile[0], q0 = s_tile[1], seqlen = s_tile[2];
   const bool valid_tile = s_tile[3] != 0;
   const int kv_end = min(q0 + ATT_BQ, seqlen);
-  const int nblk = valid_tile ? (kv_end + ATT_BKV - 1) / ATT_BKV : 0;
+  const int pstart = s_tile[4], plen = s_tile[5];
+  const int pblk = (plen + ATT_BKV - 1) / ATT_BKV;  // key blocks of the parent, in front of the own ones
+  const int nblk = valid_tile ? pblk + (kv_end + ATT_BKV - 1) / ATT_BKV : 0;
   constexpr uint32_t TM_S0 = 0, TM_O = 128;
 
   if (warp == 0) {
@@ -128,10 +140,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           break;
         }
         mbar_expect_tx(&kv_full[st], 2 * L::KV_BYTES);
+        const int krow = j < pblk ? pstart + j * ATT_BKV : seq_start + (j - pblk) * ATT_BKV;
 #pragma unroll
         for (int c = 0; c < PANELS; ++c) {
-          tma_load_2d(sK + st * L::KV_BYTES + c * (ATT_BKV * 128), &tm_k, &kv_full[st], kvh * HD + 64 * c, seq_start + j * ATT_BKV);
-          tma_load_2d(sV + st * L::KV_BYTES + c * (ATT_BKV * 128), &tm_v, &kv_full[st], kvh * HD + 64 * c, seq_start + j * ATT_BKV);
+          tma_load_2d(sK + st * L::KV_BYTES + c * (ATT_BKV * 128), &tm_k, &kv_full[st], kvh * HD + 64 * c, krow);
+          tma_load_2d(sV + st * L::KV_BYTES + c * (ATT_BKV * 128), &tm_v, &kv_full[st], kvh * HD + 64 * c, krow);
         }
       }
     }
@@ -188,15 +201,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       tmem_ld_32x32(tmem_base + TM_S0 + (j & 1) * ATT_BKV + lane_off, x0);
       tmem_ld_32x32(tmem_base + TM_S0 + (j & 1) * ATT_BKV + 32 + lane_off, x1);
       tmem_ld_wait();
-      const int col0 = j * ATT_BKV;
-      const bool need_mask = col0 + ATT_BKV - 1 > q0;  // block touches the diagonal of some row of the tile
+      // columns of this block that the row sees: the parent's keys up to its length, the own ones up to the diagonal
+      const int col0 = (j - pblk) * ATT_BKV;
+      const int limit = j < pblk ? plen - j * ATT_BKV : row - col0 + 1;
+      const bool need_mask = j < pblk ? limit < ATT_BKV : col0 + ATT_BKV - 1 > q0;
       float mx = -INFINITY;
 #pragma unroll
       for (int c = 0; c < 32; ++c) {
         float a = __uint_as_float(x0[c]) * p.scale_log2, b = __uint_as_float(x1[c]) * p.scale_log2;
         if (need_mask) {
-          if (col0 + c > row) a = -INFINITY;
-          if (col0 + 32 + c > row) b = -INFINITY;
+          if (c >= limit) a = -INFINITY;
+          if (32 + c >= limit) b = -INFINITY;
         }
         x0[c] = __float_as_uint(a);
         x1[c] = __float_as_uint(b);
@@ -310,8 +325,8 @@ using namespace vb;
 // q: [T, nh, hd] view (row stride ldq elements), k/v: [T, nkv, hd] views. max_seqlen bounds nothing here; the tile
 // count upper bound T/128 + num_seqs is used for the grid so no host copy of cu_seqlens is needed.
 extern "C" int vb_attn_fwd(const void* q, const void* k, const void* v, long long ldq, long long ldk, long long ldv,
-                           const int* cu_seqlens, int num_seqs, int total_tokens, int nh, int nkv, int hd, float scale,
-                           void* out, long long ldo, float* lse, cudaStream_t stream) {
+                           const int* cu_seqlens, const int* parent, int num_seqs, int total_tokens, int nh, int nkv, int hd,
+                           float scale, void* out, long long ldo, float* lse, cudaStream_t stream) {
   if (total_tokens <= 0 || num_seqs <= 0) return 0;
   if (hd != 64 && hd != 128) return -2;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (ldo % 8) || (nh % nkv)) return -1;
@@ -323,7 +338,7 @@ extern "C" int vb_attn_fwd(const void* q, const void* k, const void* v, long lon
   static int* status = nullptr;
   if (status == nullptr) cudaGetSymbolAddress(reinterpret_cast<void**>(&status), g_attn_status);
   AttnFwdParams p{};
-  p.cu_seqlens = cu_seqlens; p.num_seqs = num_seqs; p.nh = nh; p.nkv = nkv;
+  p.cu_seqlens = cu_seqlens; p.parent = parent; p.num_seqs = num_seqs; p.nh = nh; p.nkv = nkv;
   p.out = reinterpret_cast<__nv_bfloat16*>(out); p.ldo = ldo; p.lse = lse; p.total_tokens = total_tokens;
   p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   const int max_tiles = (total_tokens + ATT_BQ - 1) / ATT_BQ + num_seqs;

@@ -163,57 +163,87 @@ int64_t gemm_status() {
   return a != 0 ? a : (b != 0 ? 100 + b : (c != 0 ? 200 + c : 0));
 }
 
+// [T, heads, hd] view of bf16 rows with packed heads whose 16-byte pieces are aligned.
+void check_heads(const Tensor& t, const char* who) {
+  CHECK_BF16(t);
+  TORCH_CHECK(t.dim() == 3 && t.stride(2) == 1 && t.stride(1) == t.size(2), who, ": [T, heads, hd] views with packed heads");
+}
+// cu_seqlens int32 [B+1], parent int32 [B] (optional)
+const int* check_seqs(const Tensor& cu, const OptTensor& parent, const char* who) {
+  TORCH_CHECK(cu.is_cuda() && cu.scalar_type() == at::kInt && cu.is_contiguous(), who, ": cu_seqlens is a contiguous int32 CUDA tensor");
+  if (!parent.has_value()) return nullptr;
+  TORCH_CHECK(parent->is_cuda() && parent->scalar_type() == at::kInt && parent->is_contiguous() && parent->numel() == cu.numel() - 1, who,
+              ": parent is int32, one entry per sequence");
+  return parent->data_ptr<int>();
+}
+
 // Causal GQA attention over packed sequences. q [T, nh, hd], k/v [T, nkv, hd] (strided views), cu_seqlens int32 [B+1].
-// Returns (out [T, nh, hd] bf16, lse [nh, T] fp32).
+// parent (int32 [B], -1: none): the sequence whose keys a sequence's queries see in front of their own; it must have no parent itself,
+// and its children follow it directly. Returns (out [T, nh, hd] bf16, lse [nh, T] fp32).
 std::tuple<Tensor, Tensor> attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_seqlens,
-                                    double scale) {
-  CHECK_BF16(q);
-  CHECK_BF16(k);
-  CHECK_BF16(v);
-  TORCH_CHECK(q.dim() == 3 && k.dim() == 3 && q.stride(2) == 1 && q.stride(1) == q.size(2) && k.stride(1) == k.size(2) &&
-              v.stride(1) == v.size(2), "attn_fwd: [T, heads, hd] views with packed heads");
-  TORCH_CHECK(cu_seqlens.is_cuda() && cu_seqlens.scalar_type() == at::kInt && cu_seqlens.is_contiguous());
+                                    double scale, const OptTensor& parent) {
+  check_heads(q, "attn_fwd");
+  check_heads(k, "attn_fwd");
+  check_heads(v, "attn_fwd");
+  const int* pr = check_seqs(cu_seqlens, parent, "attn_fwd");
   const c10::cuda::CUDAGuard guard(q.device());
   const int64_t T = q.size(0), nh = q.size(1), hd = q.size(2), nkv = k.size(1);
   Tensor out = at::empty({T, nh, hd}, q.options());
   Tensor lse = at::empty({nh, T}, q.options().dtype(at::kFloat));
   count(1);
   const int rc = vb_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), q.stride(0), k.stride(0), v.stride(0),
-                             cu_seqlens.data_ptr<int>(), (int)cu_seqlens.numel() - 1, (int)T, (int)nh, (int)nkv, (int)hd,
+                             cu_seqlens.data_ptr<int>(), pr, (int)cu_seqlens.numel() - 1, (int)T, (int)nh, (int)nkv, (int)hd,
                              (float)scale, out.data_ptr(), out.stride(0), lse.data_ptr<float>(), cur_stream());
   CHECK_RC(rc, "vb_attn_fwd");
   return {out, lse};
+}
+
+// Gradients of attn_fwd into dq [T, nh, hd], dk / dv [T, nkv, hd] (strided views). With pos (int32 [T]) and the rotary tables the results
+// are the gradients in front of the rotary embedding of q and k. max_seqlen: longest sequence of cu_seqlens.
+void attn_bwd_into_(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& out, const Tensor& lse,
+                    const Tensor& cu_seqlens, int64_t max_seqlen, double scale, const OptTensor& parent, Tensor dq, Tensor dk, Tensor dv,
+                    const OptTensor& pos, const OptTensor& cos_t, const OptTensor& sin_t) {
+  for (const Tensor& t : {q, k, v, out, dout, dq, dk, dv}) check_heads(t, "attn_bwd");
+  CHECK_F32(lse);
+  TORCH_CHECK(lse.is_contiguous());
+  const int* pr = check_seqs(cu_seqlens, parent, "attn_bwd");
+  const c10::cuda::CUDAGuard guard(q.device());
+  const int64_t T = q.size(0), nh = q.size(1), hd = q.size(2), nkv = k.size(1);
+  TORCH_CHECK(dq.sizes() == q.sizes() && dk.sizes() == k.sizes() && dv.sizes() == k.sizes() && v.sizes() == k.sizes() &&
+              out.sizes() == q.sizes() && dout.sizes() == q.sizes(), "attn_bwd: shapes");
+  for (const Tensor& t : {dq, dk, dv, out, dout})
+    TORCH_CHECK(reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0, "attn_bwd: rows start on 16-byte boundaries");
+  if (pos.has_value()) {
+    TORCH_CHECK(cos_t.has_value() && sin_t.has_value() && pos->is_cuda() && pos->scalar_type() == at::kInt && pos->is_contiguous() &&
+                pos->numel() == T, "attn_bwd: pos is int32 [T]");
+    CHECK_F32((*cos_t));
+    CHECK_F32((*sin_t));
+    TORCH_CHECK(cos_t->is_contiguous() && sin_t->is_contiguous() && cos_t->size(-1) == hd / 2 && sin_t->size(-1) == hd / 2);
+  }
+  if (T == 0) return;
+  auto fo = q.options().dtype(at::kFloat);
+  Tensor delta = at::empty({nh, T}, fo);
+  Tensor dq32 = at::empty({T, nh * hd}, fo);
+  Tensor dkv32 = at::empty({2, T, nkv * hd}, fo);
+  count(3);
+  const int rc = vb_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(), q.stride(0), k.stride(0),
+                             v.stride(0), out.stride(0), dout.stride(0), lse.data_ptr<float>(), cu_seqlens.data_ptr<int>(), pr,
+                             (int)cu_seqlens.numel() - 1, (int)T, (int)nh, (int)nkv, (int)hd, (float)scale, dq.data_ptr(),
+                             dk.data_ptr(), dv.data_ptr(), dq.stride(0), dk.stride(0), dv.stride(0),
+                             pos.has_value() ? pos->data_ptr<int>() : nullptr, pos.has_value() ? cos_t->data_ptr<float>() : nullptr,
+                             pos.has_value() ? sin_t->data_ptr<float>() : nullptr, delta.data_ptr<float>(), dq32.data_ptr<float>(),
+                             dkv32.data_ptr<float>(), (int)max_seqlen, cur_stream());
+  CHECK_RC(rc, "vb_attn_bwd");
 }
 
 // (dq, dk, dv) of causal varlen GQA attention; q/out/dout: [T, nh, hd] views, k/v: [T, nkv, hd] views, lse [nh, T].
 std::tuple<Tensor, Tensor, Tensor> attn_bwd(const Tensor& dout, const Tensor& q, const Tensor& k, const Tensor& v,
                                             const Tensor& out, const Tensor& lse, const Tensor& cu_seqlens, int64_t max_seqlen,
                                             double scale) {
-  CHECK_BF16(q);
-  CHECK_BF16(k);
-  CHECK_BF16(v);
-  CHECK_BF16(out);
-  CHECK_BF16(dout);
-  CHECK_F32(lse);
-  auto packed = [](const Tensor& t) { return t.dim() == 3 && t.stride(2) == 1 && t.stride(1) == t.size(2); };
-  TORCH_CHECK(packed(q) && packed(k) && packed(v) && packed(out) && packed(dout), "attn_bwd: [T, heads, hd] views with packed heads");
-  TORCH_CHECK(cu_seqlens.is_cuda() && cu_seqlens.scalar_type() == at::kInt && cu_seqlens.is_contiguous() && lse.is_contiguous());
   const c10::cuda::CUDAGuard guard(q.device());
-  const int64_t T = q.size(0), nh = q.size(1), hd = q.size(2), nkv = k.size(1);
-  Tensor dq = at::empty({T, nh, hd}, q.options());
-  Tensor dk = at::empty({T, nkv, hd}, q.options());
-  Tensor dv = at::empty({T, nkv, hd}, q.options());
-  if (T == 0) return {dq, dk, dv};
-  auto fo = q.options().dtype(at::kFloat);
-  Tensor delta = at::empty({nh, T}, fo);
-  Tensor dq32 = at::empty({T, nh * hd}, fo);
-  count(4);
-  const int rc = vb_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(), q.stride(0), k.stride(0),
-                             v.stride(0), out.stride(0), dout.stride(0), lse.data_ptr<float>(), cu_seqlens.data_ptr<int>(),
-                             (int)cu_seqlens.numel() - 1, (int)T, (int)nh, (int)nkv, (int)hd, (float)scale, dq.data_ptr(),
-                             dk.data_ptr(), dv.data_ptr(), dq.stride(0), dk.stride(0), dv.stride(0), delta.data_ptr<float>(),
-                             dq32.data_ptr<float>(), (int)max_seqlen, cur_stream());
-  CHECK_RC(rc, "vb_attn_bwd");
+  Tensor dq = at::empty(q.sizes(), q.options()), dk = at::empty(k.sizes(), q.options()), dv = at::empty(k.sizes(), q.options());
+  const bool aligned = reinterpret_cast<uintptr_t>(out.data_ptr()) % 16 == 0;
+  attn_bwd_into_(dout, q, k, v, aligned ? out : out.clone(at::MemoryFormat::Contiguous), lse, cu_seqlens, max_seqlen, scale, c10::nullopt, dq, dk, dv, c10::nullopt, c10::nullopt, c10::nullopt);
   return {dq, dk, dv};
 }
 
@@ -329,6 +359,19 @@ void rope_kv_append_(Tensor qkv, const Tensor& pos, const Tensor& cos_t, const T
                              reinterpret_cast<long long*>(slot.data_ptr()), kc.data_ptr(), vc.data_ptr(), (int)qkv.size(0), (int)nh,
                              (int)nkv, (int)hd, cur_stream()),
            "vb_rope_kv_append");
+}
+
+// out[n] += sum over rows of x [T, N] bf16 (row stride ldx), fp32, in a fixed order.
+void colsum_add_(const Tensor& x, Tensor out) {
+  CHECK_BF16(x);
+  CHECK_F32(out);
+  TORCH_CHECK(x.dim() == 2 && x.stride(1) == 1 && out.is_contiguous() && out.numel() == x.size(1), "colsum_add_: x [T, N], out [N]");
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int64_t T = x.size(0), N = x.size(1);
+  if (T == 0 || N == 0) return;
+  Tensor part = at::empty({vb_colsum_chunks((int)T), N}, out.options());
+  count(2);
+  CHECK_RC(vb_colsum_add(x.data_ptr(), x.stride(0), (int)T, (int)N, part.data_ptr<float>(), out.data_ptr<float>(), cur_stream()), "vb_colsum_add");
 }
 
 Tensor swiglu_fwd(const Tensor& gu) {
@@ -1012,7 +1055,8 @@ TORCH_LIBRARY(verl_b200, m) {
   m.def("gemm_row_ranges_", &gemm_row_ranges_);
   m.def("launch_count", &launch_count);
   m.def("add_launches", &add_launches);
-  m.def("attn_fwd", &attn_fwd);
+  m.def("attn_fwd(Tensor q, Tensor k, Tensor v, Tensor cu_seqlens, float scale, Tensor? parent=None) -> (Tensor, Tensor)", &attn_fwd);
+  m.def("attn_bwd_into_", &attn_bwd_into_);
   m.def("attn_bwd", &attn_bwd);
   m.def("lmhead_fwd", &lmhead_fwd);
   m.def("lmhead_dlogits", &lmhead_dlogits);
@@ -1020,6 +1064,7 @@ TORCH_LIBRARY(verl_b200, m) {
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("rope_", &rope_);
   m.def("swiglu_fwd", &swiglu_fwd);
+  m.def("colsum_add_", &colsum_add_);
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("embedding_fwd", &embedding_fwd);
   m.def("embedding_bwd_", &embedding_bwd_);

@@ -201,6 +201,45 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict
       __floats2bfloat162_rn(b.x * c.x + a.x * s.x, b.y * c.y + a.y * s.y);
 }
 
+// ------------------------------------------------------------------------------------------ column sums
+// Gradient of a bias: sums over the rows of a bf16 matrix. A block sums COLSUM_ROWS rows of 512 columns (two neighbouring columns per
+// thread, 128 bytes per warp and row, eight rows in flight) into a plane of partial sums, a second launch folds the planes in order.
+// 7,900 x 4608 in 20 + 12 us; casting to fp32 first and reducing that took 42 + 69 us.
+constexpr int COLSUM_ROWS = 64;
+__global__ void __launch_bounds__(256)
+colsum_part_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, int T, int N, float* __restrict__ part) {
+  const int c = (blockIdx.x * 256 + threadIdx.x) * 2;
+  if (c >= N) return;
+  const int t0 = blockIdx.y * COLSUM_ROWS, t1 = min(T, t0 + COLSUM_ROWS);
+  float a = 0.f, b = 0.f;
+  const bool pair = c + 1 < N;
+  if (pair && ldx % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0) {
+#pragma unroll 8
+    for (int t = t0; t < t1; ++t) {
+      const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(x + t * ldx + c));
+      a += v.x;
+      b += v.y;
+    }
+  } else {
+    for (int t = t0; t < t1; ++t) {
+      a += __bfloat162float(x[t * ldx + c]);
+      if (pair) b += __bfloat162float(x[t * ldx + c + 1]);
+    }
+  }
+  float* o = part + static_cast<long long>(blockIdx.y) * N + c;
+  o[0] = a;
+  if (pair) o[1] = b;
+}
+__global__ void __launch_bounds__(128)
+colsum_fold_kernel(const float* __restrict__ part, int chunks, int N, float* __restrict__ out) {
+  const int c = blockIdx.x * 128 + threadIdx.x;
+  if (c >= N) return;
+  float s = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < chunks; ++k) s += part[static_cast<long long>(k) * N + c];
+  out[c] += s;
+}
+
 // ------------------------------------------------------------------------------------------ SwiGLU
 // gu [T, 2I]: gate = gu[:, :I], up = gu[:, I:].
 __global__ void swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restrict__ out,
@@ -421,6 +460,15 @@ int vb_rope(void* x, const int* pos, const float* cos_t, const float* sin_t, int
   const long long total = static_cast<long long>(T) * nheads * (hd / 4);
   rope_kernel<<<cdiv_ll(total, 256), 256, 0, s>>>(reinterpret_cast<__nv_bfloat16*>(x), pos, cos_t, sin_t, T, nheads,
                                                   hd, ld, backward ? -1.f : 1.f);
+  return static_cast<int>(cudaGetLastError());
+}
+
+int vb_colsum_chunks(int T) { return (T + COLSUM_ROWS - 1) / COLSUM_ROWS; }
+int vb_colsum_add(const void* x, long long ldx, int T, int N, float* part, float* out, cudaStream_t s) {
+  const int chunks = vb_colsum_chunks(T);
+  if (chunks > 65535) return -4;
+  colsum_part_kernel<<<dim3((N + 511) / 512, chunks), 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), ldx, T, N, part);
+  colsum_fold_kernel<<<(N + 127) / 128, 128, 0, s>>>(part, chunks, N, out);
   return static_cast<int>(cudaGetLastError());
 }
 

@@ -59,6 +59,8 @@ int vb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rs
                    float* dw, float* scratch, int T, int H, int accumulate_dw, cudaStream_t s);
 int vb_rope(void* x, const int* pos, const float* cos_t, const float* sin_t, int T, int nheads, int hd, long long ld,
             int backward, cudaStream_t s);
+int vb_colsum_chunks(int T);
+int vb_colsum_add(const void* x, long long ldx, int T, int N, float* part, float* out, cudaStream_t s);
 int vb_swiglu_fwd(const void* gu, void* out, long long T, int I, cudaStream_t s);
 int vb_swiglu_bwd(const void* dout, const void* gu, void* dgu, long long T, int I, cudaStream_t s);
 int vb_embedding_fwd(const long long* ids, const void* w, void* out, int T, int H, int V, cudaStream_t s);
@@ -87,14 +89,15 @@ int vb_sample_topkp(const void* logits, long long ld, int B, int V, int valid_vo
                     const long long* seeds, long long step, long long* tokens, float* logprobs, cudaStream_t s);
 // attention_fwd_tcgen05.cu
 int vb_attn_fwd(const void* q, const void* k, const void* v, long long ldq, long long ldk, long long ldv,
-                const int* cu_seqlens, int num_seqs, int total_tokens, int nh, int nkv, int hd, float scale, void* out,
-                long long ldo, float* lse, cudaStream_t stream);
+                const int* cu_seqlens, const int* parent, int num_seqs, int total_tokens, int nh, int nkv, int hd, float scale,
+                void* out, long long ldo, float* lse, cudaStream_t stream);
 int vb_attn_status();
 // attention_bwd_tcgen05.cu
 int vb_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout, long long ldq, long long ldk,
-                long long ldv, long long ldo, long long lddo, const float* lse, const int* cu_seqlens, int num_seqs,
-                int total_tokens, int nh, int nkv, int hd, float scale, void* dq, void* dk, void* dv, long long lddq,
-                long long lddk, long long lddv, float* delta_ws, float* dq32_ws, int max_seqlen, cudaStream_t stream);
+                long long ldv, long long ldo, long long lddo, const float* lse, const int* cu_seqlens, const int* parent, int num_seqs,
+                int total_tokens, int nh, int nkv, int hd, float scale, void* dq, void* dk, void* dv, long long lddq, long long lddk,
+                long long lddv, const int* pos, const float* cos_t, const float* sin_t, float* delta_ws, float* dq32_ws,
+                float* dkv32_ws, int max_seqlen, cudaStream_t stream);
 int vb_attn_bwd_status();
 // paged_decode_tma.cu
 int vb_paged_decode_v2(const void* q, long long ldq, const void* kc, const void* vc, long long num_slots,

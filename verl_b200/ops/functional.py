@@ -275,6 +275,14 @@ def gemm_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, want_gate_up: bool = F
     return swiglu(gu), (gu if want_gate_up else None)
 
 
+def colsum_add_(x: torch.Tensor, out: torch.Tensor) -> None:
+    """``out += x.sum(0)`` in fp32 (the gradient of a bias)."""
+    if x.is_cuda and x.dtype == torch.bfloat16:
+        _ops().colsum_add_(x, out)
+    else:
+        out.add_(x.float().sum(0))
+
+
 def swiglu_bwd(dout: torch.Tensor, gate_up: torch.Tensor) -> torch.Tensor:
     if gate_up.is_cuda:
         return _ops().swiglu_bwd(dout, gate_up)
@@ -446,7 +454,7 @@ def attention_varlen(q, k, v, cu_seqlens, max_seqlen: int, scale: Optional[float
 def attention_varlen_bwd(dout, q, k, v, out, lse, cu_seqlens, max_seqlen: int, scale: Optional[float] = None):
     """Returns (dq, dk, dv)."""
     scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
-    if q.is_cuda and _ATTN_IMPL["bwd"] is not None and lse is not None and q.shape[-1] == 128 and q.dtype == torch.bfloat16:
+    if q.is_cuda and _ATTN_IMPL["bwd"] is not None and lse is not None and q.shape[-1] in (64, 128) and q.dtype == torch.bfloat16:
         return _ATTN_IMPL["bwd"](dout, q, k, v, out, lse, cu_seqlens.to(q.device), max_seqlen, scale)
     import contextlib
 
@@ -459,6 +467,33 @@ def attention_varlen_bwd(dout, q, k, v, out, lse, cu_seqlens, max_seqlen: int, s
         q_, k_, v_ = (t.detach().requires_grad_(True) for t in (q, k, v))
         o = _sdpa_varlen(q_, k_, v_, cu_seqlens, scale)
         return torch.autograd.grad(o, (q_, k_, v_), dout)
+
+
+def native_attention(q: torch.Tensor) -> bool:
+    """Whether attention over ``q`` [T, heads, hd] runs on the tcgen05 kernels in both directions."""
+    return (q.is_cuda and q.dtype == torch.bfloat16 and q.shape[-1] in (64, 128) and _ATTN_IMPL["fwd"] is _native_attn_fwd
+            and _ATTN_IMPL["bwd"] is _native_attn_bwd)
+
+
+def attention_shared_prefix(q, k, v, cu_seqlens, parent, scale: Optional[float] = None):
+    """Causal GQA attention over a packed stream whose sequences may continue another one: the queries of sequence ``s`` see every
+    key of sequence ``parent[s]`` (-1: none) and then their own, causally. A parent has no parent itself and its children follow it
+    directly (a prompt and the responses of its group). Native kernels only (``native_attention``). Returns (out, lse)."""
+    scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
+    return _ops().attn_fwd(q, k, v, cu_seqlens, float(scale), parent)
+
+
+def attention_bwd_into_(dout, q, k, v, out, lse, cu_seqlens, max_seqlen: int, dq, dk, dv, parent=None, rope=None,
+                        scale: Optional[float] = None) -> None:
+    """Gradients of :func:`attention_varlen` / :func:`attention_shared_prefix` written into the views ``dq``, ``dk``, ``dv``; with
+    ``rope = (positions, cos table, sin table)`` those in front of the rotary embedding that produced ``q`` and ``k``. Native kernels
+    only; ``max_seqlen``: the longest sequence of ``cu_seqlens``."""
+    scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
+    pos, cos_t, sin_t = rope if rope is not None else (None, None, None)
+    if pos is not None:
+        audit.check_index("attention_bwd_into_", "positions", pos, cos_t.shape[0])
+        pos = pos.to(torch.int32).contiguous()
+    _ops().attn_bwd_into_(dout, q, k, v, out, lse, cu_seqlens.to(torch.int32), int(max_seqlen), float(scale), parent, dq, dk, dv, pos, cos_t, sin_t)
 
 
 def _attention_query_slice(q, k, v, cu_seqlens, q_start: int, scale: float):
@@ -679,8 +714,8 @@ def _native_attn_bwd(dout, q, k, v, out, lse, cu_seqlens, max_seqlen, scale):
     return _ops().attn_bwd(dout.contiguous(), q, k, v, out, lse, cu_seqlens.to(torch.int32), int(max_seqlen), float(scale))
 
 
-# On a GPU the tcgen05 kernels are the attention path: forward for head_dim 64 / 128, backward for head_dim 128 (other
-# head sizes differentiate through the reference formulation). VERL_B200_NATIVE_ATTN_BWD=0 keeps the backward off.
+# On a GPU the tcgen05 kernels are the attention path in both directions for head_dim 64 / 128 (other head sizes
+# differentiate through the reference formulation). VERL_B200_NATIVE_ATTN_BWD=0 keeps the backward off.
 import os as _os
 
 if torch.cuda.is_available():

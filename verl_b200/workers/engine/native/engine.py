@@ -156,6 +156,7 @@ def pack_shared_prefix_batch(input_ids: torch.Tensor, attention_mask: torch.Tens
         plen = mask[:, :P].sum(-1).tolist()
         rlen = mask[:, P:].sum(-1).tolist()
     src, expand, collapse, pos_sel, lab_src, lens_e = [], [], [], [], [], []
+    seg_cu, seg_parent = [0], []                       # the stream as prompts and their continuations (PackedBatch.seg_cu)
     t_d = t_e = 0
     i = 0
     while i < b:
@@ -167,6 +168,10 @@ def pack_shared_prefix_batch(input_ids: torch.Tensor, attention_mask: torch.Tens
         src.append((i * L + P - p, p))                 # the leader's prompt tokens
         collapse.append((t_e, p))                      # represented by the leader's copy
         t_d += p
+        prompt_seg = len(seg_parent)
+        if j > i:
+            seg_cu.append(t_d)
+            seg_parent.append(-1)
         for m in range(i, j + 1):
             r = int(rlen[m])
             src.append((m * L + P, r))
@@ -179,6 +184,8 @@ def pack_shared_prefix_batch(input_ids: torch.Tensor, attention_mask: torch.Tens
                 lab_src.append((m * L + P, r))
             lens_e.append(p + r)
             t_d += r
+            seg_cu.append(t_d)
+            seg_parent.append(prompt_seg if j > i else -1)  # a prompt with one response is one sequence
             t_e += p + r
         i = j + 1
     to_dev = lambda segs: torch.from_numpy(_ranges(segs)).to(dev, non_blocking=True)
@@ -191,8 +198,12 @@ def pack_shared_prefix_batch(input_ids: torch.Tensor, attention_mask: torch.Tens
         pos_full = position_ids.reshape(-1)
     cu = torch.zeros(len(lens_e) + 1, dtype=torch.int32)
     cu[1:] = torch.cumsum(torch.tensor(lens_e, dtype=torch.int32), 0)
-    batch = PackedBatch(input_ids=ids_d.contiguous(), positions=pos_full[src_t].to(torch.int32).contiguous(), cu_seqlens=cu.to(dev),
-                        max_seqlen=max(lens_e) if lens_e else 0, cu_seqlens_cpu=cu, expand_index=to_dev(expand), collapse_index=to_dev(collapse))
+    tables = torch.cat([cu, torch.tensor(seg_cu + seg_parent, dtype=torch.int32)]).to(dev, non_blocking=True)  # one copy for the three
+    n_cu, n_seg = cu.numel(), len(seg_cu)
+    batch = PackedBatch(input_ids=ids_d.contiguous(), positions=pos_full[src_t].to(torch.int32).contiguous(), cu_seqlens=tables[:n_cu],
+                        max_seqlen=max(lens_e) if lens_e else 0, cu_seqlens_cpu=cu, expand_index=to_dev(expand), collapse_index=to_dev(collapse),
+                        seg_cu=tables[n_cu : n_cu + n_seg], seg_parent=tables[n_cu + n_seg :],
+                        seg_max=max((b - a for a, b in zip(seg_cu, seg_cu[1:])), default=0))
     return batch, to_dev(pos_sel), flat_ids[lab_t].contiguous(), mask[:, P:]
 
 
