@@ -276,3 +276,129 @@ def test_column_sums(ops, T, N, ld):
     want = out.double() + x.double().sum(0)
     F.colsum_add_(x, out)
     assert (out - want).abs().max() < 1e-6 * (10 + T)
+
+
+# ------------------------------------------------------------------------------------------------ expert products on tiles of tokens
+def _choices(T, k, E, seed, skew=False):
+    """Distinct experts per token; with ``skew`` most tokens meet the first ones and some experts stay empty."""
+    g = torch.Generator().manual_seed(seed)
+    score = torch.rand(T, E, generator=g)
+    if skew:
+        score[:, :k] += 0.9
+        score[:, E // 2 + 1 :] -= 2.0
+    return score.topk(k, dim=-1).indices.cuda()
+
+
+@pytest.mark.parametrize("tile", [16, 32, 64, 128])
+@pytest.mark.parametrize("T,k,E,skew", [(1, 1, 1, False), (3, 2, 5, True), (32, 8, 128, False), (257, 4, 60, True), (2049, 8, 128, False),
+                                        (40, 2, 1024, False)])
+def test_expert_plan_is_the_stable_sort_by_expert(ops, tile, T, k, E, skew):
+    idx = _choices(T, k, E, T + E, skew)
+    counts = torch.bincount(idx.reshape(-1), minlength=E).int()
+    for choice in (idx, idx.int()):
+        slot, src, seg, te, num = ops.moe_plan(choice.contiguous(), counts, tile)
+        pad = (counts.long() + tile - 1) // tile * tile
+        first = pad.cumsum(0) - pad
+        assert seg.tolist() == [0] + pad.cumsum(0).tolist() and int(num) == int(pad.sum()) // tile
+        flat = idx.reshape(-1)
+        order = torch.argsort(flat, stable=True)
+        rank = torch.arange(T * k, device=DEV) - (counts.long().cumsum(0) - counts.long())[flat[order]]
+        want = torch.empty_like(flat)
+        want[order] = first[flat[order]] + rank
+        assert torch.equal(slot.reshape(-1).long(), want)
+        rows = torch.full_like(src, -1)
+        rows[want] = (torch.arange(T * k, device=DEV) // k).int()
+        assert torch.equal(src, rows)
+        used = int(num)
+        assert torch.equal(te[:used].long(), torch.repeat_interleave(torch.arange(E, device=DEV), pad // tile))
+        assert src.numel() % tile == 0 and used <= te.numel()
+
+
+@pytest.mark.parametrize("tile", [16, 32, 64, 128])
+@pytest.mark.parametrize("T,k,E,N,K", [(1, 1, 1, 8, 128), (33, 3, 7, 136, 256), (70, 4, 9, 384, 1152), (300, 2, 4, 128, 384)])
+def test_grouped_tiles_match_the_product_per_expert(ops, tile, T, k, E, N, K):
+    """bf16 operands: products are exact in fp32, so the bound is the rounding of the result (2^-9) and of fp32 sums of K terms.
+    fp8: the same for the dequantised operands."""
+    from verl_b200.ops import functional as F
+
+    idx = _choices(T, k, E, N + K)
+    counts = torch.bincount(idx.reshape(-1), minlength=E).int()
+    slot, src, seg, te, num = ops.moe_plan(idx.contiguous(), counts, tile)
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, K, generator=g).cuda().bfloat16()
+    w = (torch.randn(E, N, K, generator=g) * 0.05).cuda().bfloat16()
+    xp = ops.moe_gather_tiles(x, src, None, num, tile)
+    rows = slot.reshape(-1).long()
+    tok, exp = torch.arange(T * k, device=DEV) // k, idx.reshape(-1)
+    assert torch.equal(xp[rows], x[tok])
+    y = ops.gemm_grouped_tiles(xp, w, te, num, tile)[rows].double()
+    want = torch.einsum("rk,rnk->rn", x[tok].double(), w[exp].double())
+    size = torch.einsum("rk,rnk->rn", x[tok].double().abs(), w[exp].double().abs())
+    assert ((y - want).abs() <= want.abs() * 2.0**-8 + size * K * 2.0**-24).all()
+    xq, xs = F.fp8_quantize_1x128(xp)
+    xd = F.fp8_dequantize_1x128(xq, xs).double()[rows]
+    wq, ws = F.fp8_quantize_1x128(w.reshape(E * N, K))
+    wd = F.fp8_dequantize_1x128(wq, ws).view(E, N, K).double()
+    want, size = torch.einsum("rk,rnk->rn", xd, wd[exp]), torch.einsum("rk,rnk->rn", xd.abs(), wd[exp].abs())
+    if tile == 128:
+        y = ops.gemm_fp8_blockscale_grouped(xq, xs, wq, ws, N, te, num)[rows].double()
+        assert ((y - want).abs() <= want.abs() * 2.0**-8 + size * K * 2.0**-24).all()
+    if N % 128 == 0 and K % 128 == 0:  # the whole expert: gate, up of width N / 2 and back
+        I = N // 2 if (N // 2) % 128 == 0 else N
+        wgu = (torch.randn(E, 2 * I, K, generator=g) * 0.05).cuda().bfloat16()
+        wdn = (torch.randn(E, K, I, generator=g) * 0.05).cuda().bfloat16()
+        a, b = F.fp8_quantize_1x128(wgu.reshape(-1, K)), F.fp8_quantize_1x128(wdn.reshape(-1, I))
+        y = ops.moe_experts_fp8(x, src, a[0], a[1], b[0], b[1], I, te, num, tile)[rows]
+        gu = torch.einsum("rk,rnk->rn", xd, F.fp8_dequantize_1x128(*a).view(E, 2 * I, K).double()[exp]).bfloat16()
+        act = F.swiglu(gu.contiguous())
+        ad = F.fp8_dequantize_1x128(*F.fp8_quantize_1x128(act)).double()
+        want = torch.einsum("rk,rnk->rn", ad, F.fp8_dequantize_1x128(*b).view(E, K, I).double()[exp])
+        # a gate or up value rounded the other way moves an e4m3 activation by up to 2^-3 of itself: a few per row
+        assert float((y.double() - want).norm() / want.norm()) < 0.02
+    assert int(ops.gemm_status()) == 0
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 32, 33, 64, 65, 129, 300])
+def test_fp8_block_scaled_product_over_token_tiles(ops, M):
+    from verl_b200.ops import functional as F
+
+    N, K = 200, 384
+    g = torch.Generator().manual_seed(M)
+    x, w = torch.randn(M, K, generator=g).cuda().bfloat16(), torch.randn(N, K, generator=g).cuda().bfloat16()
+    bias = torch.randn(N, generator=g).cuda().bfloat16()
+    xq, xs = F.fp8_quantize_1x128(x)
+    wq, ws = F.fp8_quantize_1x128(w)
+    y = ops.gemm_fp8_blockscale(xq, xs, wq, ws, bias).double()
+    xd, wd = F.fp8_dequantize_1x128(xq, xs).double(), F.fp8_dequantize_1x128(wq, ws).double()
+    want = xd @ wd.T + bias.double()
+    assert ((y - want).abs() <= want.abs() * 2.0**-8 + (xd.abs() @ wd.abs().T) * K * 2.0**-24).all()
+
+
+@pytest.mark.parametrize("T,nh,nkv,hd", [(1, 1, 1, 64), (5, 4, 2, 128), (33, 3, 1, 256), (70, 8, 8, 96), (2000, 8, 2, 128)])
+def test_qk_norm_rotation_and_append_in_one(ops, T, nh, nkv, hd):
+    """The bits of the separate kernels."""
+    from verl_b200.ops import functional as F
+
+    g = torch.Generator().manual_seed(T + hd)
+    qkv = torch.randn(T, (nh + 2 * nkv) * hd, generator=g).cuda().bfloat16()
+    wq, wk = (1 + 0.1 * torch.randn(2, hd, generator=g)).cuda().bfloat16()
+    cos, sin = F.rope_table(128, hd, 1e4, DEV)
+    pos = torch.randint(0, 128, (T,), generator=g).int().cuda()
+    slots = torch.randperm(3 * T + 4, generator=g)[:T].cuda()
+    slots[0] = -1 if T > 1 else slots[0]
+    kc, vc = torch.zeros(2, (3 * T + 5) // 2 + 1, 2, nkv, hd, device=DEV, dtype=torch.bfloat16)
+    kr, vr = kc.clone(), vc.clone()
+    ref = qkv.clone()
+    q, k, v = (t.view(T, -1, hd) for t in ref.split([nh * hd, nkv * hd, nkv * hd], -1))
+    qp, kp = q.reshape(-1, hd).clone(), k.reshape(-1, hd).clone()
+    qn, _, rq = F.rms_norm(qp, wq, 1e-6)
+    kn, _, rk = F.rms_norm(kp, wk, 1e-6)
+    q.copy_(qn.view_as(q))
+    k.copy_(kn.view_as(k))
+    F.apply_rope_(q, pos, cos, sin)
+    F.apply_rope_(k, pos, cos, sin)
+    F.kv_append_(k, v, slots, kr, vr)
+    saved = F.qk_norm_rope_(qkv, pos, cos, sin, wq, wk, 1e-6, nh, nkv, hd, slots, kc, vc, save=True)
+    assert torch.equal(saved[0], qp) and torch.equal(saved[1], kp)
+    assert torch.equal(saved[2], rq) and torch.equal(saved[3], rk)
+    assert int((qkv != ref).sum()) == 0 and torch.equal(kc, kr) and torch.equal(vc, vr)

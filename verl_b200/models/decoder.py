@@ -506,16 +506,14 @@ class DecoderModel:
         q = qkv[:, :Q].view(T, nh, hd)
         k = qkv[:, Q : Q + KV].view(T, nkv, hd)
         v = qkv[:, Q + KV :].view(T, nkv, hd)
-        if cfg.qk_norm:
-            qp, kp = q.reshape(T * nh, hd).contiguous(), k.reshape(T * nkv, hd).contiguous()
-            qn, _, rq = F.rms_norm(qp, W["self_attn.q_norm.weight"], cfg.rms_norm_eps)
-            kn, _, rk = F.rms_norm(kp, W["self_attn.k_norm.weight"], cfg.rms_norm_eps)
-            q.copy_(qn.view(T, nh, hd))
-            k.copy_(kn.view(T, nkv, hd))
-            if S is not None:
-                S.update(q_pre=qp, k_pre=kp, rstd_q=rq, rstd_k=rk)
         pos = batch.positions if self.sp is None else batch.positions[self.sp.local_rows(batch.num_tokens, batch.positions.device)]
-        F.apply_rope_(qkv[:, : Q + KV].view(T, nh + nkv, hd), pos, self._cos, self._sin)  # q and k heads lie side by side
+        if cfg.qk_norm:
+            saved = F.qk_norm_rope_(qkv, pos, self._cos, self._sin, W["self_attn.q_norm.weight"], W["self_attn.k_norm.weight"],
+                                    cfg.rms_norm_eps, nh, nkv, hd, save=S is not None)
+            if S is not None:
+                S.update(q_pre=saved[0], k_pre=saved[1], rstd_q=saved[2], rstd_k=saved[3])
+        else:
+            F.apply_rope_(qkv[:, : Q + KV].view(T, nh + nkv, hd), pos, self._cos, self._sin)  # q and k heads lie side by side
         if self.kv_hook is not None:
             self.kv_hook(layer_idx, k, v)
         native_ok = q.is_cuda and F._ATTN_IMPL["fwd"] is not None and hd in (64, 128)
@@ -784,7 +782,7 @@ class DecoderModel:
         return w, idx
 
     def _routing(self, logits: torch.Tensor):
-        """(weights fp32 [T, k], experts int64 [T, k], per-expert counts) with record / replay of the choice."""
+        """(weights fp32 [T, k], experts int32 or int64 [T, k], per-expert counts) with record / replay of the choice."""
         cfg, rr = self.cfg, self.router_replay
         E, k = cfg.num_experts, cfg.num_experts_per_tok
         if rr is not None and rr.mode == "replay":
@@ -792,7 +790,6 @@ class DecoderModel:
             return w, idx, torch.bincount(idx.reshape(-1), minlength=E).int()
         if logits.is_cuda and logits.dtype == torch.bfloat16 and E <= 1024:
             w, idx, counts = F._ops().moe_route_topk(logits, k, bool(cfg.norm_topk_prob))
-            idx = idx.long()
         else:
             w, idx = self._route(logits)
             counts = torch.bincount(idx.reshape(-1), minlength=E).int()
@@ -802,27 +799,19 @@ class DecoderModel:
 
     # -- device path: router, expert-grouped layout and grouped tcgen05 GEMMs; no host synchronisation anywhere --------
     @staticmethod
-    def _moe_plan(idx: torch.Tensor, counts: torch.Tensor, T: int, k: int, E: int) -> dict:
-        """Expert-grouped row layout in which every expert's rows start at a multiple of 128 (padding rows are zero).
+    def _moe_plan(idx: torch.Tensor, counts: torch.Tensor, T: int, k: int, E: int, tile: int = 128) -> dict:
+        """Expert-grouped row layout in which every expert's rows start at a multiple of ``tile`` (padding rows are zero).
         ``slot[t, j]`` = row of the j-th expert copy of token t; ``src[row]`` = source token or -1 for padding."""
-        dev = idx.device
-        flat_e = idx.reshape(-1).long()
-        order = torch.argsort(flat_e, stable=True)
-        cnt = counts.long()
-        seg = torch.zeros(E + 1, dtype=torch.int64, device=dev)
-        seg[1:] = ((cnt + 127) // 128 * 128).cumsum(0)
-        first = cnt.cumsum(0) - cnt
-        e_sorted = flat_e[order]
-        slot_sorted = seg[e_sorted] + (torch.arange(T * k, device=dev) - first[e_sorted])
-        cap = ((T * k + 127) // 128 + E) * 128  # upper bound of the padded row count, known without reading `counts`
-        slot = torch.empty(T * k, dtype=torch.int32, device=dev)
-        slot[order] = slot_sorted.int()
-        src = torch.full((cap,), -1, dtype=torch.int32, device=dev)
-        src[slot_sorted] = torch.div(order, k, rounding_mode="floor").int()
-        tiles = torch.arange(cap // 128, device=dev) * 128
-        tile_expert = torch.searchsorted(seg[1:].contiguous(), tiles, right=True).clamp_(max=E - 1).int()
-        return dict(slot=slot.view(T, k), src=src, seg=seg.int(), tile_expert=tile_expert,
-                    num_mtiles=(seg[E:] // 128).int(), cap=cap)
+        slot, src, seg, tile_expert, num = F._ops().moe_plan(idx.reshape(T, k).contiguous(), counts.int().contiguous(), tile)
+        return dict(slot=slot, src=src, seg=seg, tile_expert=tile_expert, num_mtiles=num, cap=src.numel(), tile=tile)
+
+    @staticmethod
+    def _moe_tile(choices: int, experts: int) -> int:
+        """Rows per tile of a forward-only pass. Decode steps have a few rows per expert: a tile that holds about twice the mean reads
+        an expert's weights once and pads little. From 64 rows per expert on the products are bound by the tensor cores and run on
+        tiles of 128."""
+        mean = choices / experts
+        return 16 if mean <= 8 else 32 if mean <= 16 else 64 if mean <= 32 else 128
 
     def _moe_fwd_native(self, W, h2, S: Optional[dict]):
         cfg = self.cfg
@@ -832,17 +821,23 @@ class DecoderModel:
         logits = F.gemm(h2, W["mlp.gate.weight"])
         w, idx, counts = self._routing(logits)
         w = w.float().contiguous()
-        plan = self._moe_plan(idx, counts, T, k, E)
-        xp = ops.moe_gather_rows(h2, plan["src"], None)
+        tile = 128 if S is not None else self._moe_tile(T * k, E)
+        plan = self._moe_plan(idx, counts, T, k, E, tile)
+        te, nt = plan["tile_expert"], plan["num_mtiles"]
         Wgu, Wd = W["mlp.experts.gate_up_proj"], W["mlp.experts.down_proj"]
         q_gu = self.fp8_weights.get(Wgu.data_ptr()) if (S is None and self.fp8_weights is not None) else None
         q_d = self.fp8_weights.get(Wd.data_ptr()) if (S is None and self.fp8_weights is not None) else None
         if q_gu is not None and q_d is not None:  # forward-only with fp8 expert copies installed (rollout precision)
-            gu = F.linear_fp8_grouped(xp, q_gu[0], q_gu[1], Wgu.shape[1], plan["tile_expert"], plan["num_mtiles"])
-            y = F.linear_fp8_grouped(F.swiglu(gu), q_d[0], q_d[1], Wd.shape[1], plan["tile_expert"], plan["num_mtiles"])
+            gu = None
+            y = ops.moe_experts_fp8(h2, plan["src"], q_gu[0], q_gu[1], q_d[0], q_d[1], Wd.shape[2], te, nt, tile)
+        elif tile < 128:
+            xp = ops.moe_gather_tiles(h2, plan["src"], None, nt, tile)
+            gu = ops.gemm_grouped_tiles(xp, Wgu, te, nt, tile)
+            y = ops.gemm_grouped_tiles(ops.moe_swiglu(gu, nt, tile), Wd, te, nt, tile)
         else:
-            gu = ops.gemm_grouped_rows(xp, Wgu, False, plan["tile_expert"], plan["num_mtiles"])
-            y = ops.gemm_grouped_rows(F.swiglu(gu), Wd, False, plan["tile_expert"], plan["num_mtiles"])
+            xp = ops.moe_gather_tiles(h2, plan["src"], None, nt, tile)
+            gu = ops.gemm_grouped_rows(xp, Wgu, False, te, nt)
+            y = ops.gemm_grouped_rows(ops.moe_swiglu(gu, nt, tile), Wd, False, te, nt)
         out = ops.moe_combine(y, plan["slot"], w)
         if S is not None:
             S.update(moe=dict(native=True, logits=logits, w=w, idx=idx, plan=plan, gu=gu, y=y))
@@ -859,16 +854,16 @@ class DecoderModel:
         g_w = self._etp_sum(ops.moe_combine_bwd_w(g_d, y, plan["slot"]))   # y holds this rank's part of every expert output
         w_rows = torch.zeros(plan["cap"], dtype=torch.float32, device=h2.device)
         w_rows[plan["slot"].reshape(-1).long()] = w.reshape(-1)
-        g_y = ops.moe_gather_rows(g_d, plan["src"], w_rows)
+        g_y = ops.moe_gather_tiles(g_d, plan["src"], w_rows, plan["num_mtiles"], plan["tile"])
         Wgu, Wd = W["mlp.experts.gate_up_proj"], W["mlp.experts.down_proj"]
-        act = F.swiglu(gu)
+        act = ops.moe_swiglu(gu, plan["num_mtiles"], plan["tile"])
         g_act = ops.gemm_grouped_rows(g_y, Wd, True, plan["tile_expert"], plan["num_mtiles"])
         if getattr(Wd, "main_grad", None) is not None:
             ops.gemm_grouped_wgrad_(g_y, act, Wd.main_grad, plan["seg"], True)
         g_gu = F.swiglu_bwd(g_act, gu)
         g_xp = ops.gemm_grouped_rows(g_gu, Wgu, True, plan["tile_expert"], plan["num_mtiles"])
         if getattr(Wgu, "main_grad", None) is not None:
-            xp = ops.moe_gather_rows(h2, plan["src"], None)
+            xp = ops.moe_gather_tiles(h2, plan["src"], None, plan["num_mtiles"], plan["tile"])
             ops.gemm_grouped_wgrad_(g_gu, xp, Wgu.main_grad, plan["seg"], True)
         g_h2 = self._etp_sum(ops.moe_combine(g_xp, plan["slot"], None).float())
         with torch.enable_grad():
@@ -884,6 +879,10 @@ class DecoderModel:
         c = self.cfg
         return (h2.is_cuda and h2.dtype == torch.bfloat16 and c.num_experts <= 1024 and c.hidden_size % 64 == 0
                 and c.moe_intermediate_size % 64 == 0 and os.environ.get("VERL_B200_MOE_NATIVE", "1") != "0")
+
+    def decode_capturable(self) -> bool:
+        """Whether a decode step of this model can be captured: the expert layers must take the path without host reads."""
+        return not self.cfg.is_moe or (self.ep is None and self.etp_sum is None and self._moe_native_ok(self.params["embed_tokens.weight"]))
 
     # -- expert-parallel path: token copies travel to the owner of their expert and back -------------------------------
     def _experts_apply(self, W, x, counts: list, S: Optional[dict]):

@@ -361,6 +361,43 @@ void rope_kv_append_(Tensor qkv, const Tensor& pos, const Tensor& cos_t, const T
            "vb_rope_kv_append");
 }
 
+// Norm of every q and k head and rotary embedding in place; with slot / kc / vc also the append to the cache. save: returns the heads in
+// front of the norm and their 1 / rms (q [T * nh, hd], k [T * nkv, hd], fp32 [T * nh], [T * nkv]), else nothing.
+std::vector<Tensor> qk_norm_rope_(Tensor qkv, const Tensor& pos, const Tensor& cos_t, const Tensor& sin_t, const Tensor& wq, const Tensor& wk,
+                                  double eps, int64_t nh, int64_t nkv, int64_t hd, const OptTensor& slot, const OptTensor& kc, const OptTensor& vc,
+                                  bool save) {
+  CHECK_BF16(qkv);
+  CHECK_BF16(wq);
+  CHECK_BF16(wk);
+  CHECK_F32(cos_t);
+  CHECK_F32(sin_t);
+  const int64_t T = qkv.size(0);
+  TORCH_CHECK(qkv.dim() == 2 && qkv.stride(1) == 1 && qkv.size(1) == (nh + 2 * nkv) * hd, "qk_norm_rope: qkv [T, (nh + 2 nkv) * hd]");
+  TORCH_CHECK(pos.scalar_type() == at::kInt && pos.is_cuda() && pos.is_contiguous() && pos.numel() == T && wq.numel() == hd && wk.numel() == hd &&
+              wq.is_contiguous() && wk.is_contiguous() && cos_t.is_contiguous() && sin_t.is_contiguous() && cos_t.size(-1) == hd / 2);
+  const long long* sp = nullptr;
+  if (slot.has_value()) {
+    TORCH_CHECK(kc.has_value() && vc.has_value() && slot->scalar_type() == at::kLong && slot->is_contiguous() && slot->numel() == T);
+    CHECK_BF16((*kc));
+    CHECK_BF16((*vc));
+    TORCH_CHECK(kc->is_contiguous() && vc->is_contiguous() && kc->dim() == 4 && kc->size(2) == nkv && kc->size(3) == hd && kc->sizes() == vc->sizes());
+    sp = reinterpret_cast<const long long*>(slot->data_ptr());
+  }
+  const c10::cuda::CUDAGuard guard(qkv.device());
+  std::vector<Tensor> out;
+  if (save)
+    out = {at::empty({T * nh, hd}, qkv.options()), at::empty({T * nkv, hd}, qkv.options()), at::empty({T * nh}, cos_t.options()),
+           at::empty({T * nkv}, cos_t.options())};
+  if (T == 0) return out;
+  count(1);
+  CHECK_RC(vb_qk_norm_rope(qkv.data_ptr(), qkv.stride(0), pos.data_ptr<int>(), cos_t.data_ptr<float>(), sin_t.data_ptr<float>(), wq.data_ptr(),
+                           wk.data_ptr(), (float)eps, sp, sp ? kc->data_ptr() : nullptr, sp ? vc->data_ptr() : nullptr,
+                           save ? out[0].data_ptr() : nullptr, save ? out[1].data_ptr() : nullptr, save ? out[2].data_ptr<float>() : nullptr,
+                           save ? out[3].data_ptr<float>() : nullptr, (int)T, (int)nh, (int)nkv, (int)hd, cur_stream()),
+           "vb_qk_norm_rope");
+  return out;
+}
+
 // out[n] += sum over rows of x [T, N] bf16 (row stride ldx), fp32, in a fixed order.
 void colsum_add_(const Tensor& x, Tensor out) {
   CHECK_BF16(x);
@@ -870,10 +907,103 @@ Tensor gemm_fp8_blockscale_grouped(const Tensor& aq, const Tensor& sa, const Ten
   Tensor d = at::zeros({rows, N}, aq.options().dtype(at::kBFloat16));
   count(1);
   CHECK_RC(vb_gemm_fp8_blockscale_grouped(aq.data_ptr(), sa.data_ptr<float>(), bq.data_ptr(), sb.data_ptr<float>(), d.data_ptr(), (int)rows,
-                                          (int)N, (int)K, (int)(EN / N), aq.stride(0), bq.stride(0), d.stride(0),
+                                          (int)N, (int)K, (int)(EN / N), aq.stride(0), bq.stride(0), d.stride(0), 128,
                                           tile_expert.data_ptr<int>(), num_mtiles.data_ptr<int>(), cur_stream()),
            "vb_gemm_fp8_blockscale_grouped");
   return d;
+}
+
+// ---- expert products on tiles of 16, 32, 64 or 128 rows. Rows of tiles that are not in use are neither read nor written (undefined).
+void check_tiles(const Tensor& tile_expert, const Tensor& num_mtiles, int64_t rows, int64_t tile_rows) {
+  TORCH_CHECK(tile_rows == 16 || tile_rows == 32 || tile_rows == 64 || tile_rows == 128, "tile_rows must be 16, 32, 64 or 128");
+  TORCH_CHECK(rows % tile_rows == 0 && tile_expert.scalar_type() == at::kInt && tile_expert.is_cuda() && tile_expert.is_contiguous() &&
+                  tile_expert.numel() >= rows / tile_rows && num_mtiles.scalar_type() == at::kInt && num_mtiles.is_cuda() && num_mtiles.numel() >= 1,
+              "rows in whole tiles, tile_expert int32 with an entry per tile, num_mtiles int32");
+}
+
+// silu(x W_gate^T) * (x W_up^T) W_down^T in block-scaled fp8 for rows x[src] grouped by expert; wgu [E * 2 I, H], wd [E * H, I].
+Tensor moe_experts_fp8(const Tensor& x, const Tensor& src, const Tensor& wgu, const Tensor& sgu, const Tensor& wd, const Tensor& sd, int64_t I,
+                       const Tensor& tile_expert, const Tensor& num_mtiles, int64_t tile_rows) {
+  CHECK_BF16(x);
+  CHECK_F32(sgu);
+  CHECK_F32(sd);
+  const int64_t H = x.size(1), rows = src.numel();
+  TORCH_CHECK(x.dim() == 2 && x.stride(1) == 1 && x.stride(0) % 4 == 0 && src.scalar_type() == at::kInt && src.is_cuda() && src.is_contiguous());
+  TORCH_CHECK(wgu.scalar_type() == at::kByte && wd.scalar_type() == at::kByte && wgu.is_contiguous() && wd.is_contiguous() && I > 0 &&
+                  wgu.dim() == 2 && wd.dim() == 2 && wgu.size(1) == H && wd.size(1) == I && wgu.size(0) % (2 * I) == 0 &&
+                  wd.size(0) == wgu.size(0) / (2 * I) * H && H % 128 == 0 && I % 128 == 0, "moe_experts_fp8: [E * 2 I, H] and [E * H, I] e4m3");
+  TORCH_CHECK(sgu.is_contiguous() && sd.is_contiguous() && sgu.numel() == H / 128 * wgu.size(0) && sd.numel() == I / 128 * wd.size(0));
+  check_tiles(tile_expert, num_mtiles, rows, tile_rows);
+  const c10::cuda::CUDAGuard guard(x.device());
+  const int E = (int)(wd.size(0) / H);
+  const auto bytes = x.options().dtype(at::kByte), f32 = x.options().dtype(at::kFloat);
+  Tensor xq = at::empty({rows, H}, bytes), xs = at::empty({H / 128, rows}, f32), gu = at::empty({rows, 2 * I}, x.options());
+  Tensor aq = at::empty({rows, I}, bytes), as = at::empty({I / 128, rows}, f32), y = at::empty({rows, H}, x.options());
+  if (rows == 0) return y;
+  const int* te = tile_expert.data_ptr<int>();
+  const int* nt = num_mtiles.data_ptr<int>();
+  count(4);
+  CHECK_RC(vb_moe_gather_quant(x.data_ptr(), x.stride(0), src.data_ptr<int>(), xq.data_ptr(), xs.data_ptr<float>(), (int)rows, (int)H, nt,
+                               (int)tile_rows, cur_stream()), "vb_moe_gather_quant");
+  CHECK_RC(vb_gemm_fp8_blockscale_grouped(xq.data_ptr(), xs.data_ptr<float>(), wgu.data_ptr(), sgu.data_ptr<float>(), gu.data_ptr(), (int)rows,
+                                          (int)(2 * I), (int)H, E, H, H, 2 * I, (int)tile_rows, te, nt, cur_stream()), "vb_gemm_fp8_blockscale_grouped");
+  CHECK_RC(vb_moe_swiglu_quant(gu.data_ptr(), aq.data_ptr(), as.data_ptr<float>(), (int)rows, (int)I, nt, (int)tile_rows, cur_stream()),
+           "vb_moe_swiglu_quant");
+  CHECK_RC(vb_gemm_fp8_blockscale_grouped(aq.data_ptr(), as.data_ptr<float>(), wd.data_ptr(), sd.data_ptr<float>(), y.data_ptr(), (int)rows, (int)H,
+                                          (int)I, E, I, I, H, (int)tile_rows, te, nt, cur_stream()), "vb_gemm_fp8_blockscale_grouped");
+  return y;
+}
+
+// a [rows, K] bf16 grouped by expert in tiles of tile_rows rows, w [E, N, K]: rows of expert e times w[e]^T.
+Tensor gemm_grouped_tiles(const Tensor& a, const Tensor& w, const Tensor& tile_expert, const Tensor& num_mtiles, int64_t tile_rows) {
+  CHECK_BF16(a);
+  CHECK_BF16(w);
+  TORCH_CHECK(a.dim() == 2 && a.stride(1) == 1 && w.dim() == 3 && w.is_contiguous() && w.size(2) == a.size(1), "gemm_grouped_tiles: [rows, K], [E, N, K]");
+  check_tiles(tile_expert, num_mtiles, a.size(0), tile_rows);
+  const c10::cuda::CUDAGuard guard(a.device());
+  const int64_t rows = a.size(0), K = a.size(1), E = w.size(0), N = w.size(1);
+  Tensor d = at::empty({rows, N}, a.options());
+  if (rows == 0) return d;
+  count(1);
+  CHECK_RC(vb_gemm_bf16_grouped_tiles(a.data_ptr(), w.data_ptr(), d.data_ptr(), (int)rows, (int)N, (int)K, (int)E, a.stride(0), K, N,
+                                      (int)tile_rows, tile_expert.data_ptr<int>(), num_mtiles.data_ptr<int>(), cur_stream()),
+           "vb_gemm_bf16_grouped_tiles");
+  return d;
+}
+
+// (slot int32 [T, k], src int32 [cap], seg int32 [E + 1], tile_expert int32 [cap / tile], num_mtiles int32 [1]) of choices [T, k]
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> moe_plan(const Tensor& experts, const Tensor& counts, int64_t tile) {
+  TORCH_CHECK(experts.is_cuda() && experts.dim() == 2 && experts.is_contiguous() && (experts.scalar_type() == at::kInt || experts.scalar_type() == at::kLong));
+  TORCH_CHECK(counts.scalar_type() == at::kInt && counts.is_cuda() && counts.is_contiguous() && counts.numel() >= 1 && counts.numel() <= 1024 && tile > 0);
+  const c10::cuda::CUDAGuard guard(experts.device());
+  const int64_t n = experts.numel(), k = experts.size(1), E = counts.numel();
+  TORCH_CHECK(n < (int64_t(1) << 30), "moe_plan: too many choices");
+  const int64_t cap = ((n + tile - 1) / tile + std::min(E, n)) * tile;
+  const auto opt = counts.options();
+  Tensor slot = at::empty({experts.size(0), k}, opt), src = at::empty({cap}, opt), seg = at::empty({E + 1}, opt);
+  Tensor tile_expert = at::empty({cap / tile}, opt), num = at::empty({1}, opt);
+  if (n == 0) {
+    seg.zero_();
+    num.zero_();
+    return {slot, src, seg, tile_expert, num};
+  }
+  count(1);
+  CHECK_RC(vb_moe_plan(experts.data_ptr(), experts.scalar_type() == at::kLong, counts.data_ptr<int>(), (int)n, (int)k, (int)E, (int)tile, (int)cap,
+                       slot.data_ptr<int>(), src.data_ptr<int>(), seg.data_ptr<int>(), tile_expert.data_ptr<int>(), num.data_ptr<int>(), cur_stream()),
+           "vb_moe_plan");
+  return {slot, src, seg, tile_expert, num};
+}
+
+// silu(gate) * up of gu [rows, 2 I], rows of the tiles in use
+Tensor moe_swiglu(const Tensor& gu, const Tensor& num_mtiles, int64_t tile_rows) {
+  CHECK_BF16(gu);
+  TORCH_CHECK(gu.is_contiguous() && gu.dim() == 2 && num_mtiles.scalar_type() == at::kInt && num_mtiles.is_cuda() && num_mtiles.numel() >= 1);
+  const c10::cuda::CUDAGuard guard(gu.device());
+  Tensor out = at::empty({gu.size(0), gu.size(1) / 2}, gu.options());
+  count(1);
+  CHECK_RC(vb_moe_swiglu(gu.data_ptr(), out.data_ptr(), (int)gu.size(0), (int)(gu.size(1) / 2), num_mtiles.data_ptr<int>(), (int)tile_rows,
+                         cur_stream()), "vb_moe_swiglu");
+  return out;
 }
 
 // ---- mixture of experts
@@ -892,8 +1022,8 @@ std::tuple<Tensor, Tensor, Tensor> moe_route_topk(const Tensor& logits, int64_t 
   return {w, idx, counts};
 }
 
-// dst[r] = src[map[r]] (* scale[r]) or zeros where map[r] < 0
-Tensor moe_gather_rows(const Tensor& src, const Tensor& map, const OptTensor& scale) {
+// dst[r] = src[map[r]] (* scale[r]) or zeros where map[r] < 0; with num_mtiles only the rows of the tiles in use
+Tensor moe_gather_tiles(const Tensor& src, const Tensor& map, const OptTensor& scale, const OptTensor& num_mtiles, int64_t tile_rows) {
   CHECK_BF16(src);
   TORCH_CHECK(src.dim() == 2 && src.stride(1) == 1 && map.scalar_type() == at::kInt && map.is_contiguous() && map.is_cuda());
   const c10::cuda::CUDAGuard guard(src.device());
@@ -905,9 +1035,17 @@ Tensor moe_gather_rows(const Tensor& src, const Tensor& map, const OptTensor& sc
     sc = scale->data_ptr<float>();
   }
   count(1);
+  const int* nt = nullptr;
+  if (num_mtiles.has_value()) {
+    TORCH_CHECK(num_mtiles->scalar_type() == at::kInt && num_mtiles->is_cuda() && num_mtiles->numel() >= 1);
+    nt = num_mtiles->data_ptr<int>();
+  }
   CHECK_RC(vb_moe_gather_rows(src.data_ptr(), src.stride(0), map.data_ptr<int>(), sc, dst.data_ptr(), dst.stride(0), (int)rows,
-                              (int)H, cur_stream()), "vb_moe_gather_rows");
+                              (int)H, nt, (int)tile_rows, cur_stream()), "vb_moe_gather_rows");
   return dst;
+}
+Tensor moe_gather_rows(const Tensor& src, const Tensor& map, const OptTensor& scale) {
+  return moe_gather_tiles(src, map, scale, c10::nullopt, 0);
 }
 
 // out[t] = sum_j w[t,j] * y[slot[t,j]]   (w optional: plain sum)
@@ -1042,6 +1180,11 @@ TORCH_LIBRARY(verl_b200, m) {
   m.def("gemm_fp8_blockscale", &gemm_fp8_blockscale);
   m.def("moe_route_topk", &moe_route_topk);
   m.def("moe_gather_rows", &moe_gather_rows);
+  m.def("moe_gather_tiles", &moe_gather_tiles);
+  m.def("moe_experts_fp8", &moe_experts_fp8);
+  m.def("gemm_grouped_tiles", &gemm_grouped_tiles);
+  m.def("moe_plan", &moe_plan);
+  m.def("moe_swiglu", &moe_swiglu);
   m.def("moe_combine", &moe_combine);
   m.def("moe_combine_bwd_w", &moe_combine_bwd_w);
   m.def("moe_dispatch_peer_", &moe_dispatch_peer_);
@@ -1077,6 +1220,7 @@ TORCH_LIBRARY(verl_b200, m) {
   m.def("paged_decode", &paged_decode);
   m.def("paged_decode_grouped", &paged_decode_grouped);
   m.def("rope_kv_append_", &rope_kv_append_);
+  m.def("qk_norm_rope_", &qk_norm_rope_);
   m.def("sample", &sample);
   m.def("sample_topkp", &sample_topkp);
   m.def("grpo_advantage", &grpo_advantage);

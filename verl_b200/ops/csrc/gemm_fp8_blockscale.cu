@@ -1,16 +1,25 @@
-// fp8 (e4m3) GEMM with 1x128 block scaling on both operands, and the quantiser that produces such operands.
+// GEMMs whose rows come in tiles of 16 to 128 tokens: fp8 (e4m3) with 1x128 block scaling on both operands, plain or grouped by expert,
+// and the bf16 product of a mixture-of-experts layer with few tokens per expert. Also the quantisers that produce fp8 operands.
 //
-//   D[M,N] (bf16) = sum over 128-wide K blocks kb of  sa[kb, m] * sb[kb, n] * ( Aq[m, kb] . Bq[n, kb] )
+//   fp8:  D[m, n] (bf16) = sum over 128-wide K blocks kb of  sx[kb, m] * sw[kb, n] * ( Xq[m, kb] . Wq[n, kb] )
+//   bf16: D[m, n] (bf16) = X[m, :] . W[n, :]
 //
-// Aq [M, K], Bq [N, K] are e4m3, K-major, K % 128 == 0. Scales are fp32 and stored block-major: sa [K/128, M],
-// sb [K/128, N], so the 128 scales a tile needs for one K block are contiguous.
+// Xq [M, K], Wq [N, K] are e4m3, K-major, K % 128 == 0. Scales are fp32 and stored block-major: sx [K/128, M], sw [K/128, N].
 //
-// One CTA per 128 x 128 output tile:
-//   warp 0      TMA: A and B tiles of one K block (128 rows x 128 bytes, 128B swizzle) through a 4-stage ring
-//   warp 1      MMA: four tcgen05.mma kind::f8f6f4 (K = 32 each) per K block into one of two TMEM buffers (fresh
-//               accumulation per block, because the block's scale factors differ per row and column)
-//   warps 2..5  thread == output row: tcgen05.ld the block's 128 partial sums, multiply by sa[m] * sb[n], accumulate in
-//               registers; after the last block store the row as bf16
+// The product is computed transposed: 128 weight rows are the M axis of the MMA, a tile of R = 16, 32, 64 or 128 tokens its N axis. A
+// decode step of a mixture-of-experts layer (32 tokens, 8 of 128 experts each) has about two tokens per expert and is bound by reading
+// the weights of ~110 experts once; tiles of 128 tokens made it pad, write, quantise and read 60 times the rows. A persistent grid
+// walks over (token tile, weight tile) with one ring of 6 to 10 stages, so that the loads of the next tile run under the end of the
+// last one. The scales of a stage travel with its operands (cp.async into the same stage, counted on the same barrier): fetched by the
+// epilogue when it needed them they were a serial chain of one memory latency per K block.
+// A decode step of Qwen3-30B-A3B, 32 tokens, fp8: the two products of a layer's experts (523 MB of weights) 103 us (5.1 TB/s); they and
+// the two dense projections together 790 -> 130 us.
+//
+//   warp 0      producer: TMA of a weight tile (128 rows x 128 bytes) and a token tile (R x 128 bytes), cp.async of their scales
+//   warp 1      MMA issue; fp8: into one of two TMEM buffers per K block (the block's scale factors differ per row and column);
+//               bf16: one of two buffers per output tile
+//   warps 2..   epilogue, thread == weight row (R >= 32: two threads, half of the tokens each): tcgen05.ld, fp8: times sw[n] * sx[m] into
+//               fp32 registers; after the last block store column by column (64 bytes of a token's row per warp)
 #include "tcgen05_common.cuh"
 
 #include <cuda_fp8.h>
@@ -18,70 +27,93 @@
 
 namespace vb {
 
-constexpr int F8_BM = 128, F8_BN = 128, F8_BK = 128, F8_STAGES = 4, F8_THREADS = 192;
+constexpr int TG_BM = 128;   // weight rows per tile
+constexpr int TG_BK = 128;   // bytes of K per stage
 
-struct Fp8GemmParams {
-  int M, N, K;
-  const float* sa;  // [K/128, M]
-  const float* sb;  // [K/128, N]
+struct TileGemmParams {
+  int M, N, K;                  // tokens (rows of X), output columns, depth in elements
+  int ntiles;                   // weight tiles of one matrix
+  int mtiles;                   // token tiles (grouped: upper bound)
+  const float* sx;              // [K/128, M]
+  const float* sw;              // [K/128, ldsw]
+  long long ldsw;               // N, or E * N when grouped
   __nv_bfloat16* D;
   long long ldd;
   const __nv_bfloat16* bias;
   int* status;
-  // grouped (mixture-of-experts) mode: A rows are grouped by expert in 128-row aligned segments, B holds E stacked [N, K]
-  // matrices and sb E stacked column-scale rows; the 128-row tile i belongs to expert grp_tile_expert[i]
-  const int* grp_tile_expert;  // nullptr = plain GEMM
-  const int* grp_num_mtiles;   // device scalar: tiles in use (tiles beyond it return at once)
-  long long ldsb;              // row stride of sb (N, or E * N when grouped)
+  const int* tile_expert;       // grouped: expert of token tile i; W holds E stacked [N, K] matrices. nullptr = plain
+  const int* num_mtiles;        // grouped: device scalar, tiles in use
 };
 
-struct Fp8Smem {
-  static constexpr int TILE = F8_BM * F8_BK;  // 16 KB (one byte per element)
-  static constexpr int OFF_B = F8_STAGES * TILE;
-  static constexpr int OFF_SB = 2 * F8_STAGES * TILE;              // per epilogue warp: [2][128] fp32 column scales
-  static constexpr int OFF_BAR = OFF_SB + 4 * 2 * F8_BN * 4;
+template <bool FP8, int R>
+struct TileGemm {
+  static constexpr int STAGES = R <= 32 ? 10 : (R == 64 ? 8 : 6);
+  static constexpr int W_BYTES = TG_BM * TG_BK, X_BYTES = R * TG_BK;
+  static constexpr int SC_BYTES = FP8 ? 1024 : 0;  // 128 weight scales, then R token scales
+  static constexpr int STAGE = W_BYTES + X_BYTES + SC_BYTES;
+  static constexpr int EW = R >= 32 ? 8 : 4;       // epilogue warps
+  static constexpr int COLS = R / (EW / 4);        // tokens per epilogue thread
+  static constexpr int THREADS = 64 + 32 * EW;
+  static constexpr int TMEM_COLS = 2 * R < 32 ? 32 : 2 * R;
+  static constexpr int OFF_BAR = STAGES * STAGE;
   static constexpr int TOTAL = OFF_BAR + 256 + 1024;
+  static_assert(TOTAL <= 232448, "shared memory of a CTA");
 };
 
-__global__ void __launch_bounds__(F8_THREADS, 1)
-gemm_fp8_blockscale_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                           const Fp8GemmParams p) {
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+        "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+// arrives on `bar` (counted in its init) once the thread's cp.async so far have landed
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
+template <bool FP8, int R>
+__global__ void __launch_bounds__(TileGemm<FP8, R>::THREADS, 1)
+tile_gemm_kernel(const __grid_constant__ CUtensorMap tma_x, const __grid_constant__ CUtensorMap tma_w, const TileGemmParams p) {
+  using L = TileGemm<FP8, R>;
+  constexpr int STAGES = L::STAGES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* smem_a = smem;
-  uint8_t* smem_b = smem + Fp8Smem::OFF_B;
-  float* s_sb = reinterpret_cast<float*>(smem + Fp8Smem::OFF_SB);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Fp8Smem::OFF_BAR);
-  uint64_t* full_bar = bars;                       // [STAGES]
-  uint64_t* empty_bar = bars + F8_STAGES;          // [STAGES]
-  uint64_t* acc_full = bars + 2 * F8_STAGES;       // [2]
-  uint64_t* acc_empty = bars + 2 * F8_STAGES + 2;  // [2]
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * F8_STAGES + 4);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
+  uint64_t* full_bar = bars;                    // [STAGES]
+  uint64_t* empty_bar = bars + STAGES;          // [STAGES]
+  uint64_t* acc_full = bars + 2 * STAGES;       // [2]
+  uint64_t* acc_empty = bars + 2 * STAGES + 2;  // [2]
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int n0 = blockIdx.x * F8_BN, m0 = blockIdx.y * F8_BM;
-  const int num_kb = p.K / F8_BK;
-  int b_row0 = n0;  // first row of the B operand (and column of sb) of this tile
-  if (p.grp_tile_expert != nullptr) {
-    if (static_cast<int>(blockIdx.y) >= *p.grp_num_mtiles) return;  // uniform over the CTA; nothing allocated yet
-    b_row0 = p.grp_tile_expert[blockIdx.y] * p.N + n0;
-  }
+  const int num_kb = FP8 ? p.K / 128 : (p.K + 63) / 64;
+  const int mtiles = p.tile_expert != nullptr ? min(*p.num_mtiles, p.mtiles) : p.mtiles;
+  const int items = mtiles * p.ntiles;
+  if (static_cast<int>(blockIdx.x) >= items) return;  // uniform over the CTA; nothing allocated yet
 
   if (threadIdx.x == 0) {
-    tma_prefetch_desc(&tma_a);
-    tma_prefetch_desc(&tma_b);
-    for (int s = 0; s < F8_STAGES; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+    tma_prefetch_desc(&tma_x);
+    tma_prefetch_desc(&tma_w);
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full_bar[s], FP8 ? 1 + 32 : 1);           // the TMA's expectation, and every lane's scales
+      mbar_init(&empty_bar[s], FP8 ? 1 + L::EW : 1);       // the MMAs, and the readers of the scales
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
-      mbar_init(&acc_empty[a], 4);
+      mbar_init(&acc_empty[a], L::EW);
     }
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(tmem_holder, 2 * F8_BN);
+    tmem_alloc(tmem_holder, L::TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -90,108 +122,155 @@ gemm_fp8_blockscale_kernel(const __grid_constant__ CUtensorMap tma_a, const __gr
   const uint32_t tmem_base = *tmem_holder;
 
   if (warp == 0) {
-    if (lane == 0) {
+    // ------------------------------------------------------------------ producer (all lanes: they carry the scales)
+    int st = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+      const int mt = it / p.ntiles, n0 = (it - mt * p.ntiles) * TG_BM;
+      const int w_row0 = (p.tile_expert != nullptr ? p.tile_expert[mt] * p.N : 0) + n0;
+      const int m0 = mt * R;
       for (int kb = 0; kb < num_kb; ++kb) {
-        const int st = kb % F8_STAGES;
-        if (!mbar_wait(&empty_bar[st], ((kb / F8_STAGES) & 1) ^ 1)) {
-          atomicExch(p.status, ST_TIMEOUT_PRODUCER);
-          break;
+        ok = __all_sync(0xffffffffu, mbar_wait(&empty_bar[st], phase ^ 1));
+        if (!ok) break;
+        uint8_t* sw = smem + st * L::STAGE;
+        if (lane == 0) {
+          mbar_expect_tx(&full_bar[st], L::W_BYTES + L::X_BYTES);
+          const int k0 = kb * (FP8 ? 128 : 64);
+          tma_load_2d(sw, &tma_w, &full_bar[st], k0, w_row0);
+          tma_load_2d(sw + L::W_BYTES, &tma_x, &full_bar[st], k0, m0);
         }
-        mbar_expect_tx(&full_bar[st], 2 * Fp8Smem::TILE);
-        tma_load_2d(smem_a + st * Fp8Smem::TILE, &tma_a, &full_bar[st], kb * F8_BK, m0);
-        tma_load_2d(smem_b + st * Fp8Smem::TILE, &tma_b, &full_bar[st], kb * F8_BK, b_row0);
+        if constexpr (FP8) {
+          float* sc = reinterpret_cast<float*>(sw + L::W_BYTES + L::X_BYTES);
+          // N % 8 == 0: the 16-byte pieces are aligned and inside or outside as a whole
+          if (n0 + lane * 4 < p.N) cp_async16(sc + lane * 4, p.sw + static_cast<long long>(kb) * p.ldsw + w_row0 + lane * 4);
+#pragma unroll
+          for (int u = 0; u < (R + 31) / 32; ++u) {
+            const int j = u * 32 + lane;
+            if (j < R && m0 + j < p.M) cp_async4(sc + TG_BM + j, p.sx + static_cast<long long>(kb) * p.M + m0 + j);
+          }
+          cp_async_arrive(&full_bar[st]);
+        }
+        if (++st == STAGES) { st = 0; phase ^= 1; }
       }
     }
+    if (!ok && lane == 0) atomicExch(p.status, ST_TIMEOUT_PRODUCER);
+    if constexpr (FP8) asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
     if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_e4m3(F8_BM, F8_BN);
+      constexpr uint32_t idesc = FP8 ? make_idesc_e4m3(TG_BM, R) : make_idesc_f16(TG_BM, R, false, false);
+      int st = 0, buf = 0;
+      uint32_t phase = 0, buf_phase = 0;
       bool ok = true;
-      for (int kb = 0; kb < num_kb && ok; ++kb) {
-        const int st = kb % F8_STAGES, buf = kb & 1;
-        if (!mbar_wait(&acc_empty[buf], ((kb >> 1) & 1) ^ 1) || !mbar_wait(&full_bar[st], (kb / F8_STAGES) & 1)) {
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const uint32_t sa = smem_u32(smem_a + st * Fp8Smem::TILE), sb = smem_u32(smem_b + st * Fp8Smem::TILE);
+      for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+        for (int kb = 0; kb < num_kb; ++kb) {
+          if ((FP8 || kb == 0) && !mbar_wait(&acc_empty[buf], buf_phase ^ 1)) { ok = false; break; }
+          if (!mbar_wait(&full_bar[st], phase)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t sw = smem_u32(smem + st * L::STAGE), sx = sw + L::W_BYTES;
 #pragma unroll
-        for (int k = 0; k < F8_BK / 32; ++k) {
-          const uint64_t da = make_smem_desc_sw128(sa + k * 32, 16, 1024);
-          const uint64_t db = make_smem_desc_sw128(sb + k * 32, 16, 1024);
-          tc_mma_f8_ss(tmem_base + buf * F8_BN, da, db, idesc, k > 0 ? 1u : 0u);
+          for (int k = 0; k < 4; ++k) {  // 32 bytes of K per instruction
+            const uint64_t da = make_smem_desc_sw128(sw + k * 32, 16, 1024);
+            const uint64_t db = make_smem_desc_sw128(sx + k * 32, 16, 1024);
+            if constexpr (FP8) tc_mma_f8_ss(tmem_base + buf * R, da, db, idesc, k > 0 ? 1u : 0u);
+            else tc_mma_f16_ss(tmem_base + buf * R, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          }
+          tc_commit(&empty_bar[st]);
+          if (FP8 || kb == num_kb - 1) {
+            tc_commit(&acc_full[buf]);
+            if (++buf == 2) { buf = 0; buf_phase ^= 1; }
+          }
+          if (++st == STAGES) { st = 0; phase ^= 1; }
         }
-        tc_commit(&empty_bar[st]);
-        tc_commit(&acc_full[buf]);
       }
       if (!ok) atomicExch(p.status, ST_TIMEOUT_MMA);
     }
   } else {
-    const int q = warp & 3;
-    const int row = m0 + q * 32 + lane;
-    const bool row_ok = row < p.M;
+    // ------------------------------------------------------------------ epilogue
+    const int q = warp & 3, half = (warp - 2) >> 2;  // TMEM lane quarter, half of the tokens
+    const int c0 = half * L::COLS;
+    constexpr int CH = L::COLS < 32 ? 16 : 32;       // columns per tcgen05.ld
     const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
-    float* my_sb = s_sb + q * (2 * F8_BN);
-    float acc[F8_BN];
-#pragma unroll
-    for (int j = 0; j < F8_BN; ++j) acc[j] = 0.f;
+    int st = 0, buf = 0;
+    uint32_t phase = 0, buf_phase = 0;
     bool ok = true;
-    for (int kb = 0; kb < num_kb; ++kb) {
-      const int buf = kb & 1;
-      // column scales of this K block (each warp keeps its own copy: no barrier across warps)
-      float* csb = my_sb + buf * F8_BN;
+    for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+      const int mt = it / p.ntiles, n = (it - mt * p.ntiles) * TG_BM + q * 32 + lane;
+      float acc[L::COLS];
 #pragma unroll
-      for (int u = 0; u < F8_BN / 32; ++u) {
-        const int n = n0 + lane + 32 * u;
-        csb[lane + 32 * u] = n < p.N ? p.sb[static_cast<long long>(kb) * p.ldsb + (b_row0 - n0) + n] : 0.f;
-      }
-      const float ra = row_ok ? p.sa[static_cast<long long>(kb) * p.M + row] : 0.f;
-      __syncwarp();
-      if (!mbar_wait(&acc_full[buf], (kb >> 1) & 1)) {
-        ok = false;
-        break;
-      }
-      tc_fence_after();
+      for (int j = 0; j < L::COLS; ++j) acc[j] = 0.f;
+      const int reps = FP8 ? num_kb : 1;
+      for (int kb = 0; kb < reps; ++kb) {
+        if (FP8 && !mbar_wait(&full_bar[st], phase)) { ok = false; break; }  // the stage's scales; passes once the MMAs have run
+        if (!mbar_wait(&acc_full[buf], buf_phase)) { ok = false; break; }
+        tc_fence_after();
+        const float* sc = reinterpret_cast<const float*>(smem + st * L::STAGE + L::W_BYTES + L::X_BYTES);
+        const float rw = FP8 ? sc[q * 32 + lane] : 1.f;
 #pragma unroll
-      for (int c = 0; c < F8_BN / 32; ++c) {
-        uint32_t r[32];
-        tmem_ld_32x32(tmem_base + buf * F8_BN + c * 32 + lane_off, r);
-        tmem_ld_wait();
+        for (int c = 0; c < L::COLS; c += CH) {
+          uint32_t r[CH];
+          if constexpr (CH == 16) tmem_ld_32x16(tmem_base + buf * R + c0 + c + lane_off, r);
+          else tmem_ld_32x32(tmem_base + buf * R + c0 + c + lane_off, r);
+          tmem_ld_wait();
+          if constexpr (FP8) {
+            const float4* sx4 = reinterpret_cast<const float4*>(sc + TG_BM + c0 + c);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) acc[c * 32 + j] = fmaf(__uint_as_float(r[j]), ra * csb[c * 32 + j], acc[c * 32 + j]);
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[buf]);
-    }
-    if (!ok) {
-      if (lane == 0) atomicExch(p.status, ST_TIMEOUT_EPILOGUE);
-    } else if (row_ok) {
-      __nv_bfloat16* out = p.D + static_cast<long long>(row) * p.ldd + n0;
+            for (int j = 0; j < CH; j += 4) {
+              const float4 s4 = sx4[j >> 2];
+              acc[c + j] = fmaf(__uint_as_float(r[j]), rw * s4.x, acc[c + j]);
+              acc[c + j + 1] = fmaf(__uint_as_float(r[j + 1]), rw * s4.y, acc[c + j + 1]);
+              acc[c + j + 2] = fmaf(__uint_as_float(r[j + 2]), rw * s4.z, acc[c + j + 2]);
+              acc[c + j + 3] = fmaf(__uint_as_float(r[j + 3]), rw * s4.w, acc[c + j + 3]);
+            }
+          } else {
 #pragma unroll
-      for (int j = 0; j < F8_BN; j += 8) {
-        if (n0 + j < p.N) {
-          float b[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-          if (p.bias != nullptr) {
-#pragma unroll
-            for (int u = 0; u < 8; ++u) b[u] = __bfloat162float(p.bias[n0 + j + u]);
+            for (int j = 0; j < CH; ++j) acc[c + j] = __uint_as_float(r[j]);
           }
-          uint4 v;
-          v.x = pack_bf16x2(acc[j] + b[0], acc[j + 1] + b[1]);
-          v.y = pack_bf16x2(acc[j + 2] + b[2], acc[j + 3] + b[3]);
-          v.z = pack_bf16x2(acc[j + 4] + b[4], acc[j + 5] + b[5]);
-          v.w = pack_bf16x2(acc[j + 6] + b[6], acc[j + 7] + b[7]);
-          *reinterpret_cast<uint4*>(out + j) = v;
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(&acc_empty[buf]);
+          if (FP8) mbar_arrive(&empty_bar[st]);
+        }
+        if (++buf == 2) { buf = 0; buf_phase ^= 1; }
+        if (FP8 && ++st == STAGES) { st = 0; phase ^= 1; }
+      }
+      if (ok && n < p.N) {
+        const float b = p.bias != nullptr ? __bfloat162float(p.bias[n]) : 0.f;
+        const int m0 = mt * R + c0;
+        __nv_bfloat16* d = p.D + static_cast<long long>(m0) * p.ldd + n;
+#pragma unroll
+        for (int j = 0; j < L::COLS; ++j)
+          if (m0 + j < p.M) d[static_cast<long long>(j) * p.ldd] = __float2bfloat16(acc[j] + b);
       }
     }
+    if (!ok && lane == 0) atomicExch(p.status, ST_TIMEOUT_EPILOGUE);
   }
 
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 2 * F8_BN);
+    tmem_dealloc(tmem_base, L::TMEM_COLS);
   }
+}
+
+template <bool FP8, int R>
+static int launch_tile_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const TileGemmParams& p, cudaStream_t stream) {
+  using L = TileGemm<FP8, R>;
+  auto kern = tile_gemm_kernel<FP8, R>;
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured = true;
+  }
+  const long long items = static_cast<long long>(p.mtiles) * p.ntiles;
+  const int sms = num_sms();
+  kern<<<static_cast<int>(items < sms ? items : sms), L::THREADS, L::TOTAL, stream>>>(tx, tw, p);
+  return static_cast<int>(cudaGetLastError());
 }
 
 // x [R, C] bf16 -> q [R, C] e4m3 and scales [C/128, R] fp32 with  x ~= q * scale,  scale = amax(block) / 448.
@@ -215,6 +294,57 @@ __global__ void fp8_quant_1x128_kernel(const __nv_bfloat16* __restrict__ x, long
   __nv_fp8x4_e4m3 packed(make_float4(a.x * inv, a.y * inv, c.x * inv, c.y * inv));
   *reinterpret_cast<uint32_t*>(q + static_cast<long long>(r) * ldq + b * 128 + lane * 4) = *reinterpret_cast<uint32_t*>(&packed);
   if (lane == 0) scales[static_cast<long long>(b) * R + r] = scale;
+}
+
+// The same quantisation fused with what produces its input, for the rows of the tiles in use (num_mtiles * tile_rows; null: all).
+// One warp per (row, 128-column block).
+__device__ __forceinline__ void quant_block(const float (&f)[4], uint8_t* q, float* scale, int lane) {
+  float amax = fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3])));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  const float sc = fmaxf(amax, 1e-12f) / 448.f;
+  const float inv = 1.f / sc;
+  __nv_fp8x4_e4m3 packed(make_float4(f[0] * inv, f[1] * inv, f[2] * inv, f[3] * inv));
+  *reinterpret_cast<uint32_t*>(q + lane * 4) = *reinterpret_cast<uint32_t*>(&packed);
+  if (lane == 0) *scale = sc;
+}
+
+// q[r] = quantised src[map[r]], zeros where map[r] < 0
+__global__ void __launch_bounds__(256)
+moe_gather_quant_kernel(const __nv_bfloat16* __restrict__ src, long long lds, const int* __restrict__ map, uint8_t* __restrict__ q,
+                        float* __restrict__ scales, int R, int C, const int* __restrict__ num_mtiles, int tile_rows) {
+  const long long w = (blockIdx.x * 256LL + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31, nblk = C / 128;
+  const int r = static_cast<int>(w / nblk), b = static_cast<int>(w - static_cast<long long>(r) * nblk);
+  if (r >= min(R, *num_mtiles * tile_rows)) return;
+  const int s = map[r];
+  float f[4] = {0.f, 0.f, 0.f, 0.f};
+  if (s >= 0) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(src + static_cast<long long>(s) * lds + b * 128 + lane * 4);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    const float2 x = __bfloat1622float2(h[0]), y = __bfloat1622float2(h[1]);
+    f[0] = x.x; f[1] = x.y; f[2] = y.x; f[3] = y.y;
+  }
+  quant_block(f, q + static_cast<long long>(r) * C + b * 128, scales + static_cast<long long>(b) * R + r, lane);
+}
+
+// q = quantised silu(gate) * up of gu [R, 2 C] (rounded to bf16 in between, as the two kernels it replaces did)
+__global__ void __launch_bounds__(256)
+moe_swiglu_quant_kernel(const __nv_bfloat16* __restrict__ gu, uint8_t* __restrict__ q, float* __restrict__ scales, int R, int C,
+                        const int* __restrict__ num_mtiles, int tile_rows) {
+  const long long w = (blockIdx.x * 256LL + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31, nblk = C / 128;
+  const int r = static_cast<int>(w / nblk), b = static_cast<int>(w - static_cast<long long>(r) * nblk);
+  if (r >= min(R, *num_mtiles * tile_rows)) return;
+  const __nv_bfloat16* row = gu + static_cast<long long>(r) * 2 * C + b * 128 + lane * 4;
+  const uint2 rg = *reinterpret_cast<const uint2*>(row), ru = *reinterpret_cast<const uint2*>(row + C);
+  const __nv_bfloat162 *hg = reinterpret_cast<const __nv_bfloat162*>(&rg), *hu = reinterpret_cast<const __nv_bfloat162*>(&ru);
+  const float2 g0 = __bfloat1622float2(hg[0]), g1 = __bfloat1622float2(hg[1]), u0 = __bfloat1622float2(hu[0]), u1 = __bfloat1622float2(hu[1]);
+  const float g[4] = {g0.x, g0.y, g1.x, g1.y}, u[4] = {u0.x, u0.y, u1.x, u1.y};
+  float f[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) f[j] = __bfloat162float(__float2bfloat16(g[j] / (1.f + __expf(-g[j])) * u[j]));
+  quant_block(f, q + static_cast<long long>(r) * C + b * 128, scales + static_cast<long long>(b) * R + r, lane);
 }
 
 // w [R, C] bf16 -> q [R, C] e4m3 and scale_inv [ceil(R/128), ceil(C/128)] fp32: one scale per 128 x 128 block
@@ -284,6 +414,24 @@ extern "C" int vb_fp8_quant_1x128(const void* x, long long ldx, void* q, long lo
   return static_cast<int>(cudaGetLastError());
 }
 
+extern "C" int vb_moe_gather_quant(const void* src, long long lds, const int* map, void* q, float* scales, int R, int C,
+                                   const int* num_mtiles, int tile_rows, cudaStream_t s) {
+  if (R <= 0 || C <= 0) return 0;
+  if ((C % 128) || (lds % 4) || (reinterpret_cast<uintptr_t>(src) & 7)) return -1;
+  const long long blocks = (static_cast<long long>(R) * (C / 128) + 7) / 8;
+  moe_gather_quant_kernel<<<static_cast<int>(blocks), 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(src), lds, map,
+                                                                   reinterpret_cast<uint8_t*>(q), scales, R, C, num_mtiles, tile_rows);
+  return static_cast<int>(cudaGetLastError());
+}
+extern "C" int vb_moe_swiglu_quant(const void* gu, void* q, float* scales, int R, int C, const int* num_mtiles, int tile_rows, cudaStream_t s) {
+  if (R <= 0 || C <= 0) return 0;
+  if (C % 128) return -1;
+  const long long blocks = (static_cast<long long>(R) * (C / 128) + 7) / 8;
+  moe_swiglu_quant_kernel<<<static_cast<int>(blocks), 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(gu), reinterpret_cast<uint8_t*>(q),
+                                                                   scales, R, C, num_mtiles, tile_rows);
+  return static_cast<int>(cudaGetLastError());
+}
+
 extern "C" int vb_fp8_quant_128x128(const void* w, long long ldw, void* q, long long ldq, float* scale_inv, int R, int C, cudaStream_t s) {
   if (R <= 0 || C <= 0) return 0;
   if ((C % 4) || (ldw % 4) || (ldq % 4)) return -1;
@@ -293,58 +441,57 @@ extern "C" int vb_fp8_quant_128x128(const void* w, long long ldw, void* q, long 
   return static_cast<int>(cudaGetLastError());
 }
 
-extern "C" int vb_gemm_fp8_blockscale(const void* Aq, const float* sa, const void* Bq, const float* sb, void* D, const void* bias, int M,
-                                      int N, int K, long long lda, long long ldb, long long ldd, cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if ((K % 128) || (N % 8) || (lda % 16) || (ldb % 16) || (ldd % 8)) return -1;
-  if ((reinterpret_cast<uintptr_t>(Aq) | reinterpret_cast<uintptr_t>(Bq) | reinterpret_cast<uintptr_t>(D)) & 15) return -2;
-  CUtensorMap ta, tb;
-  if (!make_tmap_2d(&ta, Aq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, M, K, lda, F8_BK, F8_BM, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
-  if (!make_tmap_2d(&tb, Bq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, N, K, ldb, F8_BK, F8_BN, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
+// X [M, K], W [N, K] (grouped: E stacked matrices, w_rows = E * N), rows of X in tiles of R tokens.
+template <bool FP8>
+static int tile_gemm(const void* X, const float* sx, const void* W, const float* sw, void* D, const void* bias, int M, int N, int K, int E,
+                     long long ldx, long long ldw, long long ldd, int R, const int* tile_expert, const int* num_mtiles, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || E <= 0) return 0;
+  constexpr int eb = FP8 ? 1 : 2;
+  const bool grouped = tile_expert != nullptr;
+  if ((K % (FP8 ? 128 : 8)) || (N % 8) || ((ldx * eb) % 16) || ((ldw * eb) % 16) || (grouped && (M % R))) return -1;
+  if ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W) | reinterpret_cast<uintptr_t>(sw)) & 15) return -2;
+  const long long mtiles = (M + R - 1) / R, ntiles = (N + TG_BM - 1) / TG_BM;
+  if (mtiles * ntiles > 0x7fffffffLL - 65536 || static_cast<long long>(E) * N > 0x7fffffffLL) return -4;
+  CUtensorMap tx, tw;
+  const auto dt = FP8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  if (!make_tmap_2d(&tx, X, dt, eb, M, K, ldx, TG_BK / eb, R, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
+  if (!make_tmap_2d(&tw, W, dt, eb, static_cast<uint64_t>(E) * N, K, ldw, TG_BK / eb, TG_BM, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
   static int* status = nullptr;
   if (status == nullptr) cudaGetSymbolAddress(reinterpret_cast<void**>(&status), g_fp8_status);
-  Fp8GemmParams p{};
-  p.M = M; p.N = N; p.K = K; p.sa = sa; p.sb = sb; p.D = reinterpret_cast<__nv_bfloat16*>(D); p.ldd = ldd;
-  p.bias = reinterpret_cast<const __nv_bfloat16*>(bias); p.status = status;
-  p.ldsb = N;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_blockscale_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Fp8Smem::TOTAL);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
+  TileGemmParams p{};
+  p.M = M; p.N = N; p.K = K; p.ntiles = static_cast<int>(ntiles); p.mtiles = static_cast<int>(mtiles);
+  p.sx = sx; p.sw = sw; p.ldsw = static_cast<long long>(E) * N;
+  p.D = reinterpret_cast<__nv_bfloat16*>(D); p.ldd = ldd; p.bias = reinterpret_cast<const __nv_bfloat16*>(bias); p.status = status;
+  p.tile_expert = tile_expert; p.num_mtiles = num_mtiles;
+  switch (R) {
+    case 16: return launch_tile_gemm<FP8, 16>(tx, tw, p, stream);
+    case 32: return launch_tile_gemm<FP8, 32>(tx, tw, p, stream);
+    case 64: return launch_tile_gemm<FP8, 64>(tx, tw, p, stream);
+    case 128: return launch_tile_gemm<FP8, 128>(tx, tw, p, stream);
   }
-  dim3 grid((N + F8_BN - 1) / F8_BN, (M + F8_BM - 1) / F8_BM);
-  gemm_fp8_blockscale_kernel<<<grid, F8_THREADS, Fp8Smem::TOTAL, stream>>>(ta, tb, p);
-  return static_cast<int>(cudaGetLastError());
+  return -1;
 }
 
-// Grouped variant for mixture-of-experts layers: D[rows, N] = A[rows, K] * B_e^T for the expert e of each 128-row tile.
-//  Aq [rows_cap, K] e4m3 with scales sa [K/128, rows_cap]; Bq [E * N, K] e4m3 with scales sb [K/128, E * N];
+// The smallest token tile that covers the rows in one: the weights are read once.
+extern "C" int vb_gemm_fp8_blockscale(const void* Aq, const float* sa, const void* Bq, const float* sb, void* D, const void* bias, int M,
+                                      int N, int K, long long lda, long long ldb, long long ldd, cudaStream_t stream) {
+  const int R = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+  return tile_gemm<true>(Aq, sa, Bq, sb, D, bias, M, N, K, 1, lda, ldb, ldd, R, nullptr, nullptr, stream);
+}
+
+// Grouped variants for mixture-of-experts layers: D[rows, N] = A[rows, K] * B_e^T for the expert e of each tile of tile_rows rows
+// (16, 32, 64 or 128; rows_cap a multiple of it).
+//  B [E * N, K]; fp8: scales sa [K/128, rows_cap], sb [K/128, E * N];
 //  tile_expert[i] = expert of tile i, num_mtiles (device scalar) = tiles in use. Rows of unused tiles are not written.
 extern "C" int vb_gemm_fp8_blockscale_grouped(const void* Aq, const float* sa, const void* Bq, const float* sb, void* D, int rows_cap,
-                                              int N, int K, int E, long long lda, long long ldb, long long ldd, const int* tile_expert,
-                                              const int* num_mtiles, cudaStream_t stream) {
-  if (rows_cap <= 0 || N <= 0 || K <= 0 || E <= 0) return 0;
-  if ((K % 128) || (N % 8) || (rows_cap % F8_BM) || (lda % 16) || (ldb % 16) || (ldd % 8)) return -1;
-  if ((reinterpret_cast<uintptr_t>(Aq) | reinterpret_cast<uintptr_t>(Bq) | reinterpret_cast<uintptr_t>(D)) & 15) return -2;
-  CUtensorMap ta, tb;
-  if (!make_tmap_2d(&ta, Aq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, rows_cap, K, lda, F8_BK, F8_BM, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
-  if (!make_tmap_2d(&tb, Bq, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, static_cast<uint64_t>(E) * N, K, ldb, F8_BK, F8_BN, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
-  static int* status = nullptr;
-  if (status == nullptr) cudaGetSymbolAddress(reinterpret_cast<void**>(&status), g_fp8_status);
-  Fp8GemmParams p{};
-  p.M = rows_cap; p.N = N; p.K = K; p.sa = sa; p.sb = sb; p.D = reinterpret_cast<__nv_bfloat16*>(D); p.ldd = ldd;
-  p.bias = nullptr; p.status = status;
-  p.grp_tile_expert = tile_expert; p.grp_num_mtiles = num_mtiles; p.ldsb = static_cast<long long>(E) * N;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_fp8_blockscale_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Fp8Smem::TOTAL);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
-  dim3 grid((N + F8_BN - 1) / F8_BN, rows_cap / F8_BM);
-  gemm_fp8_blockscale_kernel<<<grid, F8_THREADS, Fp8Smem::TOTAL, stream>>>(ta, tb, p);
-  return static_cast<int>(cudaGetLastError());
+                                              int N, int K, int E, long long lda, long long ldb, long long ldd, int tile_rows,
+                                              const int* tile_expert, const int* num_mtiles, cudaStream_t stream) {
+  return tile_gemm<true>(Aq, sa, Bq, sb, D, nullptr, rows_cap, N, K, E, lda, ldb, ldd, tile_rows, tile_expert, num_mtiles, stream);
+}
+extern "C" int vb_gemm_bf16_grouped_tiles(const void* A, const void* B, void* D, int rows_cap, int N, int K, int E, long long lda,
+                                          long long ldb, long long ldd, int tile_rows, const int* tile_expert, const int* num_mtiles,
+                                          cudaStream_t stream) {
+  return tile_gemm<false>(A, nullptr, B, nullptr, D, nullptr, rows_cap, N, K, E, lda, ldb, ldd, tile_rows, tile_expert, num_mtiles, stream);
 }
 
 extern "C" int vb_fp8_status() {

@@ -83,6 +83,9 @@ int vb_paged_decode_grouped(const void* q, long long ldq, const void* kc, const 
                             int nsplit, float* part_o, float* part_ml, cudaStream_t stream);
 int vb_rope_kv_append(void* qkv, long long ld, const int* pos, const float* cos_t, const float* sin_t, const long long* slot,
                       void* kc, void* vc, int T, int nh, int nkv, int hd, cudaStream_t s);
+int vb_qk_norm_rope(void* qkv, long long ld, const int* pos, const float* cos_t, const float* sin_t, const void* wq, const void* wk, float eps,
+                    const long long* slot, void* kc, void* vc, void* pre_q, void* pre_k, float* rstd_q, float* rstd_k, int T, int nh, int nkv,
+                    int hd, cudaStream_t s);
 int vb_sample(const void* logits, long long ld, int B, int V, int valid_vocab, float inv_temp, const long long* seeds,
               long long step, long long* tokens, float* logprobs, cudaStream_t s);
 int vb_sample_topkp(const void* logits, long long ld, int B, int V, int valid_vocab, float inv_temp, int top_k, float top_p,
@@ -125,8 +128,13 @@ int vb_fp8_quant_1x128(const void* x, long long ldx, void* q, long long ldq, flo
 int vb_gemm_fp8_blockscale(const void* Aq, const float* sa, const void* Bq, const float* sb, void* D, const void* bias, int M, int N,
                            int K, long long lda, long long ldb, long long ldd, cudaStream_t stream);
 int vb_gemm_fp8_blockscale_grouped(const void* Aq, const float* sa, const void* Bq, const float* sb, void* D, int rows_cap, int N, int K,
-                                   int E, long long lda, long long ldb, long long ldd, const int* tile_expert, const int* num_mtiles,
-                                   cudaStream_t s);
+                                   int E, long long lda, long long ldb, long long ldd, int tile_rows, const int* tile_expert,
+                                   const int* num_mtiles, cudaStream_t s);
+int vb_gemm_bf16_grouped_tiles(const void* A, const void* B, void* D, int rows_cap, int N, int K, int E, long long lda, long long ldb,
+                               long long ldd, int tile_rows, const int* tile_expert, const int* num_mtiles, cudaStream_t s);
+int vb_moe_gather_quant(const void* src, long long lds, const int* map, void* q, float* scales, int R, int C, const int* num_mtiles,
+                        int tile_rows, cudaStream_t s);
+int vb_moe_swiglu_quant(const void* gu, void* q, float* scales, int R, int C, const int* num_mtiles, int tile_rows, cudaStream_t s);
 int vb_fp8_quant_128x128(const void* w, long long ldw, void* q, long long ldq, float* scale_inv, int R, int C, cudaStream_t s);
 int vb_fp8_status();
 int vb_latent_decode_status();
@@ -138,7 +146,10 @@ int vb_delta_chunk_status();
 int vb_moe_route_topk(const void* logits, long long ld, int T, int E, int k, int renorm, float* weights, int* experts, int* counts,
                       cudaStream_t s);
 int vb_moe_gather_rows(const void* src, long long lds, const int* map, const float* scale, void* dst, long long ldd, int rows, int H,
-                       cudaStream_t s);
+                       const int* num_mtiles, int tile_rows, cudaStream_t s);
+int vb_moe_swiglu(const void* gu, void* out, int rows, int I, const int* num_mtiles, int tile_rows, cudaStream_t s);
+int vb_moe_plan(const void* experts, int wide, const int* counts, int n, int k, int E, int tile, int cap, int* slot, int* src, int* seg,
+                int* tile_expert, int* num_mtiles, cudaStream_t s);
 int vb_moe_combine(const void* y, long long ldy, const int* slot, const float* w, void* out, long long ldo, int T, int H, int k,
                    cudaStream_t s);
 int vb_moe_combine_bwd_w(const void* g, long long ldg, const void* y, long long ldy, const int* slot, float* gw, int T, int H, int k,

@@ -596,6 +596,37 @@ def rope_kv_append_(qkv: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin
     kv_append_(k, v, slots, k_cache, v_cache)
 
 
+def qk_norm_rope_(qkv: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, wq: torch.Tensor, wk: torch.Tensor, eps: float,
+                  nh: int, nkv: int, hd: int, slots: Optional[torch.Tensor] = None, k_cache: Optional[torch.Tensor] = None,
+                  v_cache: Optional[torch.Tensor] = None, save: bool = False):
+    """RMSNorm of every q and k head of ``qkv`` [T, (nh + 2 nkv) * hd] and their rotation, in place; with ``slots`` also the append of the
+    rotated k and of v to the paged caches (negative: skip). ``save``: returns (q, k in front of the norm, their 1 / rms) for the
+    backward pass. One kernel on a GPU; the same steps through the separate ops elsewhere."""
+    if audit.enabled():
+        audit.check_index("qk_norm_rope_", "pos", pos, cos.shape[0])
+        if slots is not None:
+            audit.check_index("qk_norm_rope_", "slots", slots, k_cache.numel() // (nkv * hd), skip_negative=True)
+    if (qkv.is_cuda and qkv.dtype == torch.bfloat16 and hd % 16 == 0 and hd <= 256 and qkv.stride(0) % 8 == 0
+            and all(t.data_ptr() % 16 == 0 for t in (qkv, wq, wk))):
+        out = _ops().qk_norm_rope_(qkv, pos.to(torch.int32), cos, sin, wq, wk, eps, int(nh), int(nkv), int(hd), slots, k_cache, v_cache, bool(save))
+        return tuple(out) if save else None
+    T = qkv.shape[0]
+    q = qkv[:, : nh * hd].view(T, nh, hd)
+    k = qkv[:, nh * hd : (nh + nkv) * hd].view(T, nkv, hd)
+    qp, kp = q.reshape(T * nh, hd).contiguous(), k.reshape(T * nkv, hd).contiguous()
+    if save:  # a single head makes the reshape a view of what is overwritten below
+        qp, kp = qp.clone(), kp.clone()
+    qn, _, rq = rms_norm(qp, wq, eps)
+    kn, _, rk = rms_norm(kp, wk, eps)
+    q.copy_(qn.view(T, nh, hd))
+    k.copy_(kn.view(T, nkv, hd))
+    apply_rope_(q, pos, cos, sin)
+    apply_rope_(k, pos, cos, sin)
+    if slots is not None:
+        kv_append_(k, qkv[:, (nh + nkv) * hd :].view(T, nkv, hd), slots, k_cache, v_cache)
+    return (qp, kp, rq, rk) if save else None
+
+
 def paged_decode_attention(q, k_cache, v_cache, block_table, ctx_len, scale: Optional[float] = None, groups=None):
     """One query token per sequence against a paged cache [num_blocks, block_size, nkv, hd].
 

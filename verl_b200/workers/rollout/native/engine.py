@@ -764,12 +764,10 @@ class RolloutEngine:
             q = qkv[:, :Q].view(S, nh, hd)
             k = qkv[:, Q : Q + KV].view(S, nkv, hd)
             v = qkv[:, Q + KV :].view(S, nkv, hd)
-            if cfg.qk_norm:
-                qn = F.rms_norm(q.reshape(S * nh, hd).contiguous(), W["self_attn.q_norm.weight"], cfg.rms_norm_eps)[0]
-                kn = F.rms_norm(k.reshape(S * nkv, hd).contiguous(), W["self_attn.k_norm.weight"], cfg.rms_norm_eps)[0]
-                q.copy_(qn.view(S, nh, hd))
-                k.copy_(kn.view(S, nkv, hd))
-            if cfg.qk_norm or not qkv.is_contiguous() or not self.fused_rope_append:
+            if cfg.qk_norm:  # one launch: norm and rotation of q and k in the projection output, append of k and v to the cache
+                F.qk_norm_rope_(qkv, self.pos, cos, sin, W["self_attn.q_norm.weight"], W["self_attn.k_norm.weight"], cfg.rms_norm_eps,
+                                nh, nkv, hd, slot_map, self.kv[i, 0], self.kv[i, 1])
+            elif not qkv.is_contiguous() or not self.fused_rope_append:
                 F.apply_rope_(q, self.pos, cos, sin)
                 F.apply_rope_(k, self.pos, cos, sin)
                 F.kv_append_(k, v, slot_map, self.kv[i, 0], self.kv[i, 1])
@@ -837,7 +835,7 @@ class RolloutEngine:
         if self.is_cuda:  # device time of the decode steps, read at the next host synchronisation (``_sync_retire``)
             ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
             ev[0].record()
-        if not self.use_graph or self.cfg.is_moe:
+        if not self.use_graph or not (self.cfg.is_stack or self.model.decode_capturable()):
             for _ in range(n):
                 self._decode_body()
         else:
