@@ -402,3 +402,23 @@ def test_qk_norm_rotation_and_append_in_one(ops, T, nh, nkv, hd):
     assert torch.equal(saved[0], qp) and torch.equal(saved[1], kp)
     assert torch.equal(saved[2], rq) and torch.equal(saved[3], rk)
     assert int((qkv != ref).sum()) == 0 and torch.equal(kc, kr) and torch.equal(vc, vr)
+
+
+# ------------------------------------------------------------------------------------------------ products of at most 64 tokens
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("N,K", [(2, 8), (24, 64), (130, 72), (896, 4864), (1152, 896), (9600, 136)])
+def test_few_tokens(ops, M, N, K):
+    """bf16 products are exact in fp32: the bound is the rounding of the result (2^-9, twice with the activation's inputs) and of the sums."""
+    g = torch.Generator().manual_seed(M + N + K)
+    x = torch.randn(M, K + 8, generator=g).to(DEV).bfloat16()[:, :K]
+    w = (torch.randn(2 * N, K, generator=g) * 0.1).to(DEV).bfloat16()
+    bias = torch.randn(N, generator=g).to(DEV).bfloat16()
+    full, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    for b in (None, bias):
+        want = full[:, :N] + (b.double() if b is not None else 0)
+        y = ops.gemm_few_tokens(x, w[:N], b, False).double()
+        assert ((y - want).abs() <= want.abs() * 2.0**-8 + size[:, :N] * K * 2.0**-24 + 1e-30).all()
+    gu = ops.gemm_few_tokens(x, w, None, False)
+    act = ops.gemm_few_tokens(x, w, None, True)
+    want = torch.nn.functional.silu(gu[:, :N].double()) * gu[:, N:].double()
+    assert rel(act, want) < 4e-3  # 2^-9 for the result, 2^-9 where another order of the sums rounds a gate or an up value differently

@@ -75,9 +75,26 @@ bool gemm_row_ranges_(const Tensor& a, const Tensor& w, const OptTensor& bias, s
   return true;
 }
 
+// X W^T (+bias), or silu(X Wg^T) * (X Wu^T) for W = [Wg; Wu], by the kernel for at most 64 tokens, whatever the dispatch of `gemm` says.
+Tensor gemm_few_tokens(const Tensor& x, const Tensor& w, const OptTensor& bias, bool swiglu) {
+  CHECK_BF16(x);
+  CHECK_BF16(w);
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.stride(1) == 1 && w.stride(1) == 1 && x.size(1) == w.size(1) && x.size(0) <= 64 &&
+              (!swiglu || (w.size(0) % 2 == 0 && !bias.has_value())), "gemm_few_tokens: x [M <= 64, K], w [N, K]");
+  const int64_t M = x.size(0), N = swiglu ? w.size(0) / 2 : w.size(0), K = x.size(1);
+  if (bias.has_value()) TORCH_CHECK(bias->scalar_type() == at::kBFloat16 && bias->numel() == N && bias->is_contiguous());
+  const c10::cuda::CUDAGuard guard(x.device());
+  Tensor d = at::empty({M, N}, x.options());
+  if (M == 0 || N == 0) return d;
+  count(1);
+  CHECK_RC(vb_gemm_few_tokens(x.data_ptr(), w.data_ptr(), d.data_ptr(), optr(bias), (int)M, (int)N, (int)K, x.stride(0), w.stride(0),
+                              d.stride(0), swiglu, cur_stream()), "vb_gemm_few_tokens");
+  return d;
+}
+
 // D = A * B^T (+bias).  a: [M,K] (or [K,M] when a_mn), b: [N,K] (or [K,N] when b_mn); rows may be strided.
-Tensor gemm(const Tensor& a, const Tensor& b, const OptTensor& bias, const OptTensor& out, bool a_mn, bool b_mn,
-            bool out_f32, bool accumulate, int64_t max_ctas) {
+Tensor gemm_dispatch(const Tensor& a, const Tensor& b, const OptTensor& bias, const OptTensor& out, bool a_mn, bool b_mn,
+                     bool out_f32, bool accumulate, int64_t max_ctas, bool few_tokens) {
   CHECK_BF16(a);
   CHECK_BF16(b);
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1, "gemm: 2-D row-major operands");
@@ -105,7 +122,13 @@ Tensor gemm(const Tensor& a, const Tensor& b, const OptTensor& bias, const OptTe
   if (skinny_enabled() && M <= 1024 && !a_mn && !b_mn && !out_f32 && !accumulate && max_ctas == 0 && N % 8 == 0 && K % 8 == 0 &&
       a.stride(0) % 8 == 0 && b.stride(0) % 8 == 0 && d.stride(0) % 4 == 0 && reinterpret_cast<uintptr_t>(d.data_ptr()) % 8 == 0 &&
       reinterpret_cast<uintptr_t>(a.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(b.data_ptr()) % 16 == 0) {
-    // few tokens: the transposed kernel (128 weight rows x up to 512 tokens per CTA, K split with the fold inside the launch)
+    if (few_tokens && vb_few_tokens_better((int)M, (int)N, (int)K, 0)) {
+      count(1);
+      CHECK_RC(vb_gemm_few_tokens(a.data_ptr(), b.data_ptr(), d.data_ptr(), bias_ptr, (int)M, (int)N, (int)K, a.stride(0), b.stride(0),
+                                  d.stride(0), 0, cur_stream()), "vb_gemm_few_tokens");
+      return d;
+    }
+    // more tokens or weights: the transposed kernel (128 weight rows x up to 512 tokens per CTA, K split with the fold inside the launch)
     const int s = vb_gemm_skinny_splits((int)M, (int)N, (int)K);
     if (s >= 1) {
       Tensor ws;
@@ -127,6 +150,15 @@ Tensor gemm(const Tensor& a, const Tensor& b, const OptTensor& bias, const OptTe
                                  splits > 1 ? ws.data_ptr<float>() : nullptr, cur_stream());
   TORCH_CHECK(rc == 0, "vb_gemm_bf16 failed with code ", rc, " (M=", M, " N=", N, " K=", K, ")");
   return d;
+}
+
+Tensor gemm(const Tensor& a, const Tensor& b, const OptTensor& bias, const OptTensor& out, bool a_mn, bool b_mn, bool out_f32, bool accumulate,
+            int64_t max_ctas) {
+  return gemm_dispatch(a, b, bias, out, a_mn, b_mn, out_f32, accumulate, max_ctas, true);
+}
+Tensor gemm_tcgen05(const Tensor& a, const Tensor& b, const OptTensor& bias, const OptTensor& out, bool a_mn, bool b_mn, bool out_f32,
+                    bool accumulate, int64_t max_ctas) {
+  return gemm_dispatch(a, b, bias, out, a_mn, b_mn, out_f32, accumulate, max_ctas, false);
 }
 
 // act = silu(a W_gate^T) * (a W_up^T) for the stacked weight w = [W_gate; W_up] ([2I, K]); with want_gu the pre-activation
@@ -1193,6 +1225,11 @@ TORCH_LIBRARY(verl_b200, m) {
   m.def("gemm_grouped_rows", &gemm_grouped_rows);
   m.def("gemm_grouped_wgrad_", &gemm_grouped_wgrad_);
   m.def("gemm", &gemm);
+  m.def("gemm_tcgen05", &gemm_tcgen05);
+  m.def("gemm_few_tokens", &gemm_few_tokens);
+  m.def("few_tokens_better", [](int64_t M, int64_t N, int64_t K, bool swiglu) {
+    return skinny_enabled() && vb_few_tokens_better((int)std::min<int64_t>(M, 65), (int)N, (int)K, swiglu) != 0;
+  });
   m.def("gemm_status", &gemm_status);
   m.def("gemm_swiglu", &gemm_swiglu);
   m.def("gemm_row_ranges_", &gemm_row_ranges_);

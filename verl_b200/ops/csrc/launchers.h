@@ -121,6 +121,10 @@ int vb_peer_share(const unsigned long long* buf_ptrs, const unsigned long long* 
 int vb_scatter_copy(const void* jobs, const int* block_start, int njobs, int total_blocks, cudaStream_t s);
 int vb_allreduce_peer(const unsigned long long* buf_ptrs, void* out, long long n, int W, int rank, cudaStream_t s);
 int vb_comm_status();
+// gemm_few_tokens.cu
+int vb_gemm_few_tokens(const void* X, const void* W, void* D, const void* bias, int M, int N, int K, long long ldx, long long ldw,
+                       long long ldd, int swiglu, cudaStream_t s);
+int vb_few_tokens_better(int M, int N, int K, int swiglu);
 // gemm_fp8_blockscale.cu
 int vb_nvfp4_fake_quant(const void* x, long long ldx, void* y, long long ldy, long long rows, int cols, float global_scale,
                         cudaStream_t s);
