@@ -422,3 +422,38 @@ def test_few_tokens(ops, M, N, K):
     act = ops.gemm_few_tokens(x, w, None, True)
     want = torch.nn.functional.silu(gu[:, :N].double()) * gu[:, N:].double()
     assert rel(act, want) < 4e-3  # 2^-9 for the result, 2^-9 where another order of the sums rounds a gate or an up value differently
+
+
+# ------------------------------------------------------------------------------------------------ weight gradients added in L2
+@pytest.mark.parametrize("M,N,K", [(32, 136, 64), (96, 264, 72), (128, 256, 64), (160, 776, 200), (2048, 768, 640), (40, 264, 128)])
+def test_weight_gradient_accumulates(ops, M, N, K):
+    g = torch.Generator().manual_seed(M + N + K)
+    dy, x = torch.randn(K, M, generator=g).to(DEV).bfloat16(), torch.randn(K, N, generator=g).to(DEV).bfloat16()
+    out = torch.randn(M, N + 8, generator=g).to(DEV)
+    before = out.clone()
+    for _ in range(2):
+        ops.gemm(dy, x, None, out[:, :N], True, True, True, True, 0)
+    want = before[:, :N].double() + 2 * (dy.double().T @ x.double())
+    size = dy.double().abs().T @ x.double().abs()
+    assert ((out[:, :N].double() - want).abs() <= (2 * size * K + before[:, :N].double().abs() + want.abs()) * 2.0**-23).all()
+    assert torch.equal(out[:, N:], before[:, N:])
+    assert int(ops.gemm_status()) == 0
+
+
+@pytest.mark.parametrize("M,N", [(128, 256), (160, 264), (96, 768), (72, 264)])
+def test_weight_gradient_per_expert_accumulates(ops, M, N):
+    counts = [130, 0, 128, 5, 0]
+    seg = torch.tensor([0] + np.cumsum([(c + 127) // 128 * 128 for c in counts]).tolist(), dtype=torch.int32, device=DEV)
+    rows = int(seg[-1]) + 128
+    g = torch.Generator().manual_seed(M + N)
+    dy, x = torch.zeros(rows, M, device=DEV, dtype=torch.bfloat16), torch.zeros(rows, N, device=DEV, dtype=torch.bfloat16)
+    for e, c in enumerate(counts):
+        dy[seg[e] : seg[e] + c] = torch.randn(c, M, generator=g).to(DEV).bfloat16()
+        x[seg[e] : seg[e] + c] = torch.randn(c, N, generator=g).to(DEV).bfloat16()
+    out = torch.randn(len(counts), M, N, generator=g).to(DEV)
+    want = out.double()
+    for e, c in enumerate(counts):
+        want[e] += dy[seg[e] : seg[e] + c].double().T @ x[seg[e] : seg[e] + c].double()
+    ops.gemm_grouped_wgrad_(dy, x, out, seg, True)
+    assert float((out.double() - want).abs().max()) < 1e-3  # sums of at most 130 products of size 1..10 in fp32
+    assert int(ops.gemm_status()) == 0

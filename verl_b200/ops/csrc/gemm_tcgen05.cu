@@ -45,7 +45,12 @@ constexpr int GEMM_THREADS = 192;
 //               also written in the stacked layout ([M, 2I], what the backward pass of a kept layer reads).
 //  EPI_MIXER    elementwise epilogues of the mixer stack (`mixer_epilogue.cuh`): erf-gelu, residual add with the next norm,
 //               or an output whose last columns stay fp32
-enum { EPI_STORE = 0, EPI_LSE = 1, EPI_DLOGITS = 2, EPI_ALLREDUCE = 3, EPI_SWIGLU = 4, EPI_MIXER = 5 };
+//  EPI_ACC32    D (fp32) += acc: a warp's 32 x 32 pieces go through shared memory into TMA reductions, two in flight, and the addition
+//               happens in L2. Read back by the epilogue, every piece cost a memory latency with 16 bytes per row and request: of
+//               little account behind a long contraction, but the weight gradients of experts with 350 tokens each were bound by
+//               it: 128 x [2048, 768] (1.6 GB read and written) 1052 us, 128 x [1536, 2048] (3.2 GB) 2018 us; all weight gradients
+//               of two such layers and the head 9.3 -> 5.0 ms.
+enum { EPI_STORE = 0, EPI_LSE = 1, EPI_DLOGITS = 2, EPI_ALLREDUCE = 3, EPI_SWIGLU = 4, EPI_MIXER = 5, EPI_ACC32 = 6 };
 
 constexpr int AR_MAX_RANKS = 8;
 
@@ -152,6 +157,8 @@ struct GemmSmem {
   static constexpr int TOTAL = RING + 256 + 1024;  // barriers + alignment slack
   static constexpr int STAGE_LD = 36;              // EPI_MIXER: row pitch (floats) of a warp's 32 x 32 transposition tile
   static constexpr int TOTAL_MIXER = TOTAL + 4 * 32 * STAGE_LD * 4;
+  static constexpr int ACC_PIECE = 32 * 32 * 4;    // EPI_ACC32: two pieces per epilogue warp, between the ring and the barriers
+  static constexpr int TOTAL_ACC = TOTAL + 4 * 2 * ACC_PIECE;
 };
 
 // Pass B of the all-reduce epilogue for one warp's slab (32 rows x BN columns): sum the bf16 partials of all ranks in rank
@@ -219,14 +226,16 @@ __device__ __forceinline__ void ar_sum_slab(const GemmParams& p, long long half,
 
 // Kernel body. FETCH adds copy warps that stage peer memory into local memory (see GemmParams::fetch_*).
 template <int BN, bool A_MN, bool B_MN, int STAGES, int EPI, bool FETCH>
-__device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtensorMap& tma_b, const GemmParams& p) {
+__device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtensorMap& tma_b, const GemmParams& p,
+                                          const CUtensorMap* tma_d = nullptr) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int A_BYTES = GemmSmem<BN, STAGES>::A_BYTES;
   constexpr int B_BYTES = GemmSmem<BN, STAGES>::B_BYTES;
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + STAGES * A_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + GemmSmem<BN, STAGES>::RING);
+  constexpr int OFF_BARS = GemmSmem<BN, STAGES>::RING + (EPI == EPI_ACC32 ? 4 * 2 * GemmSmem<BN, STAGES>::ACC_PIECE : 0);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BARS);
   uint64_t* full_bar = bars;                   // [STAGES]
   uint64_t* empty_bar = bars + STAGES;         // [STAGES]
   uint64_t* acc_full = bars + 2 * STAGES;      // [2]
@@ -475,6 +484,7 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
     int acc = 0;
     uint32_t acc_phase = 0;
     bool ok = true;
+    int pieces = 0;  // EPI_ACC32: pieces so far, alternating between the warp's two buffers
     float mix_alpha = 0.f, mix_palpha = 0.f;
     // residual stream of the 32 x 32 block at (row0, col): lanes sweep the columns, four rows per round, so that reads and
     // writes are whole 128-byte lines
@@ -715,6 +725,21 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
               }
             }
           }
+        } else if constexpr (EPI == EPI_ACC32) {
+          // 32 rows of 128 bytes, 16-byte pieces swizzled by the row; columns past N are clipped by the tensor map
+          uint8_t* piece = smem + GemmSmem<BN, STAGES>::RING + (q * 2 + (pieces & 1)) * GemmSmem<BN, STAGES>::ACC_PIECE;
+          if (lane == 0) tma_store_wait_read<1>();  // the reduction before the last has read this piece
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<uint4*>(piece + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && m0 + q * 32 < p.M) {  // M % 32 == 0: a slab of 32 rows belongs to one output
+            tma_reduce_add_2d(tma_d, piece, col0, static_cast<int>(d_off) + m0 + q * 32);
+            tma_store_commit();
+          }
+          ++pieces;
         } else if (row_ok) {
           if (p.bias != nullptr) {
 #pragma unroll
@@ -885,6 +910,9 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
   }
 
   // ------------------------------------------------------------------ teardown
+  if constexpr (EPI == EPI_ACC32) {
+    if (warp >= 2 && lane == 0) tma_store_wait_all<0>();
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -910,6 +938,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
                  const GemmParams p) {
   gemm_body<BN, A_MN, B_MN, STAGES, EPI, false>(tma_a, tma_b, p);
+}
+
+template <int BN, int STAGES>
+__global__ void __launch_bounds__(GEMM_THREADS, 1)
+gemm_bf16_acc_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
+                     const __grid_constant__ CUtensorMap tma_d, const GemmParams p) {
+  gemm_body<BN, true, true, STAGES, EPI_ACC32, false>(tma_a, tma_b, p, &tma_d);
 }
 
 constexpr int GEMM_FETCH_THREADS = GEMM_THREADS + 32 * FETCH_WARPS;
@@ -946,6 +981,26 @@ static cudaError_t launch_variant(const CUtensorMap& ta, const CUtensorMap& tb, 
   const int grid = tiles < sms ? tiles : sms;
   kern<<<grid, GEMM_THREADS, smem, stream>>>(ta, tb, p);
   return cudaGetLastError();
+}
+
+// Weight gradient D (fp32 [d_rows, N]) += A^T B with the addition in L2; both operands stored [K, M|N]. Serves whole slabs of 32 rows
+// and outputs wider than 128 columns; `tiles` is an upper bound. Returns -1 for others.
+static int launch_acc(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, long long d_rows, long long tiles, int sms,
+                      cudaStream_t stream) {
+  if (p.N <= 128 || (p.M % 32) || p.bias != nullptr || (p.ldd % 4) || d_rows > 0x7fffffffLL) return -1;
+  CUtensorMap td;
+  if (!make_tmap_2d(&td, p.D, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, d_rows, p.N, p.ldd, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B)) return -1;
+  auto kern = gemm_bf16_acc_kernel<256, 4>;
+  constexpr int smem = GemmSmem<256, 4>::TOTAL_ACC;
+  static_assert(smem <= 232448, "shared memory of a CTA");
+  static bool configured = false;
+  if (!configured) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    configured = true;
+  }
+  kern<<<static_cast<int>(tiles < sms ? tiles : sms), GEMM_THREADS, smem, stream>>>(ta, tb, td, p);
+  return static_cast<int>(cudaGetLastError());
 }
 
 }  // namespace vb
@@ -1167,6 +1222,10 @@ extern "C" int vb_gemm_bf16_ex(const void* A, const void* B, void* D, const void
     p.k_splits = k_splits; p.D = splitk_ws; p.ldd = N; p.bias = nullptr; p.out_f32 = 1; p.accumulate = 0;
   }
   cudaError_t e;
+  if (wide && a_mn && b_mn && out_f32 && accumulate && p.k_splits == 1) {
+    const int rc = launch_acc(ta, tb, p, M, static_cast<long long>((M + BM - 1) / BM) * ((N + 255) / 256), sms, stream);
+    if (rc >= 0) return rc;
+  }
 #define VB_LAUNCH(BN_, AM, BMJ, ST) e = launch_variant<BN_, AM, BMJ, ST>(ta, tb, p, sms, stream)
   if (wide) {
     if (!a_mn && !b_mn) VB_LAUNCH(256, false, false, 4);
@@ -1492,6 +1551,10 @@ extern "C" int vb_gemm_grouped(int mode, const void* A, const void* B, void* D, 
     if (!make_tmap_2d(&tb, B, bf, 2, rows_cap, N, ldb, 64, BK, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
     max_tiles = E * ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
     const int grid = max_tiles < sms ? max_tiles : sms;
+    if (wide && accumulate) {
+      const int rc = launch_acc(ta, tb, p, static_cast<long long>(E) * M, max_tiles, sms, stream);
+      if (rc >= 0) return rc;
+    }
     if (wide) {
       auto kern = gemm_bf16_kernel<256, true, true, 4, EPI_STORE>;
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<256, 4>::TOTAL);
