@@ -457,3 +457,51 @@ def test_weight_gradient_per_expert_accumulates(ops, M, N):
     ops.gemm_grouped_wgrad_(dy, x, out, seg, True)
     assert float((out.double() - want).abs().max()) < 1e-3  # sums of at most 130 products of size 1..10 in fp32
     assert int(ops.gemm_status()) == 0
+
+
+# ------------------------------------------------------------------------------------------------ norms
+@pytest.mark.parametrize("T,H", [(1, 8), (3, 248), (5, 264), (639, 264), (1183, 896), (1184, 1024), (640, 1032), (700, 2040), (1185, 2048),
+                                 (641, 2056), (9, 3584), (700, 3584), (640, 4096), (640, 4104), (2, 8192), (1300, 3592)])
+def test_rmsnorm_rows(ops, T, H):
+    g = torch.Generator().manual_seed(T + H)
+    x, res, dy, dres = (torch.randn(T, H, generator=g).to(DEV).bfloat16() for _ in range(4))
+    w = (1 + 0.1 * torch.randn(H, generator=g)).to(DEV).bfloat16()
+    for r in (None, res):
+        y, xe, rstd = ops.rmsnorm_fwd(x, r, w, 1e-6)
+        if r is not None:
+            assert torch.equal(xe, (x.float() + r.float()).bfloat16())
+        xd = xe.double()
+        want = torch.rsqrt(xd.square().mean(-1) + 1e-6)
+        torch.testing.assert_close(rstd.double(), want, rtol=2e-6, atol=0)  # fp32 sums of squares and the approximate root
+        full = xd * want[:, None] * w.double()
+        assert ((y.double() - full).abs() <= 2.0**-8 * full.abs() + 1e-30).all()
+        few = ops.rmsnorm_fwd(x[:3].contiguous(), None if r is None else r[:3].contiguous(), w, 1e-6)
+        assert torch.equal(few[0], y[:3]) and torch.equal(few[2], rstd[:3])  # a row's bits do not depend on the number of rows
+    dw = torch.randn(H, generator=g).to(DEV)
+    dw0 = dw.clone()
+    dx = ops.rmsnorm_bwd(dy, x, w, ops.rmsnorm_fwd(x, None, w, 1e-6)[2], dres, dw, True)
+    xd = x.double().requires_grad_()
+    wd = w.double().requires_grad_()
+    (xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-6) * wd).backward(dy.double())
+    assert rel(dx, xd.grad + dres.double()) < 4e-3  # rounding of the result
+    assert rel(dw - dw0, wd.grad) < 1e-5
+
+
+@pytest.mark.parametrize("T,nh,nkv,hd", [(1, 1, 1, 64), (5, 4, 2, 128), (33, 3, 1, 256), (70, 8, 8, 96), (1000, 32, 4, 128)])
+def test_qk_norm_backward_in_place(ops, T, nh, nkv, hd):
+    from verl_b200.ops import functional as F
+
+    g = torch.Generator().manual_seed(T + hd)
+    gq = torch.randn(T, (nh + 2 * nkv) * hd, generator=g).to(DEV).bfloat16()
+    pre = [torch.randn(T * n, hd, generator=g).to(DEV).bfloat16() for n in (nh, nkv)]
+    w = [(1 + 0.1 * torch.randn(hd, generator=g)).to(DEV).bfloat16() for _ in range(2)]
+    rstd = [torch.rsqrt(p.float().square().mean(-1) + 1e-6) for p in pre]
+    dw = [torch.ones(hd, device=DEV) for _ in range(2)]
+    out = gq.clone()
+    F.qk_norm_bwd_(out, *pre, *rstd, *w, *dw, nh, nkv, hd)
+    assert torch.equal(out[:, (nh + nkv) * hd :], gq[:, (nh + nkv) * hd :])
+    for i, sl in enumerate((slice(0, nh * hd), slice(nh * hd, (nh + nkv) * hd))):
+        xd, wd = pre[i].double().requires_grad_(), w[i].double().requires_grad_()
+        (xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-6) * wd).backward(gq[:, sl].reshape(-1, hd).double())
+        assert rel(out[:, sl].reshape(-1, hd), xd.grad) < 4e-3
+        assert rel(dw[i] - 1, wd.grad) < 1e-5

@@ -646,17 +646,10 @@ class DecoderModel:
     def _qkv_bwd(self, W, g_qkv, h1, S: dict):
         """From the gradient of the rotated-back q, k and v to the gradient of the projection's input."""
         cfg = self.cfg
-        T = g_qkv.shape[0]
-        nh, nkv, hd, Q, KV = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim, cfg.q_size, cfg.kv_size
-        gq, gk = g_qkv[:, :Q].view(T, nh, hd), g_qkv[:, Q : Q + KV].view(T, nkv, hd)
+        nh, nkv, hd = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
         if cfg.qk_norm:
             wq, wk = W["self_attn.q_norm.weight"], W["self_attn.k_norm.weight"]
-            dqp = F.rms_norm_bwd(gq.reshape(T * nh, hd).contiguous(), S["q_pre"], wq, S["rstd_q"], None,
-                                 self._grad_of(wq), True)
-            dkp = F.rms_norm_bwd(gk.reshape(T * nkv, hd).contiguous(), S["k_pre"], wk, S["rstd_k"], None,
-                                 self._grad_of(wk), True)
-            gq.copy_(dqp.view(T, nh, hd))
-            gk.copy_(dkp.view(T, nkv, hd))
+            F.qk_norm_bwd_(g_qkv, S["q_pre"], S["k_pre"], S["rstd_q"], S["rstd_k"], wq, wk, self._grad_of(wq), self._grad_of(wk), nh, nkv, hd)
         if self.tp_linear_sum is not None:
             g_h1 = self.tp_linear_sum(g_qkv, W["self_attn.qkv_proj.weight"], True)
         else:

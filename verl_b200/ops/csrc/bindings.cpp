@@ -364,6 +364,25 @@ Tensor rmsnorm_bwd(const Tensor& dy, const Tensor& x, const Tensor& w, const Ten
   return dx;
 }
 
+// Backward of the norms of the q and k heads in place in g_qkv [T, (nh + 2 nkv) * hd]; the weights' gradients are added to dwq, dwk.
+void qk_norm_bwd_(Tensor g_qkv, const Tensor& pre_q, const Tensor& pre_k, const Tensor& rstd_q, const Tensor& rstd_k, const Tensor& wq,
+                  const Tensor& wk, Tensor dwq, Tensor dwk, int64_t nh, int64_t nkv, int64_t hd) {
+  for (const Tensor& t : {g_qkv, pre_q, pre_k, wq, wk}) CHECK_BF16(t);
+  for (const Tensor& t : {rstd_q, rstd_k, dwq, dwk}) CHECK_F32(t);
+  const int64_t T = g_qkv.size(0);
+  TORCH_CHECK(g_qkv.dim() == 2 && g_qkv.stride(1) == 1 && g_qkv.size(1) == (nh + 2 * nkv) * hd && pre_q.is_contiguous() && pre_k.is_contiguous() &&
+              pre_q.numel() == T * nh * hd && pre_k.numel() == T * nkv * hd && rstd_q.is_contiguous() && rstd_k.is_contiguous() &&
+              rstd_q.numel() == T * nh && rstd_k.numel() == T * nkv, "qk_norm_bwd: g_qkv [T, (nh + 2 nkv) * hd], heads in front of the norm, 1 / rms");
+  for (const Tensor& t : {wq, wk, dwq, dwk}) TORCH_CHECK(t.is_contiguous() && t.numel() == hd, "qk_norm_bwd: weights [hd]");
+  const c10::cuda::CUDAGuard guard(g_qkv.device());
+  if (T == 0) return;
+  Tensor partial = at::empty({2, (int64_t)vb_rmsnorm_bwd_blocks((int)T), hd}, rstd_q.options());
+  count(3);
+  CHECK_RC(vb_qk_norm_bwd(g_qkv.data_ptr(), g_qkv.stride(0), pre_q.data_ptr(), pre_k.data_ptr(), rstd_q.data_ptr<float>(),
+                          rstd_k.data_ptr<float>(), wq.data_ptr(), wk.data_ptr(), dwq.data_ptr<float>(), dwk.data_ptr<float>(),
+                          partial.data_ptr<float>(), (int)T, (int)nh, (int)nkv, (int)hd, cur_stream()), "vb_qk_norm_bwd");
+}
+
 // In-place rotary embedding on x [T, nheads, hd] (a view with row stride x.stride(0)).
 void rope_(Tensor x, const Tensor& pos, const Tensor& cos_t, const Tensor& sin_t, bool backward) {
   CHECK_BF16(x);
@@ -1258,6 +1277,7 @@ TORCH_LIBRARY(verl_b200, m) {
   m.def("paged_decode_grouped", &paged_decode_grouped);
   m.def("rope_kv_append_", &rope_kv_append_);
   m.def("qk_norm_rope_", &qk_norm_rope_);
+  m.def("qk_norm_bwd_", &qk_norm_bwd_);
   m.def("sample", &sample);
   m.def("sample_topkp", &sample_topkp);
   m.def("grpo_advantage", &grpo_advantage);

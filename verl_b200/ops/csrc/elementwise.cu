@@ -95,60 +95,173 @@ __global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __
   }
 }
 
+// The same for many rows of at most 4096: a warp per row that keeps the row in registers, so nothing is read twice and no barrier is met.
+// The sums are those of the kernel above to the bit, because a router behind a norm turns a changed last bit into another choice of
+// experts: NW = 4 or 8 (the warps it has) partial sums per lane, each over every NW-th piece of 32 x 16 bytes, halved lane by lane
+// (16, 8, 4, 2, 1) and then warp by warp (4, 2, 1); the halving steps exchange the partial sums they do not keep, 12 shuffles in place
+// of 43. With residual, 16,000 rows of 896 / 2048 / 3584: 28.1 -> 22.8, 59.2 -> 48.7, 98.8 -> 92.1 us (5.0, 5.4, 5.0 TB/s).
+template <int J, int NW>
+__global__ void __launch_bounds__(128)
+rmsnorm_fwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ residual, const __nv_bfloat16* __restrict__ w,
+                        __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd_out, int T, int H,
+                        float eps) {
+  const long long row = blockIdx.x * static_cast<long long>(blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= T) return;
+  const int lane = threadIdx.x & 31, nv = H >> 3;
+  const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * H);
+  const bf16x8* wv = reinterpret_cast<const bf16x8*>(w);
+  bf16x8 v[J], g[J];  // g: first the residual, then the weight; every load of an array is issued before the first is used
+#pragma unroll
+  for (int j = 0; j < J; ++j)
+    if (j * 32 + lane < nv) v[j] = xr[j * 32 + lane];
+  if (residual != nullptr) {
+    const bf16x8* rr = reinterpret_cast<const bf16x8*>(residual + row * H);
+    bf16x8* ro = reinterpret_cast<bf16x8*>(res_out + row * H);
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+      if (j * 32 + lane < nv) g[j] = rr[j * 32 + lane];
+#pragma unroll
+    for (int j = 0; j < J; ++j) {
+      float a[8], b[8];
+      unpack8(v[j], a);
+      unpack8(g[j], b);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] += b[i];
+      v[j] = pack8(a);
+    }
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+      if (j * 32 + lane < nv) ro[j * 32 + lane] = v[j];
+  }
+#pragma unroll
+  for (int j = 0; j < J; ++j)
+    if (j * 32 + lane < nv) g[j] = wv[j * 32 + lane];
+  float p[NW];
+#pragma unroll
+  for (int k = 0; k < NW; ++k) p[k] = 0.f;
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    if (j * 32 + lane < nv) {
+      float a[8];
+      unpack8(v[j], a);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) p[j % NW] += a[i] * a[i];
+    }
+  }
+  // lanes 16 and 8 (and 4) apart: each keeps half of the partial sums
+#pragma unroll
+  for (int n = NW / 2, o = 16; n > 0; n >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < n; ++k) {
+      const float other = __shfl_xor_sync(0xffffffffu, up ? p[k] : p[n + k], o);
+      p[k] = (up ? p[n + k] : p[k]) + other;
+    }
+  }
+  float ss = p[0];
+#pragma unroll
+  for (int o = 16 / NW; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+#pragma unroll
+  for (int o = 16; o >= 32 / NW; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  const float rstd = rsqrtf(ss / H + eps);
+  if (lane == 0 && rstd_out) rstd_out[row] = rstd;
+  bf16x8* yr = reinterpret_cast<bf16x8*>(y + row * H);
+#pragma unroll
+  for (int j = 0; j < J; ++j) {
+    if (j * 32 + lane < nv) {
+      float a[8], b[8];
+      unpack8(v[j], a);
+      unpack8(g[j], b);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = a[i] * rstd * b[i];
+      yr[j * 32 + lane] = pack8(a);
+    }
+  }
+}
+
 // dx = rstd * (dy*w) - x * rstd^3 * mean(dy*w*x) (+ dres_in);  dw partial per block -> scratch[grid, H].
-// Each block walks rows blockIdx.x, +gridDim.x, ...; each thread owns fixed column vectors so the dw
-// partial stays in registers (H <= 8 * VEC_PER_THREAD * blockDim.x).
-template <int VPT>
+// A block walks over groups of RB rows; each thread owns fixed column vectors so the dw partial stays in registers
+// (H <= 8 * VPT * blockDim.x). The rows of a group are loaded together and share one exchange over the block, which alternates between
+// two buffers and so needs one barrier: with a row and two barriers at a time the block waited for memory once per row. With the fold of
+// the partial sums, 16,000 rows of 896 / 3584: 58.4 -> 36.0, 165.5 -> 134.9 us.
+template <int VPT, int RB>
 __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                                    const __nv_bfloat16* __restrict__ dres_in, __nv_bfloat16* __restrict__ dx,
                                    float* __restrict__ dw_partial, int T, int H) {
-  __shared__ float red[32];
-  const int nv = H >> 3;
+  __shared__ float red[2][RB][8];
+  const int nv = H >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;  // at most 8
   float dwacc[VPT][8];
-  float wreg[VPT][8];
+  bf16x8 wreg[VPT];
 #pragma unroll
   for (int v = 0; v < VPT; ++v) {
     const int i = threadIdx.x + v * blockDim.x;
 #pragma unroll
     for (int j = 0; j < 8; ++j) dwacc[v][j] = 0.f;
-    if (i < nv) unpack8(reinterpret_cast<const bf16x8*>(w)[i], wreg[v]);
+    if (i < nv) wreg[v] = reinterpret_cast<const bf16x8*>(w)[i];
   }
-  for (long long row = blockIdx.x; row < T; row += gridDim.x) {
-    const bf16x8* dyr = reinterpret_cast<const bf16x8*>(dy + row * H);
-    const bf16x8* xr = reinterpret_cast<const bf16x8*>(x + row * H);
-    const float rs = rstd[row];
-    float dyv[VPT][8], xv[VPT][8];
-    float dot = 0.f;
+  int buf = 0;
+  for (long long row0 = static_cast<long long>(blockIdx.x) * RB; row0 < T; row0 += static_cast<long long>(gridDim.x) * RB, buf ^= 1) {
+    bf16x8 dyv[RB][VPT], xv[RB][VPT], dr[RB][VPT];
+    float rs[RB], dot[RB];
 #pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int i = threadIdx.x + v * blockDim.x;
-      if (i < nv) {
-        unpack8(dyr[i], dyv[v]);
-        unpack8(xr[i], xv[v]);
+    for (int r = 0; r < RB; ++r) {
+      const long long row = min(row0 + r, static_cast<long long>(T) - 1);  // rows past the end repeat the last one and count nothing
+      rs[r] = rstd[row];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          dot += dyv[v][j] * wreg[v][j] * xv[v][j];
-          dwacc[v][j] += dyv[v][j] * xv[v][j] * rs;
+      for (int v = 0; v < VPT; ++v) {
+        const int i = threadIdx.x + v * blockDim.x;
+        if (i < nv) {
+          dyv[r][v] = reinterpret_cast<const bf16x8*>(dy + row * H)[i];
+          xv[r][v] = reinterpret_cast<const bf16x8*>(x + row * H)[i];
+          if (dres_in != nullptr) dr[r][v] = reinterpret_cast<const bf16x8*>(dres_in + row * H)[i];
         }
       }
     }
-    dot = block_sum(dot, red);
-    const float c = dot * rs * rs * rs / H;
 #pragma unroll
-    for (int v = 0; v < VPT; ++v) {
-      const int i = threadIdx.x + v * blockDim.x;
-      if (i < nv) {
-        float o[8];
+    for (int r = 0; r < RB; ++r) {
+      dot[r] = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rs * dyv[v][j] * wreg[v][j] - xv[v][j] * c;
-        if (dres_in) {
-          float d[8];
-          unpack8(reinterpret_cast<const bf16x8*>(dres_in + row * H)[i], d);
+      for (int v = 0; v < VPT; ++v) {
+        if (static_cast<int>(threadIdx.x + v * blockDim.x) < nv) {
+          float a[8], b[8], c[8];
+          unpack8(dyv[r][v], a);
+          unpack8(xv[r][v], b);
+          unpack8(wreg[v], c);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += d[j];
+          for (int j = 0; j < 8; ++j) {
+            dot[r] += a[j] * c[j] * b[j];
+            if (row0 + r < T) dwacc[v][j] += a[j] * b[j] * rs[r];
+          }
         }
-        reinterpret_cast<bf16x8*>(dx + row * H)[i] = pack8(o);
+      }
+      dot[r] = warp_sum(dot[r]);
+      if (lane == 0) red[buf][r][warp] = dot[r];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < RB; ++r) {
+      if (row0 + r >= T) break;
+      float d = 0.f;
+      for (int k = 0; k < warps; ++k) d += red[buf][r][k];
+      const float c = d * rs[r] * rs[r] * rs[r] / H;
+#pragma unroll
+      for (int v = 0; v < VPT; ++v) {
+        const int i = threadIdx.x + v * blockDim.x;
+        if (i < nv) {
+          float a[8], b[8], g[8], o[8];
+          unpack8(dyv[r][v], a);
+          unpack8(xv[r][v], b);
+          unpack8(wreg[v], g);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] = rs[r] * a[j] * g[j] - b[j] * c;
+          if (dres_in != nullptr) {
+            unpack8(dr[r][v], a);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] += a[j];
+          }
+          reinterpret_cast<bf16x8*>(dx + (row0 + r) * H)[i] = pack8(o);
+        }
       }
     }
   }
@@ -163,14 +276,100 @@ __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const _
   }
 }
 
-// dw[h] (+)= sum_b partial[b, h]
-__global__ void colsum_kernel(const float* __restrict__ partial, float* __restrict__ out, int B, int H,
-                              int accumulate) {
-  const int h = blockIdx.x * blockDim.x + threadIdx.x;
-  if (h >= H) return;
+// dw[h] (+)= sum_b partial[b, h]: 32 columns per block, every warp an eighth of the rows, folded in a fixed order: 7 us for 592 rows of
+// 896. (A thread per column walked all rows one after the other on four blocks: 24 us.)
+__global__ void __launch_bounds__(256)
+colsum_kernel(const float* __restrict__ partial, float* __restrict__ out, int B, int H, int accumulate) {
+  __shared__ float part[8][33];
+  const int h = blockIdx.x * 32 + (threadIdx.x & 31), warp = threadIdx.x >> 5;
   float s = 0.f;
-  for (int b = 0; b < B; ++b) s += partial[static_cast<long long>(b) * H + h];
+  if (h < H) {
+#pragma unroll 8
+    for (int b = warp; b < B; b += 8) s += partial[static_cast<long long>(b) * H + h];
+  }
+  part[warp][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (warp != 0 || h >= H) return;
+  s = 0.f;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s += part[k][threadIdx.x];
   out[h] = accumulate ? out[h] + s : s;
+}
+
+// Backward of the norms of the q and k heads, in place in the gradient of the projection [T, (nh + 2 nkv) * hd]. L lanes hold a head
+// (16 bytes each), a group of them takes RB heads at a time; the partial sums of the weights' gradients leave per block,
+// partial[0] q, partial[1] k, each [gridDim.x, hd]. In place it needs no copies of q and k to contiguous rows and back: 63 us now, with
+// the copies and a block per head 335 + 126 us for the q heads alone (8 sequences, 32 + 4 heads of 128).
+template <int L>
+__global__ void __launch_bounds__(256)
+qk_norm_bwd_kernel(__nv_bfloat16* __restrict__ g_qkv, long long ld, const __nv_bfloat16* __restrict__ pre_q,
+                   const __nv_bfloat16* __restrict__ pre_k, const float* __restrict__ rstd_q, const float* __restrict__ rstd_k,
+                   const __nv_bfloat16* __restrict__ wq, const __nv_bfloat16* __restrict__ wk, float* __restrict__ partial, int T, int nh,
+                   int nkv, int hd) {
+  constexpr int GROUPS = 256 / L, RB = 4;
+  __shared__ float s_dw[GROUPS][8 * L + 4];
+  const int l = threadIdx.x % L, group = threadIdx.x / L;
+  const bool on = l < (hd >> 3);
+  for (int kind = 0; kind < 2; ++kind) {
+    const int heads = kind ? nkv : nh;
+    const __nv_bfloat16* pre = kind ? pre_k : pre_q;
+    const float* rstd = kind ? rstd_k : rstd_q;
+    float wv[8], dw[8];
+    bf16x8 raw{};
+    if (on) raw = reinterpret_cast<const bf16x8*>(kind ? wk : wq)[l];
+    unpack8(raw, wv);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dw[j] = 0.f;
+    const long long items = static_cast<long long>(T) * heads;
+    const long long stride = static_cast<long long>(gridDim.x) * GROUPS * RB;
+    // every lane of a warp makes the same number of turns: the bound is the block's first item
+    for (long long base = static_cast<long long>(blockIdx.x) * GROUPS * RB; base < items; base += stride) {
+      bf16x8 dy[RB], x[RB];
+      float rs[RB];
+      bf16x8* at[RB];
+#pragma unroll
+      for (int r = 0; r < RB; ++r) {
+        const long long it = base + static_cast<long long>(r) * GROUPS + group;
+        const bool ok = it < items;
+        const long long t = ok ? it / heads : 0;
+        const int h = ok ? static_cast<int>(it - t * heads) : 0;
+        at[r] = reinterpret_cast<bf16x8*>(g_qkv + t * ld + static_cast<long long>(kind ? nh + h : h) * hd) + l;
+        dy[r] = bf16x8{};
+        x[r] = bf16x8{};
+        rs[r] = ok ? rstd[it] : 0.f;
+        if (ok && on) {
+          dy[r] = *at[r];
+          x[r] = reinterpret_cast<const bf16x8*>(pre + it * hd)[l];
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < RB; ++r) {
+        float a[8], b[8], dot = 0.f;
+        unpack8(dy[r], a);
+        unpack8(x[r], b);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          dot += a[j] * wv[j] * b[j];
+          dw[j] += a[j] * b[j] * rs[r];
+        }
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        const float c = dot * rs[r] * rs[r] * rs[r] / hd;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) a[j] = rs[r] * a[j] * wv[j] - b[j] * c;
+        if (on && base + static_cast<long long>(r) * GROUPS + group < items) *at[r] = pack8(a);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s_dw[group][l * 8 + j] = dw[j];
+    __syncthreads();
+    for (int i = threadIdx.x; i < hd; i += 256) {
+      float s = 0.f;
+      for (int k = 0; k < GROUPS; ++k) s += s_dw[k][i];
+      partial[(static_cast<long long>(kind) * gridDim.x + blockIdx.x) * hd + i] = s;
+    }
+    __syncthreads();
+  }
 }
 
 // ------------------------------------------------------------------------------------------ RoPE
@@ -417,6 +616,27 @@ int vb_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, 
                    int H, float eps, cudaStream_t s) {
   if (T == 0) return 0;
   if (H % 8) return -1;
+  // A warp per row where rows fill the chip. With fewer a block per row has the shorter chain of loads: with residual, 64 rows of 896 / 2048
+  // / 3584 2.2, 2.4, 2.8 us against 2.3, 3.0, 4.4 us, 320 rows 2.5, 3.5, 4.4 against 2.6, 3.2, 4.8 us; 1,000 rows 3.5, 5.6, 8.7 against
+  // 3.0, 4.3, 7.8 us. Rows of one piece per lane (heads of a norm) 1.9 against 2.1 us at 64 rows already.
+  if (H <= 4096 && (T >= 640 || H <= 256)) {
+    const int rows = T >= 1184 ? 4 : 1;  // few rows: a block each, so that they are spread over the chip
+    const int pieces = (H / 8 + 31) / 32;
+#define VB_RF(J, NW)                                                                                                                     \
+  rmsnorm_fwd_warp_kernel<J, NW><<<(T + rows - 1) / rows, 32 * rows, 0, s>>>(                                                            \
+      reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(residual), reinterpret_cast<const __nv_bfloat16*>(w), \
+      reinterpret_cast<__nv_bfloat16*>(y), reinterpret_cast<__nv_bfloat16*>(res_out), rstd, T, H, eps)
+    if (H < 2048) {
+      if (pieces <= 1) VB_RF(1, 4);
+      else if (pieces <= 4) VB_RF(4, 4);
+      else VB_RF(8, 4);
+    } else {
+      if (pieces <= 8) VB_RF(8, 8);
+      else VB_RF(16, 8);
+    }
+#undef VB_RF
+    return static_cast<int>(cudaGetLastError());
+  }
   const int threads = H >= 2048 ? 256 : 128;
   rmsnorm_fwd_kernel<<<T, threads, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(x), reinterpret_cast<const __nv_bfloat16*>(residual),
@@ -436,20 +656,41 @@ int vb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rs
   if (T == 0) return 0;
   if (H % 8) return -1;
   const int blocks = vb_rmsnorm_bwd_blocks(T);
-  const int threads = 256;
   const int nv = H / 8;
+  const int threads = nv <= 32 ? 32 : nv <= 64 ? 64 : nv <= 128 ? 128 : 256;
   const int vpt = (nv + threads - 1) / threads;
-#define VB_RB(V)                                                                                               \
-  rmsnorm_bwd_kernel<V><<<blocks, threads, 0, s>>>(                                                             \
+  const bool few = T <= 2 * blocks;  // one or two rows per block: no groups
+#define VB_RB(V, RB)                                                                                           \
+  rmsnorm_bwd_kernel<V, RB><<<blocks, threads, 0, s>>>(                                                             \
       reinterpret_cast<const __nv_bfloat16*>(dy), reinterpret_cast<const __nv_bfloat16*>(x),                   \
       reinterpret_cast<const __nv_bfloat16*>(w), rstd, reinterpret_cast<const __nv_bfloat16*>(dres_in),        \
       reinterpret_cast<__nv_bfloat16*>(dx), scratch, T, H)
-  if (vpt <= 1) VB_RB(1);
-  else if (vpt <= 2) VB_RB(2);
-  else if (vpt <= 4) VB_RB(4);
+  if (vpt <= 1 && few) VB_RB(1, 1);
+  else if (vpt <= 1) VB_RB(1, 4);
+  else if (vpt <= 2 && few) VB_RB(2, 1);
+  else if (vpt <= 2) VB_RB(2, 4);
+  else if (vpt <= 4) VB_RB(4, 1);
   else return -2;  // H > 8192
 #undef VB_RB
-  colsum_kernel<<<cdiv_ll(H, 256), 256, 0, s>>>(scratch, dw, blocks, H, accumulate_dw);
+  colsum_kernel<<<(H + 31) / 32, 256, 0, s>>>(scratch, dw, blocks, H, accumulate_dw);
+  return static_cast<int>(cudaGetLastError());
+}
+
+// partial: 2 * vb_rmsnorm_bwd_blocks(T) * hd floats; dwq, dwk are added to
+int vb_qk_norm_bwd(void* g_qkv, long long ld, const void* pre_q, const void* pre_k, const float* rstd_q, const float* rstd_k, const void* wq,
+                   const void* wk, float* dwq, float* dwk, float* partial, int T, int nh, int nkv, int hd, cudaStream_t s) {
+  if (T == 0) return 0;
+  if ((hd % 8) || hd > 256 || (ld % 8)) return -1;
+  for (const void* p : {static_cast<const void*>(g_qkv), pre_q, pre_k, wq, wk})
+    if (reinterpret_cast<uintptr_t>(p) & 15) return -2;
+  const int blocks = vb_rmsnorm_bwd_blocks(T);
+  auto bf = [](const void* p) { return reinterpret_cast<const __nv_bfloat16*>(p); };
+  auto* g = reinterpret_cast<__nv_bfloat16*>(g_qkv);
+  if (hd <= 64) qk_norm_bwd_kernel<8><<<blocks, 256, 0, s>>>(g, ld, bf(pre_q), bf(pre_k), rstd_q, rstd_k, bf(wq), bf(wk), partial, T, nh, nkv, hd);
+  else if (hd <= 128) qk_norm_bwd_kernel<16><<<blocks, 256, 0, s>>>(g, ld, bf(pre_q), bf(pre_k), rstd_q, rstd_k, bf(wq), bf(wk), partial, T, nh, nkv, hd);
+  else qk_norm_bwd_kernel<32><<<blocks, 256, 0, s>>>(g, ld, bf(pre_q), bf(pre_k), rstd_q, rstd_k, bf(wq), bf(wk), partial, T, nh, nkv, hd);
+  colsum_kernel<<<(hd + 31) / 32, 256, 0, s>>>(partial, dwq, blocks, hd, 1);
+  colsum_kernel<<<(hd + 31) / 32, 256, 0, s>>>(partial + static_cast<long long>(blocks) * hd, dwk, blocks, hd, 1);
   return static_cast<int>(cudaGetLastError());
 }
 

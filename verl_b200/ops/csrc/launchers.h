@@ -55,6 +55,8 @@ int vb_lmhead_dlogits(const void* hidden, const void* weight_chunk, const long l
 int vb_rmsnorm_fwd(const void* x, const void* residual, const void* w, void* y, void* res_out, float* rstd, int T,
                    int H, float eps, cudaStream_t s);
 int vb_rmsnorm_bwd_blocks(int T);
+int vb_qk_norm_bwd(void* g_qkv, long long ld, const void* pre_q, const void* pre_k, const float* rstd_q, const float* rstd_k, const void* wq,
+                   const void* wk, float* dwq, float* dwk, float* partial, int T, int nh, int nkv, int hd, cudaStream_t s);
 int vb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres_in, void* dx,
                    float* dw, float* scratch, int T, int H, int accumulate_dw, cudaStream_t s);
 int vb_rope(void* x, const int* pos, const float* cos_t, const float* sin_t, int T, int nheads, int hd, long long ld,

@@ -633,6 +633,19 @@ def qk_norm_rope_(qkv: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin: 
     return (qp, kp, rq, rk) if save else None
 
 
+def qk_norm_bwd_(g_qkv, q_pre, k_pre, rstd_q, rstd_k, wq, wk, dwq, dwk, nh: int, nkv: int, hd: int) -> None:
+    """Backward of the norms of ``qk_norm_rope_`` in place in ``g_qkv`` [T, (nh + 2 nkv) * hd] (rotated back already); the gradients of the
+    two weights are added to ``dwq`` / ``dwk`` (fp32)."""
+    if (g_qkv.is_cuda and g_qkv.dtype == torch.bfloat16 and hd % 8 == 0 and hd <= 256 and g_qkv.stride(0) % 8 == 0
+            and all(t.data_ptr() % 16 == 0 for t in (g_qkv, q_pre, k_pre, wq, wk))):
+        _ops().qk_norm_bwd_(g_qkv, q_pre, k_pre, rstd_q, rstd_k, wq, wk, dwq, dwk, int(nh), int(nkv), int(hd))
+        return
+    T = g_qkv.shape[0]
+    gq, gk = g_qkv[:, : nh * hd].view(T, nh, hd), g_qkv[:, nh * hd : (nh + nkv) * hd].view(T, nkv, hd)
+    gq.copy_(rms_norm_bwd(gq.reshape(T * nh, hd).contiguous(), q_pre, wq, rstd_q, None, dwq, True).view(T, nh, hd))
+    gk.copy_(rms_norm_bwd(gk.reshape(T * nkv, hd).contiguous(), k_pre, wk, rstd_k, None, dwk, True).view(T, nkv, hd))
+
+
 def paged_decode_attention(q, k_cache, v_cache, block_table, ctx_len, scale: Optional[float] = None, groups=None):
     """One query token per sequence against a paged cache [num_blocks, block_size, nkv, hd].
 
