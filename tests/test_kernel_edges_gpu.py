@@ -505,3 +505,27 @@ def test_qk_norm_backward_in_place(ops, T, nh, nkv, hd):
         (xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-6) * wd).backward(gq[:, sl].reshape(-1, hd).double())
         assert rel(out[:, sl].reshape(-1, hd), xd.grad) < 4e-3
         assert rel(dw[i] - 1, wd.grad) < 1e-5
+
+
+# ------------------------------------------------------------------------------------------------ a group's heads over several CTAs
+@pytest.mark.parametrize("nh,nkv,hd,lens", [(64, 32, 64, [700, 600]), (7, 1, 64, [1, 64, 65, 300]), (48, 16, 128, [513, 97, 700, 640]),
+                                            (14, 2, 128, [31, 33, 129])])
+def test_attention_backward_over_shares_of_heads(ops, nh, nkv, hd, lens):
+    """One CTA for all heads of a group, two, and one per head; without parents, so that a single CTA stores dK and dV."""
+    from verl_b200.ops import functional as F
+
+    T = sum(lens)
+    cu = np.cumsum([0] + lens).tolist()
+    g = torch.Generator(device=DEV).manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    q, k, v, dout = rnd(T, nh, hd), rnd(T, nkv, hd), rnd(T, nkv, hd), rnd(T, nh, hd)
+    cu_t = torch.tensor(cu, dtype=torch.int32, device=DEV)
+    out, lse = F.attention_varlen(q, k, v, cu_t, max(lens))
+    got = F.attention_varlen_bwd(dout, q, k, v, out, lse, cu_t, max(lens))
+    ref = [t.double().requires_grad_(True) for t in (q, k, v)]
+    want = _attention64(*ref, [list(range(a, a + i + 1)) for a, n in zip(cu, lens) for i in range(n)], hd**-0.5)
+    assert rel(out, want.detach()) < 6e-3
+    want.backward(dout.double())
+    for x, w in zip(got, ref):
+        assert rel(x, w.grad) < 1.5e-2  # dS is rounded to bf16 and its terms cancel
+    assert int(ops.gemm_status()) == 0

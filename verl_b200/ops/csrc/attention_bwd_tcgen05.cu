@@ -1,7 +1,7 @@
 // Causal GQA attention backward over packed (varlen) sequences on tcgen05 tensor cores (head_dim 64 and 128).
 //
-// One CTA = one (sequence, block of 128 keys, KV head). K and V of the block stay in shared memory and dK, dV stay in
-// TMEM for the whole CTA, which walks over every query head of the GQA group and every block of 64 queries at or
+// One CTA = one (sequence, block of 128 keys, KV head, share of the GQA group's query heads). K and V of the block stay in shared memory
+// and dK, dV stay in TMEM for the whole CTA, which walks over its query heads and every block of 64 queries at or
 // below the diagonal. Everything is computed in the transposed frame so that the 128 keys are the M (TMEM lane)
 // dimension and softmax threads own one key row each:
 //
@@ -10,25 +10,35 @@
 //   P^T  = exp2(S^T * c - lse2[q]) (causal),   dS^T = P^T o (dP^T - D[q]) * scale          -> bf16, shared memory
 //   dV  += P^T  dO           [128 keys, hd]     A = P^T  (K-major)   B = dO (MN-major)       TMEM-resident
 //   dK  += dS^T Q            [128 keys, hd]     A = dS^T (K-major)   B = Q  (MN-major)       TMEM-resident
-//   dQ^T = K^T dS^T          [hd, 64 q]         A = K  (MN-major)    B = dS^T (MN-major)     -> fp32 atomics into dQ
+//   dQ^T = K^T dS^T          [hd, 64 q]         A = K  (MN-major)    B = dS^T (MN-major)     -> added to dQ in fp32
 //
-// dQ^T has two TMEM buffers: the atomics of step i run after the softmax warps have handed P^T / dS^T of step i + 1 to
+// dQ^T has two TMEM buffers: the additions of step i run after the softmax warps have handed P^T / dS^T of step i + 1 to
 // the MMA warp, i.e. under the tensor-core work of step i + 1 instead of in front of it.
 // Grid = (KV head, sequence, key block counted from the END of the sequence, longest first): blocks are handed out in
 // order of decreasing work (the first key block meets every query block, the last one only its own), which keeps the
 // tail of the launch short.
 //
-//   warp 0      TMA: K, V once; Q and dO tiles through a 2-stage ring
+//   warp 0      TMA: K, V once; Q and dO tiles through a ring of 3 (head_dim 128) or 4 stages: under the load of all SMs a tile takes
+//               longer than half a step to arrive; with two stages 5 x 3072 tokens, 28 / 4 heads, took 1723 us, now 1614
 //   warp 1      MMA issue (one elected thread)
 //   warps 2..9  two threads per key row (32 of the step's 64 queries each): tcgen05.ld S^T / dP^T -> P^T, dS^T ->
-//               swizzled shared memory; drain dQ^T with coalesced red.add (lanes = 32 consecutive head-dim elements of
-//               one query); final dV (warps 2..5) / dK (warps 6..9) store
+//               swizzled shared memory; drain dQ^T: a warp's 32 queries x 32 head-dim elements transposed through shared memory
+//               into one TMA reduction (32 red.add per thread and step in place of it: 1862 us for 5 x 3072 tokens, now
+//               1723); final dV (warps 2..5) / dK (warps 6..9) store
 // D[q] = sum_d dO[q,d] O[q,d] comes from a small pre-pass; dQ, dK and dV leave in fp32 and a last pass turns them into the bf16 gradient
 // of the projection output, undoing the rotary embedding on the way (attn_bwd_finish_kernel).
 //
 // Head_dim 64: dQ^T has 64 rows, but the tensor core's M stays 128 (with M = 64 the rows would sit on half of the lanes of every warp):
 // A's second panel of 64 rows is the V tile, which lies right behind K in shared memory with the stride of a K panel, and the lanes
 // 64..127 of the result are never read. 4 of 24 MMAs of a step are spent on them.
+//
+// A step takes microseconds and the first key block of a sequence meets every query block of every head of its group, so that a launch
+// could not end before that one CTA: 14 heads of 64 over 2 KV heads, 12 sequences of about 1,000 tokens, had 192 CTAs of up to 160 steps
+// where the average SM has 82 to do. The group's heads are therefore dealt to several CTAs (hsplit, see vb_attn_bwd) which add their
+// dK / dV in fp32: 16-byte reductions, four neighbouring elements of a key row. Whole backward, before all three changes and now:
+// that case 470 -> 295 us, two prompts with five continuations each (7,900 tokens, 28 / 4 heads of 128) 984 -> 800, 5 x 3072 1862 -> 1614,
+// 8192 2491 -> 1983 us. A step of 64 queries still takes 2.5 us of which the tensor pipe works 1.1: S^T / dP^T of the next step, the
+// softmax and the products of this one follow each other, and TMEM (512 columns at head_dim 128) has no room for a second S^T / dP^T.
 //
 // With `parent` (see attention_fwd_tcgen05.cu) a key block of a prompt has queries in several sequences. They are dealt to one CTA per
 // (key block, query sequence): blockIdx.y = s is sequence s against its own keys, num_seqs + s is sequence s against those of parent[s],
@@ -48,10 +58,11 @@ struct AttnBwdParams {
   const int* cu_seqlens;
   const int* parent;   // [num_seqs] or null
   int num_seqs, nh, nkv, total_tokens, max_tiles;  // max_tiles: key blocks of the longest sequence
+  int hsplit, heads_per;  // CTAs that share a group's query heads, heads of each
   const float* lse;    // [nh, T] natural log
   const float* delta;  // [nh, T]
   float* dq32;         // [T, nh*hd] fp32, zero on entry
-  float* dk32;         // [T, nkv*hd] fp32; zero on entry with `parent`
+  float* dk32;         // [T, nkv*hd] fp32; zero on entry with `parent` or hsplit > 1
   float* dv32;
   float scale, scale_log2;
   int* status;
@@ -59,48 +70,59 @@ struct AttnBwdParams {
 
 template <int HD>
 struct AttnBwdSmem {
+  static constexpr int STAGES = HD == 128 ? 3 : 4;
   static constexpr int KV_BYTES = AB_BK * HD * 2;   // 32 KB each
   static constexpr int QO_BYTES = AB_BQ * HD * 2;   // 16 KB each, per stage
   static constexpr int PS_BYTES = AB_BK * AB_BQ * 2;  // 16 KB each
   static constexpr int OFF_K = 0;
   static constexpr int OFF_V = OFF_K + KV_BYTES;
-  static constexpr int OFF_Q = OFF_V + KV_BYTES;          // 2 stages
-  static constexpr int OFF_DO = OFF_Q + 2 * QO_BYTES;     // 2 stages
-  static constexpr int OFF_P = OFF_DO + 2 * QO_BYTES;
+  static constexpr int OFF_Q = OFF_V + KV_BYTES;
+  static constexpr int OFF_DO = OFF_Q + STAGES * QO_BYTES;
+  static constexpr int OFF_P = OFF_DO + STAGES * QO_BYTES;
   static constexpr int OFF_DS = OFF_P + PS_BYTES;
-  static constexpr int OFF_VEC = OFF_DS + PS_BYTES;       // per softmax warp (8): [2 steps][lse2 | delta][32] fp32
-  static constexpr int OFF_BAR = OFF_VEC + 8 * 2 * 2 * 32 * 4;
-  static constexpr int TOTAL = OFF_BAR + 128 + 1024;
+  static constexpr int OFF_VEC = OFF_DS + PS_BYTES;       // per softmax warp (8): [lse2 | delta][32] fp32
+  static constexpr int OFF_DQ = OFF_VEC + 8 * 2 * 32 * 4;  // per softmax warp: 32 queries x 32 head-dim elements, fp32
+  static constexpr int DQ_PIECE = 32 * 32 * 4;
+  static constexpr int OFF_BAR = OFF_DQ + 8 * DQ_PIECE;
+  // no alignment slack and no static shared memory: the dynamic window then starts 1024-byte aligned, which the kernel verifies
+  static constexpr int TOTAL = OFF_BAR + 128;
+  static_assert(TOTAL <= 232448, "shared memory of a CTA");
 };
 
 template <int HD>
 __global__ void __launch_bounds__(AB_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                 const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_do,
-                const AttnBwdParams p) {
+                const __grid_constant__ CUtensorMap tm_dq, const AttnBwdParams p) {
   using L = AttnBwdSmem<HD>;
   constexpr int PANELS = HD / 64;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  constexpr int STAGES = L::STAGES;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = smem_raw;
+  if ((smem_u32(smem) & 1023u) != 0u) {  // the swizzled TMA / MMA layouts need 1024-byte aligned tiles
+    if (threadIdx.x == 0) atomicExch(p.status, 9);
+    return;
+  }
   uint8_t* sK = smem + L::OFF_K;
   uint8_t* sV = smem + L::OFF_V;
   uint8_t* sQ = smem + L::OFF_Q;
   uint8_t* sDO = smem + L::OFF_DO;
   uint8_t* sP = smem + L::OFF_P;
   uint8_t* sDS = smem + L::OFF_DS;
-  float* sVec = reinterpret_cast<float*>(smem + L::OFF_VEC);  // [8 warps][2 steps][lse2 | delta][32]
+  float* sVec = reinterpret_cast<float*>(smem + L::OFF_VEC);  // [8 warps][lse2 | delta][32]
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
   uint64_t* kv_full = bars;        // 1
-  uint64_t* qdo_full = bars + 1;   // 2
-  uint64_t* qdo_empty = bars + 3;  // 2
-  uint64_t* bar_sdp = bars + 5;    // S^T, dP^T ready
-  uint64_t* bar_pds = bars + 6;    // P^T, dS^T written (4 warps)
-  uint64_t* bar_dq = bars + 7;     // dV, dK, dQ^T MMAs of a step done
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 8);
+  uint64_t* bar_sdp = bars + 1;    // S^T, dP^T ready
+  uint64_t* bar_pds = bars + 2;    // P^T, dS^T written (8 warps)
+  uint64_t* bar_dq = bars + 3;     // dV, dK, dQ^T MMAs of a step done
+  uint64_t* qdo_full = bars + 4;   // [STAGES]
+  uint64_t* qdo_empty = bars + 8;  // [STAGES]
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 12);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kvh = blockIdx.x;
+  const int kvh = static_cast<int>(blockIdx.x) / p.hsplit, part = static_cast<int>(blockIdx.x) - kvh * p.hsplit;
   const int G = p.nh / p.nkv;
+  const int head0 = kvh * G + part * p.heads_per, heads = min(p.heads_per, G - part * p.heads_per);  // at least one: see the launcher
   // query sequence, and the sequence of its keys: itself, or its parent
   const bool cross = static_cast<int>(blockIdx.y) >= p.num_seqs;
   const int qs = static_cast<int>(blockIdx.y) - (cross ? p.num_seqs : 0);
@@ -112,8 +134,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int ntiles = (keylen + AB_BK - 1) / AB_BK;
   if (ntiles > p.max_tiles && blockIdx.z == 0 && threadIdx.x == 0) atomicExch(p.status, ST_BAD_ARGS);  // max_seqlen too small
   if (from_end >= ntiles || seqlen <= 0) return;  // shorter sequence
-  // dK / dV of this block are also written by CTAs of other query sequences
-  const bool shared_keys = cross || (p.parent != nullptr && ks + 1 < p.num_seqs && p.parent[ks + 1] == ks);
+  // dK / dV of this block are also written by CTAs of other heads or query sequences
+  const bool shared_keys = p.hsplit > 1 || cross || (p.parent != nullptr && ks + 1 < p.num_seqs && p.parent[ks + 1] == ks);
   const int k0 = (ntiles - 1 - from_end) * AB_BK;
 
   if (threadIdx.x == 0) {
@@ -122,7 +144,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tma_prefetch_desc(&tm_v);
     tma_prefetch_desc(&tm_do);
     mbar_init(kv_full, 1);
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < STAGES; ++i) {
       mbar_init(&qdo_full[i], 1);
       mbar_init(&qdo_empty[i], 1);
     }
@@ -142,7 +164,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int i0 = cross ? 0 : k0 / AB_BQ;                        // first query block at or below the diagonal
   const int nqb = (seqlen + AB_BQ - 1) / AB_BQ;
   const int per_head = nqb - i0;
-  const int n_it = per_head * G;
+  const int n_it = per_head * heads;
   constexpr uint32_t TM_DV = 0, TM_DK = HD, TM_S = 2 * HD, TM_DP = 2 * HD + AB_BQ, TM_DQ = 2 * HD + 2 * AB_BQ;
 
   if (warp == 0) {
@@ -155,12 +177,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tma_load_2d(sV + c * (AB_BK * 128), &tm_v, kv_full, kvh * HD + 64 * c, key_start + k0);
       }
       for (int it = 0; it < n_it; ++it) {
-        const int st = it & 1;
-        if (!mbar_wait(&qdo_empty[st], ((it >> 1) & 1) ^ 1)) {
+        const int st = it % STAGES;
+        if (!mbar_wait(&qdo_empty[st], ((it / STAGES) & 1) ^ 1)) {
           atomicExch(p.status, ST_TIMEOUT_PRODUCER);
           break;
         }
-        const int head = kvh * G + it / per_head;
+        const int head = head0 + it / per_head;
         const int q0 = (i0 + it % per_head) * AB_BQ;
         mbar_expect_tx(&qdo_full[st], 2 * L::QO_BYTES);
 #pragma unroll
@@ -178,8 +200,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       constexpr uint32_t idesc_dq = make_idesc_f16(128, AB_BQ, true, true);      // dQ^T (M = hd, padded to 128)
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aP = smem_u32(sP), aDS = smem_u32(sDS);
       auto issue_sdp = [&](int it) {
-        const int st = it & 1;
-        if (!mbar_wait(&qdo_full[st], (it >> 1) & 1)) return false;
+        const int st = it % STAGES;
+        if (!mbar_wait(&qdo_full[st], (it / STAGES) & 1)) return false;
         tc_fence_after();
         const uint32_t bQ = smem_u32(sQ + st * L::QO_BYTES), bDO = smem_u32(sDO + st * L::QO_BYTES);
 #pragma unroll
@@ -204,7 +226,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         tc_fence_after();
         if (it + 1 < n_it) ok = issue_sdp(it + 1);  // S^T/dP^T columns are free: the softmax of `it` has read them
         if (!ok) break;
-        const int st = it & 1;
+        const int st = it % STAGES;
         const uint32_t bQ = smem_u32(sQ + st * L::QO_BYTES), bDO = smem_u32(sDO + st * L::QO_BYTES);
 #pragma unroll
         for (int k = 0; k < AB_BQ / 16; ++k) {  // contraction over the 64 queries of the step
@@ -239,18 +261,33 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     bool ok = true;
     constexpr float LOG2E = 1.4426950408889634f;
 
+    float* dq_piece = reinterpret_cast<float*>(smem + L::OFF_DQ + (warp - 2) * L::DQ_PIECE);
     auto drain_dq = [&](int it) {
       if (HD < 128 && q * 32 >= HD) return;  // lanes of the padding rows
-      const int head = kvh * G + it / per_head;
+      const int head = head0 + it / per_head;
       const int q0 = (i0 + it % per_head) * AB_BQ + cbase;
-      const long long row_stride = static_cast<long long>(p.nh) * HD;
-      float* base = p.dq32 + static_cast<long long>(seq_start + q0) * row_stride + static_cast<long long>(head) * HD + r;
       uint32_t v[32];
       tmem_ld_32x32(tmem_base + TM_DQ + (it & 1) * AB_BQ + cbase + lane_off, v);
       tmem_ld_wait();
+      if (q0 >= seqlen) return;
+      if (q0 + 32 > seqlen) {  // the rows behind belong to another sequence
+        const long long row_stride = static_cast<long long>(p.nh) * HD;
+        float* base = p.dq32 + static_cast<long long>(seq_start + q0) * row_stride + static_cast<long long>(head) * HD + r;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        if (q0 + j < seqlen) atomicAdd(base + j * row_stride, __uint_as_float(v[j]));
+        for (int j = 0; j < 32; ++j) {
+          if (q0 + j < seqlen) atomicAdd(base + j * row_stride, __uint_as_float(v[j]));
+        }
+        return;
+      }
+      if (lane == 0) tma_store_wait_read<0>();  // the reduction of the step before has read the piece
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 32; ++j) dq_piece[j * 32 + lane] = __uint_as_float(v[j]);
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        tma_reduce_add_2d(&tm_dq, dq_piece, head * HD + q * 32, seq_start + q0);
+        tma_store_commit();
       }
     };
 
@@ -261,7 +298,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       nl2 = 0.f;
       nde = 0.f;
       if (it < n_it && qi < seqlen) {
-        const long long o = static_cast<long long>(kvh * G + it / per_head) * p.total_tokens + seq_start + qi;
+        const long long o = static_cast<long long>(head0 + it / per_head) * p.total_tokens + seq_start + qi;
         nl2 = p.lse[o] * LOG2E;
         nde = p.delta[o] * p.scale;
       }
@@ -271,8 +308,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int q0 = (i0 + it % per_head) * AB_BQ;
       // a private copy per warp, so no barrier across warps is needed (a warp that gave up on a wait cannot leave the
       // others stuck)
-      float* vL = sVec + (((warp - 2) * 2 + (it & 1)) * 2) * 32;
+      float* vL = sVec + (warp - 2) * 64;
       float* vD = vL + 32;
+      __syncwarp();  // the step before has been read
       vL[lane] = nl2;
       vD[lane] = nde;
       __syncwarp();
@@ -354,7 +392,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
         if (!key_ok) continue;
         if (shared_keys) {
 #pragma unroll
-          for (int i = 0; i < 32; ++i) atomicAdd(dst + c * 32 + i, __uint_as_float(o[i]));
+          for (int i = 0; i < 32; i += 4)
+            asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + c * 32 + i), "f"(__uint_as_float(o[i])),
+                         "f"(__uint_as_float(o[i + 1])), "f"(__uint_as_float(o[i + 2])), "f"(__uint_as_float(o[i + 3])) : "memory");
         } else {
 #pragma unroll
           for (int i = 0; i < 32; i += 4) *reinterpret_cast<uint4*>(dst + c * 32 + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
@@ -363,6 +403,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     }
   }
 
+  if (warp >= 2 && lane == 0) tma_store_wait_all<0>();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -444,7 +485,7 @@ using namespace vb;
 namespace vb {
 template <int HD>
 static cudaError_t launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& tdo,
-                                   const AttnBwdParams& p, cudaStream_t stream) {
+                                   const CUtensorMap& tdq, const AttnBwdParams& p, cudaStream_t stream) {
   auto kern = attn_bwd_kernel<HD>;
   constexpr int smem = AttnBwdSmem<HD>::TOTAL;
   static bool configured = false;
@@ -453,8 +494,8 @@ static cudaError_t launch_attn_bwd(const CUtensorMap& tq, const CUtensorMap& tk,
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  const dim3 grid(p.nkv, p.num_seqs * (p.parent != nullptr ? 2 : 1), p.max_tiles);
-  kern<<<grid, AB_THREADS, smem, stream>>>(tq, tk, tv, tdo, p);
+  const dim3 grid(p.nkv * p.hsplit, p.num_seqs * (p.parent != nullptr ? 2 : 1), p.max_tiles);
+  kern<<<grid, AB_THREADS, smem, stream>>>(tq, tk, tv, tdo, tdq, p);
   return cudaGetLastError();
 }
 }  // namespace vb
@@ -472,12 +513,14 @@ extern "C" int vb_attn_bwd(const void* q, const void* k, const void* v, const vo
   if (max_seqlen <= 0 || num_seqs > (parent != nullptr ? 32767 : 65535)) return -4;
   if (hd != 64 && hd != 128) return -2;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (ldo % 8) || (lddo % 8) || (lddq % 8) || (lddk % 8) || (lddv % 8) || (nh % nkv)) return -1;
-  CUtensorMap tq, tk, tv, tdo;
+  CUtensorMap tq, tk, tv, tdo, tdq;
   const auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   if (!make_tmap_2d(&tq, q, bf, 2, total_tokens, (uint64_t)nh * hd, ldq, 64, AB_BQ, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
   if (!make_tmap_2d(&tdo, dout, bf, 2, total_tokens, (uint64_t)nh * hd, lddo, 64, AB_BQ, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
   if (!make_tmap_2d(&tk, k, bf, 2, total_tokens, (uint64_t)nkv * hd, ldk, 64, AB_BK, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
   if (!make_tmap_2d(&tv, v, bf, 2, total_tokens, (uint64_t)nkv * hd, ldv, 64, AB_BK, CU_TENSOR_MAP_SWIZZLE_128B)) return -3;
+  if (!make_tmap_2d(&tdq, dq32_ws, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, total_tokens, (uint64_t)nh * hd, (uint64_t)nh * hd, 32, 32,
+                    CU_TENSOR_MAP_SWIZZLE_NONE)) return -3;
   static int* status = nullptr;
   if (status == nullptr) cudaGetSymbolAddress(reinterpret_cast<void**>(&status), g_attn_bwd_status);
   const long long T = total_tokens, lanes = T * nh * (hd / 8);
@@ -487,15 +530,26 @@ extern "C" int vb_attn_bwd(const void* q, const void* k, const void* v, const vo
   float* dk32 = dkv32_ws;
   float* dv32 = dkv32_ws + T * nkv * hd;
   cudaError_t e = cudaMemsetAsync(dq32_ws, 0, sizeof(float) * static_cast<size_t>(T) * nh * hd, stream);
-  if (e == cudaSuccess && parent != nullptr) e = cudaMemsetAsync(dkv32_ws, 0, sizeof(float) * 2 * static_cast<size_t>(T) * nkv * hd, stream);
+  // Heads of a group per CTA. The longest CTA has max_seqlen / 64 steps per head; an SM has about nkv * G * T * max_seqlen / 2 / (128 * 64)
+  // / SMs of them (sequences of about the longest length). The longest CTA is to have no more steps than an SM; every further share costs
+  // 1 to 3% in loads of K and V and additions of dK and dV.
+  const int G = nh / nkv;
+  const double longest = 2.0 * 128 * num_sms() / (static_cast<double>(nkv) * total_tokens);  // in SMs' shares, all heads in one CTA
+  int hsplit = static_cast<int>(longest < G ? ceil(longest) : G);
+  if (hsplit > G) hsplit = G;
+  if (hsplit < 1) hsplit = 1;
+  const int heads_per = (G + hsplit - 1) / hsplit;
+  hsplit = (G + heads_per - 1) / heads_per;
+  if (e == cudaSuccess && (parent != nullptr || hsplit > 1)) e = cudaMemsetAsync(dkv32_ws, 0, sizeof(float) * 2 * static_cast<size_t>(T) * nkv * hd, stream);
   if (e != cudaSuccess) return static_cast<int>(e);
   AttnBwdParams p{};
   p.cu_seqlens = cu_seqlens; p.parent = parent; p.num_seqs = num_seqs; p.nh = nh; p.nkv = nkv; p.total_tokens = total_tokens;
   p.lse = lse; p.delta = delta_ws; p.dq32 = dq32_ws; p.dk32 = dk32; p.dv32 = dv32;
   p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
   p.max_tiles = (max_seqlen + AB_BK - 1) / AB_BK;
+  p.hsplit = hsplit; p.heads_per = heads_per;
   if (p.max_tiles > 65535) return -4;
-  e = hd == 128 ? launch_attn_bwd<128>(tq, tk, tv, tdo, p, stream) : launch_attn_bwd<64>(tq, tk, tv, tdo, p, stream);
+  e = hd == 128 ? launch_attn_bwd<128>(tq, tk, tv, tdo, tdq, p, stream) : launch_attn_bwd<64>(tq, tk, tv, tdo, tdq, p, stream);
   if (e != cudaSuccess) return static_cast<int>(e);
   const long long n = T * (nh + 2 * nkv) * (hd / 8);
   attn_bwd_finish_kernel<<<static_cast<int>((n + 255) / 256), 256, 0, stream>>>(
