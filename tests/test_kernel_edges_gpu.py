@@ -529,3 +529,27 @@ def test_attention_backward_over_shares_of_heads(ops, nh, nkv, hd, lens):
     for x, w in zip(got, ref):
         assert rel(x, w.grad) < 1.5e-2  # dS is rounded to bf16 and its terms cancel
     assert int(ops.gemm_status()) == 0
+
+
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("scale", [0.125, 0.0, -0.05])
+def test_attention_scales_and_growing_scores(ops, hd, scale):
+    """Scores that grow along the keys (the maximum moves in every block, in small and large steps), 33 sequences, any sign of the scale."""
+    nh, nkv = 4, 2
+    lens = [1, 3] * 16 + [700]
+    T, cu = sum(lens), np.cumsum([0] + lens).tolist()
+    g = torch.Generator(device=DEV).manual_seed(hd)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    q, k, v = rnd(T, nh, hd), rnd(T, nkv, hd), rnd(T, nkv, hd)
+    q[:, 0] = q[:, 0].abs()
+    k[:, 0] = (k[:, 0].abs() * torch.linspace(0.01, 4, T, device=DEV)[:, None]).bfloat16()
+    out, lse = ops.attn_fwd(q, k, v, torch.tensor(cu, dtype=torch.int32, device=DEV), scale, None)
+    keys = [list(range(a, a + i + 1)) for a, n in zip(cu, lens) for i in range(n)]
+    want = _attention64(q.double(), k.double(), v.double(), keys, scale)
+    assert rel(out, want) < 6e-3
+    for h in range(nh):
+        s = (q[:, h].double() @ k[:, h // 2].double().T * scale)
+        see = torch.full((T, T), -math.inf, dtype=torch.float64, device=DEV)
+        for t in range(T):
+            see[t, keys[t]] = 0
+        torch.testing.assert_close(lse[h].double(), (s + see).logsumexp(-1), rtol=1e-5, atol=1e-4)

@@ -428,6 +428,10 @@ class DecoderModel:
                                     f"verl_b200.models.generic (training engine and its cache-based rollout)")
         self.keep_layers_fn: Optional[Callable[[int], int]] = None
         self.tp: Optional[TensorParallelShard] = None  # set by the rollout engine; forward-only
+        # set by the rollout engine for dense models: its products of at most 64 tokens may take kernels that sum in another order. Scoring
+        # and updates stay on one family, so that their log-probs of a sequence agree, and so do mixture-of-experts models: a router
+        # turns a last bit of its input into another choice of experts, and log-probs of a short rollout then move by 10%
+        self.decode_kernels = False
         self.fp8_weights: Optional[dict] = None         # data_ptr of a bf16 weight -> (e4m3 copy, block scales)
         self.offloader = None                           # ActivationOffloader: inputs of recomputed layers live on the host
         self.etp_sum = None                             # all-reduce over the tensor-parallel group (experts cut over it)
@@ -666,13 +670,11 @@ class DecoderModel:
         """``x @ W[name]^T (+ bias)``; forward-only calls use the fp8 copy of the weight when one is installed."""
         w = W[name]
         b = W.get(name[: -len("weight")] + "bias")
-        # mixture-of-experts layers stay on one family of kernels: a router turns a last bit of its input into another choice of experts,
-        # and the log-probs of a short rollout then move by 10%
         if S is None and self.fp8_weights is not None:
             q = self.fp8_weights.get(w.data_ptr())
             if q is not None:
                 return F.linear_fp8(x, q[0], q[1], b)
-        return F.gemm(x, w, b, tcgen05=self.cfg.is_moe)
+        return F.gemm_decode(x, w, b) if self.decode_kernels else F.gemm(x, w, b)
 
     def quantize_linear_weights_fp8(self) -> int:
         """(Re)build e4m3 copies with 1x128 block scales of every dense projection (rollout precision of the MoE
@@ -720,7 +722,7 @@ class DecoderModel:
             # forward-only passes and the first pass of a recomputed layer: the activation runs in the epilogue of the
             # up-projection and the pre-activation is never written. (A layer that keeps its pre-activation runs the two
             # kernels: the epilogue that writes both measured slower than GEMM + activation, 4.36 vs 3.60 ms at 16k tokens.)
-            act, gu = F.gemm_swiglu(h2, W["mlp.gate_up_proj.weight"], want_gate_up=False)
+            act, gu = F.gemm_swiglu(h2, W["mlp.gate_up_proj.weight"], want_gate_up=False, decode=self.decode_kernels)
         else:
             gu = self._lin(W, "mlp.gate_up_proj.weight", h2, S)
             act = F.swiglu(gu)
@@ -813,7 +815,7 @@ class DecoderModel:
         ops = F._ops()
         T, H = h2.shape
         E, k = cfg.num_experts, cfg.num_experts_per_tok
-        logits = F.gemm(h2, W["mlp.gate.weight"], tcgen05=True)
+        logits = F.gemm(h2, W["mlp.gate.weight"])
         w, idx, counts = self._routing(logits)
         w = w.float().contiguous()
         tile = 128 if S is not None else self._moe_tile(T * k, E)
@@ -888,8 +890,8 @@ class DecoderModel:
         s0 = 0
         for e, n in enumerate(counts):
             if n:
-                F.gemm(x[s0 : s0 + n], Wgu[e], out=gu[s0 : s0 + n], tcgen05=True)
-                F.gemm(F.swiglu(gu[s0 : s0 + n]), Wd[e], out=y[s0 : s0 + n], tcgen05=True)
+                F.gemm(x[s0 : s0 + n], Wgu[e], out=gu[s0 : s0 + n])
+                F.gemm(F.swiglu(gu[s0 : s0 + n]), Wd[e], out=y[s0 : s0 + n])
                 s0 += n
         if S is not None:
             S["gu"] = gu
@@ -920,7 +922,7 @@ class DecoderModel:
         T, H = h2.shape
         E, k = cfg.num_experts, cfg.num_experts_per_tok
         El = E // ep.size
-        logits = F.gemm(h2, W["mlp.gate.weight"], tcgen05=True)
+        logits = F.gemm(h2, W["mlp.gate.weight"])
         w, idx, counts = self._routing(logits)
         flat_e = idx.reshape(-1)
         order = torch.argsort(flat_e, stable=True)          # copies sorted by global expert = by (owner, local expert)
@@ -982,9 +984,9 @@ class DecoderModel:
 
     # -- shared expert (Qwen2-MoE): a dense SwiGLU MLP applied to every token, scaled by sigmoid(h . w_gate) -------------
     def _shared_expert_fwd(self, W, h2, S: Optional[dict]):
-        gu = F.gemm(h2, W["mlp.shared_expert.gate_up_proj.weight"], tcgen05=True)
-        y = F.gemm(F.swiglu(gu), W["mlp.shared_expert.down_proj.weight"], tcgen05=True)
-        z = F.gemm(h2, W["mlp.shared_expert_gate.weight"], tcgen05=True)[:, 0].float()
+        gu = F.gemm(h2, W["mlp.shared_expert.gate_up_proj.weight"])
+        y = F.gemm(F.swiglu(gu), W["mlp.shared_expert.down_proj.weight"])
+        z = F.gemm(h2, W["mlp.shared_expert_gate.weight"])[:, 0].float()
         sg = torch.sigmoid(z)
         if S is not None:
             S["shared"] = dict(gu=gu, y=y, sg=sg)
@@ -1032,7 +1034,7 @@ class DecoderModel:
         cfg = self.cfg
         T, H = h2.shape
         E, k = cfg.num_experts, cfg.num_experts_per_tok
-        logits = F.gemm(h2, W["mlp.gate.weight"], tcgen05=True)
+        logits = F.gemm(h2, W["mlp.gate.weight"])
         w, idx, counts = self._routing(logits)
         flat_e = idx.reshape(-1)
         order = torch.argsort(flat_e, stable=True)
@@ -1046,8 +1048,8 @@ class DecoderModel:
         for e, n in enumerate(counts):
             if n == 0:
                 continue
-            F.gemm(xp[s0 : s0 + n], Wgu[e], out=gu[s0 : s0 + n], tcgen05=True)
-            F.gemm(F.swiglu(gu[s0 : s0 + n]), Wd[e], out=y[s0 : s0 + n], tcgen05=True)
+            F.gemm(xp[s0 : s0 + n], Wgu[e], out=gu[s0 : s0 + n])
+            F.gemm(F.swiglu(gu[s0 : s0 + n]), Wd[e], out=y[s0 : s0 + n])
             s0 += n
         wp = w.reshape(-1)[order].to(h2.dtype)
         out = torch.zeros(T, H, dtype=torch.float32, device=h2.device)

@@ -3,11 +3,15 @@
 // One CTA = one (sequence, 128-row query tile, query head).  Two CTAs are co-resident per SM (<= 113 KB shared
 // memory and 256 TMEM columns each), so the softmax of one tile overlaps the MMAs of the other.
 //
-//   warp 0      TMA: Q tile once, then K/V tiles of 64 keys through a 2-stage ring (128B swizzle)
+//   warp 0      TMA: Q tile once, then tiles of 64 keys of K and of V, each through a ring of its own (128B swizzle): a K tile is free
+//               once its scores are done, long before its V tile. 2 stages each at head_dim 128, 5 at head_dim 64
 //   warp 1      MMA: S_j = Q K_j^T into one of two TMEM S buffers (issued one block ahead), O += P_j V_j
 //   warps 2..5  softmax: thread == query row.  tcgen05.ld S -> scale, causal mask, online max/sum in the exp2
 //               domain -> P (bf16) written to shared memory in the K-major 128B-swizzle layout the MMA reads;
 //               O in TMEM is rescaled (tcgen05.ld / tcgen05.st) only when some row maximum of the warp moved.
+// What bounds it: the chain of a block through scores, softmax and P in shared memory; two CTAs per SM take turns. 28 / 4 heads of 128,
+// 5 x 3072 tokens: 508 us with K and V in one ring and the mask in every block, 485 with rings of their own, 454 with the mask apart
+// (745 TFLOP/s); 14 / 2 heads of 64, 12 x 1,000 tokens: 102, 102 and 98 us.
 // Epilogue: O / l -> bf16 [T, nh, hd]; LSE (natural log) -> [nh, T] for the backward pass.
 //
 // With `parent`, a sequence may be the continuation of another one (the responses of a group behind their shared prompt): its queries
@@ -41,13 +45,15 @@ struct AttnSmem {
   static constexpr int Q_BYTES = ATT_BQ * HD * 2;
   static constexpr int KV_BYTES = ATT_BKV * HD * 2;  // one of K or V, one stage
   static constexpr int P_BYTES = ATT_BQ * ATT_BKV * 2;
+  static constexpr int STAGES = HD == 128 ? 2 : 5;
   static constexpr int OFF_K = Q_BYTES;
-  static constexpr int OFF_V = OFF_K + 2 * KV_BYTES;
-  static constexpr int OFF_P = OFF_V + 2 * KV_BYTES;
+  static constexpr int OFF_V = OFF_K + STAGES * KV_BYTES;
+  static constexpr int OFF_P = OFF_V + STAGES * KV_BYTES;
   static constexpr int OFF_BAR = OFF_P + P_BYTES;
   // No alignment slack and no static shared memory: two CTAs (2 x (TOTAL + 1 KB reserved)) must fit the 228 KB of an
   // SM; the dynamic window then starts 1024-byte aligned, which the kernel verifies before touching it.
-  static constexpr int TOTAL = OFF_BAR + 128;
+  static constexpr int TOTAL = OFF_BAR + 256;
+  static_assert(2 * (TOTAL + 1024) <= 228 * 1024, "two CTAs per SM");
 };
 
 template <int HD>
@@ -67,47 +73,60 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   uint8_t* sV = smem + L::OFF_V;
   uint8_t* sP = smem + L::OFF_P;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
+  constexpr int STAGES = L::STAGES;
   uint64_t* q_full = bars;         // 1
-  uint64_t* kv_full = bars + 1;    // 2
-  uint64_t* kv_empty = bars + 3;   // 2
-  uint64_t* bar_s = bars + 5;      // 2
-  uint64_t* bar_p = bars + 7;      // 1
-  uint64_t* bar_o = bars + 8;      // 1
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 9);
-  int* s_tile = reinterpret_cast<int*>(bars + 10);  // seq start token, q0, seqlen, valid, parent's start, parent's length
+  uint64_t* bar_s = bars + 1;      // 2
+  uint64_t* bar_p = bars + 3;      // 1
+  uint64_t* bar_o = bars + 4;      // 1
+  uint64_t* k_full = bars + 5;     // [STAGES] each
+  uint64_t* k_empty = k_full + STAGES;
+  uint64_t* v_full = k_empty + STAGES;
+  uint64_t* v_empty = v_full + STAGES;
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(v_empty + STAGES);
+  int* s_tile = reinterpret_cast<int*>(tmem_holder + 2);  // seq start token, q0, seqlen, valid, parent's start, parent's length
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int head = blockIdx.y;
   const int kvh = head / (p.nh / p.nkv);
 
-  if (threadIdx.x == 0) {
-    // locate (sequence, query block) of this CTA: tiles are enumerated sequence by sequence
-    int t = blockIdx.x, found = 0, start = 0, q0 = 0, len = 0, pstart = 0, plen = 0;
-    for (int s = 0; s < p.num_seqs; ++s) {
-      const int a = p.cu_seqlens[s], b = p.cu_seqlens[s + 1];
+  if (warp == 0) {
+    // locate (sequence, query block) of this CTA: tiles are enumerated sequence by sequence, 32 sequences per turn
+    int t = blockIdx.x;
+    if (lane == 0) s_tile[0] = s_tile[1] = s_tile[2] = s_tile[3] = s_tile[4] = s_tile[5] = 0;
+    __syncwarp();
+    for (int s0 = 0; s0 < p.num_seqs; s0 += 32) {
+      const int s = s0 + lane;
+      const int a = s < p.num_seqs ? p.cu_seqlens[s] : 0, b = s < p.num_seqs ? p.cu_seqlens[s + 1] : 0;
       const int nt = (b - a + ATT_BQ - 1) / ATT_BQ;
-      if (t < nt) {
-        // heavy (late) query blocks first: they have the most key blocks
-        start = a; len = b - a; q0 = (nt - 1 - t) * ATT_BQ; found = 1;
-        const int pr = p.parent != nullptr ? p.parent[s] : -1;
-        if (pr >= 0 && pr < p.num_seqs) {
-          pstart = p.cu_seqlens[pr];
-          plen = p.cu_seqlens[pr + 1] - pstart;
+      int upto = nt;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+      }
+      const int total = __shfl_sync(0xffffffffu, upto, 31);
+      if (t < total) {
+        if (t < upto && t >= upto - nt) {
+          // heavy (late) query blocks first: they have the most key blocks
+          s_tile[0] = a; s_tile[1] = (nt - 1 - (t - (upto - nt))) * ATT_BQ; s_tile[2] = b - a; s_tile[3] = 1;
+          const int pr = p.parent != nullptr ? p.parent[s] : -1;
+          if (pr >= 0 && pr < p.num_seqs) {
+            s_tile[4] = p.cu_seqlens[pr];
+            s_tile[5] = p.cu_seqlens[pr + 1] - s_tile[4];
+          }
         }
         break;
       }
-      t -= nt;
+      t -= total;
     }
-    s_tile[0] = start; s_tile[1] = q0; s_tile[2] = len; s_tile[3] = found; s_tile[4] = pstart; s_tile[5] = plen;
+  }
+  if (threadIdx.x == 0) {
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
     mbar_init(q_full, 1);
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&kv_full[i], 1);
-      mbar_init(&kv_empty[i], 1);
-      mbar_init(&bar_s[i], 1);
-    }
+    for (int i = 0; i < 4 * STAGES; ++i) mbar_init(&k_full[i], 1);
+    for (int i = 0; i < 2; ++i) mbar_init(&bar_s[i], 1);
     mbar_init(bar_p, 4);
     mbar_init(bar_o, 1);
     mbar_fence_init();
@@ -134,18 +153,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
       for (int c = 0; c < PANELS; ++c) tma_load_2d(sQ + c * (ATT_BQ * 128), &tm_q, q_full, head * HD + 64 * c, seq_start + q0);
       for (int j = 0; j < nblk; ++j) {
-        const int st = j & 1;
-        if (!mbar_wait(&kv_empty[st], ((j >> 1) & 1) ^ 1)) {
+        const int st = j % STAGES;
+        const uint32_t free_phase = ((j / STAGES) & 1) ^ 1;
+        const int krow = j < pblk ? pstart + j * ATT_BKV : seq_start + (j - pblk) * ATT_BKV;
+        if (!mbar_wait(&k_empty[st], free_phase)) {
           atomicExch(p.status, ST_TIMEOUT_PRODUCER);
           break;
         }
-        mbar_expect_tx(&kv_full[st], 2 * L::KV_BYTES);
-        const int krow = j < pblk ? pstart + j * ATT_BKV : seq_start + (j - pblk) * ATT_BKV;
+        mbar_expect_tx(&k_full[st], L::KV_BYTES);
 #pragma unroll
-        for (int c = 0; c < PANELS; ++c) {
-          tma_load_2d(sK + st * L::KV_BYTES + c * (ATT_BKV * 128), &tm_k, &kv_full[st], kvh * HD + 64 * c, krow);
-          tma_load_2d(sV + st * L::KV_BYTES + c * (ATT_BKV * 128), &tm_v, &kv_full[st], kvh * HD + 64 * c, krow);
+        for (int c = 0; c < PANELS; ++c) tma_load_2d(sK + st * L::KV_BYTES + c * (ATT_BKV * 128), &tm_k, &k_full[st], kvh * HD + 64 * c, krow);
+        if (!mbar_wait(&v_empty[st], free_phase)) {
+          atomicExch(p.status, ST_TIMEOUT_PRODUCER);
+          break;
         }
+        mbar_expect_tx(&v_full[st], L::KV_BYTES);
+#pragma unroll
+        for (int c = 0; c < PANELS; ++c) tma_load_2d(sV + st * L::KV_BYTES + c * (ATT_BKV * 128), &tm_v, &v_full[st], kvh * HD + 64 * c, krow);
       }
     }
   } else if (warp == 1) {
@@ -154,8 +178,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       constexpr uint32_t idesc_o = make_idesc_f16(ATT_BQ, HD, false, true);
       bool ok = mbar_wait(q_full, 0);
       auto issue_s = [&](int j) {
-        const int st = j & 1;
-        if (!mbar_wait(&kv_full[st], (j >> 1) & 1)) return false;
+        const int st = j % STAGES;
+        if (!mbar_wait(&k_full[st], (j / STAGES) & 1)) return false;
         tc_fence_after();
         const uint32_t aq = smem_u32(sQ), bk = smem_u32(sK + st * L::KV_BYTES);
 #pragma unroll
@@ -164,6 +188,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           const uint64_t db = make_smem_desc_sw128(bk + (k >> 2) * (ATT_BKV * 128) + (k & 3) * 32, 16, 1024);
           tc_mma_f16_ss(tmem_base + TM_S0 + (j & 1) * ATT_BKV, da, db, idesc_s, k > 0 ? 1u : 0u);
         }
+        tc_commit(&k_empty[st]);
         tc_commit(&bar_s[j & 1]);
         return true;
       };
@@ -171,9 +196,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       for (int j = 0; j < nblk && ok; ++j) {
         if (j + 1 < nblk) ok = issue_s(j + 1);
         if (!ok) break;
-        if (!mbar_wait(bar_p, j & 1)) { ok = false; break; }
+        const int st = j % STAGES;
+        if (!mbar_wait(&v_full[st], (j / STAGES) & 1) || !mbar_wait(bar_p, j & 1)) { ok = false; break; }
         tc_fence_after();
-        const int st = j & 1;
         const uint32_t ap = smem_u32(sP), bv = smem_u32(sV + st * L::KV_BYTES);
 #pragma unroll
         for (int k = 0; k < ATT_BKV / 16; ++k) {
@@ -181,7 +206,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           const uint64_t db = make_smem_desc_sw128(bv + k * 2048, ATT_BKV * 128, 1024);
           tc_mma_f16_ss(tmem_base + TM_O, da, db, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
         }
-        tc_commit(&kv_empty[st]);
+        tc_commit(&v_empty[st]);
         tc_commit(bar_o);
       }
       if (!ok) atomicExch(p.status, ST_TIMEOUT_MMA);
@@ -205,18 +230,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       const int col0 = (j - pblk) * ATT_BKV;
       const int limit = j < pblk ? plen - j * ATT_BKV : row - col0 + 1;
       const bool need_mask = j < pblk ? limit < ATT_BKV : col0 + ATT_BKV - 1 > q0;
-      float mx = -INFINITY;
+      // The scaled score is rounded before the maximum is taken off, although one fma could do both: a last bit here moves gradients behind
+      // 24 layers by more than the rounding of bf16 does in one, and turns a router's choice of experts.
 #pragma unroll
       for (int c = 0; c < 32; ++c) {
-        float a = __uint_as_float(x0[c]) * p.scale_log2, b = __uint_as_float(x1[c]) * p.scale_log2;
-        if (need_mask) {
-          if (c >= limit) a = -INFINITY;
-          if (32 + c >= limit) b = -INFINITY;
-        }
-        x0[c] = __float_as_uint(a);
-        x1[c] = __float_as_uint(b);
-        mx = fmaxf(mx, fmaxf(a, b));
+        x0[c] = __float_as_uint(__uint_as_float(x0[c]) * p.scale_log2);
+        x1[c] = __float_as_uint(__uint_as_float(x1[c]) * p.scale_log2);
       }
+      if (need_mask) {  // uniform over the warp, and apart: in the loop below the comparisons cost every block two instructions per score
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          if (c >= limit) x0[c] = 0xff800000u;
+          if (32 + c >= limit) x1[c] = 0xff800000u;
+        }
+      }
+      float mx = -INFINITY;
+#pragma unroll
+      for (int c = 0; c < 32; ++c) mx = fmaxf(mx, fmaxf(__uint_as_float(x0[c]), __uint_as_float(x1[c])));
       const float m_new = fmaxf(m_run, mx);
       const float alpha = (m_new == -INFINITY) ? 1.f : exp2f(m_run - m_new);
       const float m_use = (m_new == -INFINITY) ? 0.f : m_new;

@@ -154,11 +154,11 @@ Tensor gemm_dispatch(const Tensor& a, const Tensor& b, const OptTensor& bias, co
 
 Tensor gemm(const Tensor& a, const Tensor& b, const OptTensor& bias, const OptTensor& out, bool a_mn, bool b_mn, bool out_f32, bool accumulate,
             int64_t max_ctas) {
-  return gemm_dispatch(a, b, bias, out, a_mn, b_mn, out_f32, accumulate, max_ctas, true);
-}
-Tensor gemm_tcgen05(const Tensor& a, const Tensor& b, const OptTensor& bias, const OptTensor& out, bool a_mn, bool b_mn, bool out_f32,
-                    bool accumulate, int64_t max_ctas) {
   return gemm_dispatch(a, b, bias, out, a_mn, b_mn, out_f32, accumulate, max_ctas, false);
+}
+// a b^T (+bias) of a decode step: the mma.sync kernel for at most 64 tokens takes part
+Tensor gemm_decode(const Tensor& a, const Tensor& b, const OptTensor& bias) {
+  return gemm_dispatch(a, b, bias, c10::nullopt, false, false, false, false, 0, true);
 }
 
 // act = silu(a W_gate^T) * (a W_up^T) for the stacked weight w = [W_gate; W_up] ([2I, K]); with want_gu the pre-activation
@@ -1244,7 +1244,7 @@ TORCH_LIBRARY(verl_b200, m) {
   m.def("gemm_grouped_rows", &gemm_grouped_rows);
   m.def("gemm_grouped_wgrad_", &gemm_grouped_wgrad_);
   m.def("gemm", &gemm);
-  m.def("gemm_tcgen05", &gemm_tcgen05);
+  m.def("gemm_decode", &gemm_decode);
   m.def("gemm_few_tokens", &gemm_few_tokens);
   m.def("few_tokens_better", [](int64_t M, int64_t N, int64_t K, bool swiglu) {
     return skinny_enabled() && vb_few_tokens_better((int)std::min<int64_t>(M, 65), (int)N, (int)K, swiglu) != 0;

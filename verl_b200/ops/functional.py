@@ -62,9 +62,8 @@ def set_fetch_rider(rider) -> None:
 
 def gemm(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, out: Optional[torch.Tensor] = None,
          a_mn: bool = False, b_mn: bool = False, out_f32: bool = False, accumulate: bool = False,
-         max_ctas: int = 0, tcgen05: bool = False) -> torch.Tensor:
-    """``D = A @ B^T (+bias)``; ``a_mn``/``b_mn`` mean the operand is stored transposed ([K, M] / [K, N]). ``tcgen05``: leave out the
-    ``mma.sync`` kernel for at most 64 tokens, whose sums come in another order."""
+         max_ctas: int = 0) -> torch.Tensor:
+    """``D = A @ B^T (+bias)``; ``a_mn``/``b_mn`` mean the operand is stored transposed ([K, M] / [K, N])."""
     if a.is_cuda:
         if _FETCH_RIDER is not None and max_ctas == 0:
             M = a.shape[1] if a_mn else a.shape[0]
@@ -74,7 +73,7 @@ def gemm(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, 
                 job = _FETCH_RIDER.take(2.0 * M * N * K)
                 if job is not None:
                     return _ops().gemm_fetch(a, b, bias, out, a_mn, b_mn, out_f32, accumulate, *job, -1, None, 2.0)
-        return (_ops().gemm_tcgen05 if tcgen05 else _ops().gemm)(a, b, bias, out, a_mn, b_mn, out_f32, accumulate, max_ctas)
+        return _ops().gemm(a, b, bias, out, a_mn, b_mn, out_f32, accumulate, max_ctas)
     A = a.t() if a_mn else a
     Bt = b if b_mn else b.t()
     d = A.float() @ Bt.float()
@@ -87,6 +86,11 @@ def gemm(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None, 
             out.copy_(d.to(out.dtype))
         return out
     return d if out_f32 else d.to(a.dtype)
+
+
+def gemm_decode(a: torch.Tensor, b: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``gemm`` of a decode step: at most 64 tokens may take the ``mma.sync`` kernel, whose sums come in another order."""
+    return _ops().gemm_decode(a, b, bias) if a.is_cuda else gemm(a, b, bias)
 
 
 def gemm_row_ranges(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ranges, out: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -263,21 +267,21 @@ def swiglu(gate_up: torch.Tensor) -> torch.Tensor:
 FUSED_SWIGLU = os.environ.get("VERL_B200_FUSED_SWIGLU", "1") != "0"
 
 
-def gemm_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, want_gate_up: bool = False):
+def gemm_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, want_gate_up: bool = False, decode: bool = False):
     """``silu(x W_gate^T) * (x W_up^T)`` for the stacked weight ``[W_gate; W_up]``; returns ``(act, gate_up or None)``.
     Training-sized inputs on the GPU run the GEMM whose epilogue applies the activation (the [tokens, 2I] pre-activation
     is only written when ``want_gate_up``, for a backward pass that keeps it); decode-sized ones keep the kernel for few
-    tokens plus the activation kernel."""
+    tokens plus the activation kernel; with ``decode`` at most 16 may take the ``mma.sync`` kernel that applies the activation, too."""
     if (x.is_cuda and FUSED_SWIGLU and x.dim() == 2 and x.shape[0] > 1024 and x.stride(1) == 1 and x.stride(0) % 8 == 0
             and w_gate_up.is_contiguous() and w_gate_up.shape[0] % 8 == 0 and w_gate_up.shape[1] % 8 == 0):
         act, gu = _ops().gemm_swiglu(x, w_gate_up, bool(want_gate_up))
         return act, (gu if want_gate_up else None)
-    if (x.is_cuda and FUSED_SWIGLU and not want_gate_up and x.dim() == 2 and x.dtype == torch.bfloat16 and 0 < x.shape[0] <= 16
+    if (decode and x.is_cuda and FUSED_SWIGLU and not want_gate_up and x.dim() == 2 and x.dtype == torch.bfloat16 and 0 < x.shape[0] <= 16
             and x.stride(1) == 1 and x.stride(0) % 8 == 0 and w_gate_up.is_contiguous() and w_gate_up.shape[0] % 16 == 0
             and w_gate_up.shape[1] % 8 == 0 and x.data_ptr() % 16 == 0 and w_gate_up.data_ptr() % 16 == 0
             and _ops().few_tokens_better(x.shape[0], w_gate_up.shape[0] // 2, x.shape[1], True)):
         return _ops().gemm_few_tokens(x, w_gate_up, None, True), None  # activation in the epilogue of the kernel for few tokens
-    gu = gemm(x, w_gate_up)
+    gu = gemm_decode(x, w_gate_up) if decode else gemm(x, w_gate_up)
     return swiglu(gu), (gu if want_gate_up else None)
 
 

@@ -146,6 +146,8 @@ class RolloutEngine:
         self._num_blocks_req = num_blocks
         self.model = build_decoder(cfg, params, max_positions=self.max_model_len + 1)
         self.model.kv_hook = self._prefill_kv_hook
+        if not cfg.is_stack:
+            self.model.decode_kernels = not cfg.is_moe
         self.cache = make_cache(cfg, params.flat.dtype, self.device, self.bs, self.S, self.tp_size)
         self.sequences: dict[str, _Sequence] = {}
         self._tp_share = None
