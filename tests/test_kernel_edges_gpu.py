@@ -440,6 +440,20 @@ def test_weight_gradient_accumulates(ops, M, N, K):
     assert int(ops.gemm_status()) == 0
 
 
+@pytest.mark.parametrize("ctas", [1, 2, 0])
+@pytest.mark.parametrize("M,N,K", [(160, 2056, 16), (96, 2056, 64), (224, 1288, 8), (32, 4104, 24)])
+def test_weight_gradient_of_slabs_behind_the_last_row(ops, ctas, M, N, K):
+    """Many short tiles per CTA, every second one with slabs of 32 rows behind the last row. Small integers: every sum is exact."""
+    g = torch.Generator().manual_seed(M + N + K)
+    dy, x = torch.randint(-4, 5, (K, M), generator=g).to(DEV).bfloat16(), torch.randint(-4, 5, (K, N), generator=g).to(DEV).bfloat16()
+    out = torch.randint(-99, 100, (M, N), generator=g).to(DEV).float()
+    want = out + 8 * (dy.float().T @ x.float())
+    for _ in range(8):
+        ops.gemm(dy, x, None, out, True, True, True, True, ctas)
+    assert torch.equal(out, want)
+    assert int(ops.gemm_status()) == 0
+
+
 @pytest.mark.parametrize("M,N", [(128, 256), (160, 264), (96, 768), (72, 264)])
 def test_weight_gradient_per_expert_accumulates(ops, M, N):
     counts = [130, 0, 128, 5, 0]

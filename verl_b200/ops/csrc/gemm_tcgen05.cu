@@ -726,20 +726,24 @@ __device__ __forceinline__ void gemm_body(const CUtensorMap& tma_a, const CUtens
             }
           }
         } else if constexpr (EPI == EPI_ACC32) {
-          // 32 rows of 128 bytes, 16-byte pieces swizzled by the row; columns past N are clipped by the tensor map
-          uint8_t* piece = smem + GemmSmem<BN, STAGES>::RING + (q * 2 + (pieces & 1)) * GemmSmem<BN, STAGES>::ACC_PIECE;
-          if (lane == 0) tma_store_wait_read<1>();  // the reduction before the last has read this piece
-          __syncwarp();
+          // 32 rows of 128 bytes, 16-byte pieces swizzled by the row; columns past N are clipped by the tensor map. M % 32 == 0: a slab of
+          // 32 rows belongs to one output or to none. A slab behind the last row leaves the buffers alone: it commits no reduction, so the
+          // wait below, which counts groups, would let it write over a piece that is still being read.
+          if (m0 + q * 32 < p.M) {
+            uint8_t* piece = smem + GemmSmem<BN, STAGES>::RING + (q * 2 + (pieces & 1)) * GemmSmem<BN, STAGES>::ACC_PIECE;
+            if (lane == 0) tma_store_wait_read<1>();  // the reduction before the last has read this piece
+            __syncwarp();
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<uint4*>(piece + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0 && m0 + q * 32 < p.M) {  // M % 32 == 0: a slab of 32 rows belongs to one output
-            tma_reduce_add_2d(tma_d, piece, col0, static_cast<int>(d_off) + m0 + q * 32);
-            tma_store_commit();
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<uint4*>(piece + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+            fence_proxy_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_reduce_add_2d(tma_d, piece, col0, static_cast<int>(d_off) + m0 + q * 32);
+              tma_store_commit();
+            }
+            ++pieces;
           }
-          ++pieces;
         } else if (row_ok) {
           if (p.bias != nullptr) {
 #pragma unroll
