@@ -122,6 +122,25 @@ def test_sampler_takes_the_token_of_the_whole_row(ops, B, V, ld, valid, scale):
         assert (lp.double() - want).abs().max() < 1e-4 * (1 + xt[xt > -math.inf].abs().max())
 
 
+@pytest.mark.parametrize("V,ld,valid", [(8, 8, 0), (1000, 1000, 0), (2049, 2056, 0), (33001, 33003, 32999)])
+def test_sampler_of_rows_without_numbers(ops, V, ld, valid):
+    """NaN and masked logits: a token of the vocabulary all the same (the first where there is none to take), and a log-prob that is NaN."""
+    from verl_b200.ops import functional as F
+
+    n = valid or V
+    lg = torch.full((5, ld), math.nan)
+    lg[1] = -math.inf
+    lg[2, : n // 2] = -math.inf
+    lg[3, n - 1] = 1.5
+    lg[4] = -math.inf
+    lg[4, n - 1] = 1.5
+    seeds = torch.arange(5, device=DEV)
+    for T in (1.0, 0.3, 0.0):
+        tok, lp = F.sample_tokens(lg.bfloat16().to(DEV)[:, :V], T, seeds, 3, valid)
+        assert tok.tolist() == [0, 0, 0, n - 1, n - 1]
+        assert lp[:4].isnan().all() and float(lp[4]) == 0.0
+
+
 # ------------------------------------------------------------------------------------------------ head and optimizer
 @pytest.mark.parametrize("T,V", [(1, 8), (31, 4096), (33, 4360), (130, 264)])
 def test_head_merges_its_tiles(ops, T, V):

@@ -431,7 +431,8 @@ sample_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int valid_
         const uint32_t h = sample_bits(key, i0 + j);
         if (!(__uint_as_float(0x4B000000u | (h >> 1)) < bound)) {  // a NaN bound counts as a candidate
           const float score = sample_score(x[j] * it, h);
-          if (score > a.best || (score == a.best && i0 + j < a.best_i)) {
+          // (a score of -inf is a masked logit, or a lane behind the vocabulary's end: it takes no token, also in a row without numbers)
+          if (score > a.best || (score == a.best && i0 + j < a.best_i && score > -INFINITY)) {
             a.best = score;
             a.best_i = i0 + j;
             a.best_x = x[j] * it;
@@ -461,7 +462,7 @@ sample_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int valid_
   if (part == 0 && threadIdx.x == 0) {
     for (int k = 1; k < parts; ++k) sample_fold(a, *cluster.map_shared_rank(&cta_part, k));
     tokens[row] = a.best_i == 0x7fffffff ? 0 : a.best_i;
-    if (logprobs) logprobs[row] = a.best_x - (a.m + __logf(a.l));
+    if (logprobs) logprobs[row] = a.m == -INFINITY ? __int_as_float(0x7fffffff) : a.best_x - (a.m + __logf(a.l));  // no token: NaN
   }
   cluster.sync();  // a CTA's shared memory is read by its cluster until here
 }
