@@ -122,6 +122,23 @@ def test_sampler_takes_the_token_of_the_whole_row(ops, B, V, ld, valid, scale):
         assert (lp.double() - want).abs().max() < 1e-4 * (1 + xt[xt > -math.inf].abs().max())
 
 
+@pytest.mark.parametrize("scale", [2.5, 20.0, 200.0])
+@pytest.mark.parametrize("T", [1.0, 0.7, 0.1, 0.01, 0.0])
+def test_sampler_log_probs_of_sharp_rows(ops, scale, T):
+    """The largest logit's term of the sum is 1, so that no log-prob is positive. Error: half a unit in the last place of m + log l and of the
+    two scaled logits (2^-24 of the next power of two each), the sum's and the fast logarithm's 4e-6."""
+    from verl_b200.ops import functional as F
+
+    g = torch.Generator(device=DEV).manual_seed(int(scale))
+    lg = (torch.randn(512, 20011, device=DEV, generator=g) * scale).bfloat16()
+    tok, lp = F.sample_tokens(lg, T, torch.arange(512, device=DEV), 3, 0)
+    x = lg.double() * (torch.tensor(1.0 / T if T else 1.0, dtype=torch.float32)).double()
+    want = x.gather(1, tok[:, None])[:, 0] - x.logsumexp(-1)
+    unit = 2.0 ** (x.max(-1).values.abs().log2().ceil() - 24)
+    assert ((lp.double() - want).abs() <= (1 if T in (1.0, 0.0) else 3) * unit + 4e-6).all()
+    assert float(lp.max()) <= 2.0**-22
+
+
 @pytest.mark.parametrize("V,ld,valid", [(8, 8, 0), (1000, 1000, 0), (2049, 2056, 0), (33001, 33003, 32999)])
 def test_sampler_of_rows_without_numbers(ops, V, ld, valid):
     """NaN and masked logits: a token of the vocabulary all the same (the first where there is none to take), and a log-prob that is NaN."""

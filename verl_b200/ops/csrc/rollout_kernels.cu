@@ -317,20 +317,29 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z) {
 // chip and many rows end together (a CTA per row: 320 rows were two waves of 148 x 2). A thread takes 8 neighbouring logits
 // at a time: one rescaling of the running sum and one exponential per logit. That exponential also decides which logits need their two
 // logarithms at all: x + g(u) can beat the warp's best score s only if u >= exp(-exp(x - s)), and exp(-t) >= 1 - t, so a logit with
-// u < 1 - t, t = e^(x - m) e^(m - s), cannot win. The bound is widened by 66 / 2^24 and a factor 1 + 2^-10 on t, far above the rounding
-// of its terms and of the logarithms, and the 64 uppermost values of u always count as candidates, so the token is the one that
-// evaluating every logit gives (of equal scores the first). What is left is the 64-bit hash: 44 instructions a logit in all, issued in
-// two of three cycles; loading a turn ahead and collecting the candidates of a turn in a mask were both slower (98 and 105 us).
-// 320 x 152064 at temperature 1: 160 us -> 96 us; greedy, where the row is what counts: 37 us (15 us for the bytes).
+// u < 1 - t, t = e^(x - m) e^(m - s), cannot win. The bound is widened by 66 / 2^24 and by 2^-10 + 2^-21 |m| in the exponent of t, far above
+// the rounding of its terms (scores as large as m carry 2^-24 |m| each) and of the logarithms, and the 64 uppermost values of u always
+// count as candidates, so the token is the one that evaluating every logit gives (of equal scores the first). The exponent is the difference
+// of two logits as stored, times the scale: with the scale folded into one fma against a rounded maximum, the largest logit's own term was
+// not 1, and log-probs near 0 were off by up to 2^-22 |m| and sometimes positive. What is left is the 64-bit hash; loading a turn ahead and
+// collecting the candidates of a turn in a mask were both slower.
+// 320 x 152064 at temperature 1, captured: 140 us with a CTA per row -> 92 us; greedy, where the row is what counts: 92 -> 34 us (15 us for the
+// bytes at the copy rate).
 constexpr int SAMPLE_THREADS = 256;
 
 struct SamplePart {
-  float m, l, best, best_x;
+  float m, l, best, best_x;  // m: largest logit as stored; l: sum of e^((x - m) / temperature)
   int best_i;
 };
-__device__ __forceinline__ void sample_fold(SamplePart& a, const SamplePart& b) {
+__device__ __forceinline__ float exp2_approx(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// it2: log2(e) / temperature
+__device__ __forceinline__ void sample_fold(SamplePart& a, const SamplePart& b, float it2) {
   const float mn = fmaxf(a.m, b.m);
-  a.l = (mn == -INFINITY) ? a.l + b.l : a.l * __expf(a.m - mn) + b.l * __expf(b.m - mn);
+  a.l = (mn == -INFINITY) ? a.l + b.l : a.l * exp2_approx((a.m - mn) * it2) + b.l * exp2_approx((b.m - mn) * it2);
   a.m = mn;
   if (b.best > a.best || (b.best == a.best && b.best_i < a.best_i)) {
     a.best = b.best;
@@ -345,11 +354,6 @@ __device__ __forceinline__ uint32_t sample_bits(uint64_t key, int i) {
   z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
   z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
   return static_cast<uint32_t>(z >> 40);
-}
-__device__ __forceinline__ float exp2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
 }
 __device__ __forceinline__ float sample_score(float x, uint32_t h) {
   const float u = (static_cast<float>(h) + 0.5f) * (1.0f / 16777216.0f);  // (0,1)
@@ -397,10 +401,9 @@ sample_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int valid_
     float mx = x[0];
 #pragma unroll
     for (int j = 1; j < 8; ++j) mx = fmaxf(mx, x[j]);
-    const float mn = fmaxf(a.m, mx * it);
+    const float mn = fmaxf(a.m, mx);
     const float ref = mn == -INFINITY ? 0.f : mn;  // nothing but masked logits so far: their exponentials are 0
-    float sum = a.l * __expf(a.m - ref);
-    const float ref2 = ref * LOG2E;
+    float sum = a.l * exp2_approx((a.m - ref) * it2);
     if (!GREEDY && warp_best == -INFINITY) {
       // a first score to beat: every lane's largest logit
       int jm = 0;
@@ -414,10 +417,11 @@ sample_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int valid_
       }
       warp_best = warp_max(a.best);
     }
-    const float t_scale = 8388608.f * 1.0009765625f * __expf(ref - warp_best);
+    const float rt = ref * it;
+    const float t_scale = 8388608.f * __expf(rt - warp_best + fmaf(fabsf(rt), 4.76837158e-7f, 9.765625e-4f));
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float e = exp2_approx(fmaf(x[j], it2, -ref2));
+      const float e = exp2_approx((x[j] - ref) * it2);
       sum += e;
       if (GREEDY) {
         if (x[j] > a.best) {
@@ -448,21 +452,21 @@ sample_kernel(const __nv_bfloat16* __restrict__ logits, long long ld, int valid_
   for (int o = 16; o > 0; o >>= 1) {
     const SamplePart b{__shfl_xor_sync(0xffffffffu, a.m, o), __shfl_xor_sync(0xffffffffu, a.l, o), __shfl_xor_sync(0xffffffffu, a.best, o),
                        __shfl_xor_sync(0xffffffffu, a.best_x, o), __shfl_xor_sync(0xffffffffu, a.best_i, o)};
-    sample_fold(a, b);
+    sample_fold(a, b, it2);
   }
   __shared__ SamplePart warp_part[SAMPLE_THREADS / 32];
   __shared__ SamplePart cta_part;
   if (lane == 0) warp_part[threadIdx.x >> 5] = a;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int k = 1; k < SAMPLE_THREADS / 32; ++k) sample_fold(a, warp_part[k]);
+    for (int k = 1; k < SAMPLE_THREADS / 32; ++k) sample_fold(a, warp_part[k], it2);
     cta_part = a;
   }
   cluster.sync();
   if (part == 0 && threadIdx.x == 0) {
-    for (int k = 1; k < parts; ++k) sample_fold(a, *cluster.map_shared_rank(&cta_part, k));
+    for (int k = 1; k < parts; ++k) sample_fold(a, *cluster.map_shared_rank(&cta_part, k), it2);
     tokens[row] = a.best_i == 0x7fffffff ? 0 : a.best_i;
-    if (logprobs) logprobs[row] = a.m == -INFINITY ? __int_as_float(0x7fffffff) : a.best_x - (a.m + __logf(a.l));  // no token: NaN
+    if (logprobs) logprobs[row] = a.m == -INFINITY ? __int_as_float(0x7fffffff) : a.best_x - (a.m * it + __logf(a.l));  // no token: NaN
   }
   cluster.sync();  // a CTA's shared memory is read by its cluster until here
 }
