@@ -843,7 +843,11 @@ class RolloutEngine:
         else:
             key = (self.temperature, self.top_k, self.top_p, self.out_cap, id(self.kv))
             if self._graph is None or self._graph_key != key:
-                snap = [t.clone() for t in (self.tok, self.pos, self.ctx, self.gen, self.active, self.seeds, self.out_tok, self.out_lp)]
+                # what a step changes and the first replay has to find as it is now (cached keys and recorded routing are written again alike)
+                kept = [self.tok, self.pos, self.ctx, self.gen, self.active, self.seeds, self.out_tok, self.out_lp]
+                if self._use_penalty:
+                    kept.append(self.seen)
+                snap = [t.clone() for t in kept]
                 side = torch.cuda.Stream(device=self.device)
                 side.wait_stream(torch.cuda.current_stream(self.device))
                 if self.cache.has_state:
@@ -851,7 +855,7 @@ class RolloutEngine:
                 with torch.cuda.stream(side):
                     self._decode_body()  # warm-up (allocator, lazy init) outside capture
                 torch.cuda.current_stream(self.device).wait_stream(side)
-                for dst, src in zip((self.tok, self.pos, self.ctx, self.gen, self.active, self.seeds, self.out_tok, self.out_lp), snap):
+                for dst, src in zip(kept, snap):
                     dst.copy_(src)
                 from ....ops import native
 
@@ -862,7 +866,7 @@ class RolloutEngine:
                     self._decode_body()
                 self._graph_kernels = native.launch_count() - n0
                 native.add_launches(-self._graph_kernels)  # captured, not launched
-                for dst, src in zip((self.tok, self.pos, self.ctx, self.gen, self.active, self.seeds, self.out_tok, self.out_lp), snap):
+                for dst, src in zip(kept, snap):
                     dst.copy_(src)
                 self._graph, self._graph_key = g, key
             for _ in range(n):
