@@ -74,6 +74,29 @@ def test_group_advantage_rows(ops, B, L, dtype):
         assert rel(score.cpu(), s) < 1e-6 and rel(adv.cpu(), want[:, None] * m.double()) < (1e-5 if B <= 1024 else 2e-4)
 
 
+@pytest.mark.parametrize("B", [2, 1024, 1025, 4000])
+@pytest.mark.parametrize("offset,spread", [(0.5, 0.3), (50.0, 0.01), (-1000.0, 0.01)])
+def test_group_advantage_of_close_scores(ops, B, offset, spread):
+    """One reward per row, so that the scores are exact: mean and deviation then leave only the rounding of the result (2^-24)."""
+    from verl_b200.ops import functional as F
+
+    g = torch.Generator().manual_seed(B)
+    ids = torch.randint((B + 4) // 5, (B,), generator=g)
+    r = torch.zeros(B, 5)
+    r[:, 3] = offset + spread * torch.randn(B, generator=g)
+    s = r.double().sum(-1)
+    n = torch.bincount(ids)[ids]
+    mean = (torch.zeros(B, dtype=torch.float64).index_add(0, ids, s)[ids] / n) * (n > 1)
+    var = torch.zeros(B, dtype=torch.float64).index_add(0, ids, (s - mean) ** 2)[ids] / (n - 1).clamp(min=1)
+    for by_std in (True, False):
+        adv, score = F.grpo_advantage(r.to(DEV), torch.ones(B, 5, device=DEV), ids.to(DEV), (B + 4) // 5, 1e-6, by_std)
+        want = (s - mean) / (torch.where(n > 1, var.sqrt(), 1.0) + 1e-6) if by_std else s - mean
+        assert torch.equal(score.cpu().double(), s)
+        # (the double sums of squares of more than 1024 rows: 2^-53 n offset^2 / spread^2 below 1e-4 of a variance at the widest ratio)
+        bound = 1e-6 + (1e-14 * (offset / spread) ** 2 if B > 1024 else 0)
+        assert rel(adv.cpu(), want[:, None].expand(B, 5)) < bound
+
+
 # ------------------------------------------------------------------------------------------------ sampler
 def _uniforms(seeds, V, step):
     """The sampler's stream of uniforms: splitmix64's finaliser on uint64, the upper 24 bits, halfway between the grid points."""

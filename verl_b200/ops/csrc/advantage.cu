@@ -6,11 +6,12 @@
 
 namespace vb {
 
-// scores[b] = sum_t rewards[b,t]; one block per row. With `stats` (zeroed by the caller) also stats[g] += {sum, sumsq, count}.
+// scores[b] = sum_t rewards[b,t]; one block per row. With `stats` (zeroed by the caller) also stats[g] += {sum, sum of squares, count}, in
+// double: sums of fp32 scores and of their squares are then good for a variance far below the square of the mean.
 template <typename I>
 __global__ void __launch_bounds__(128)
 grpo_scores_kernel(const float* __restrict__ rewards, const I* __restrict__ group, int L, float* __restrict__ scores,
-                   float* __restrict__ stats) {
+                   double* __restrict__ stats) {
   __shared__ float red[4];
   const float* row = rewards + static_cast<long long>(blockIdx.x) * L;
   float s = 0.f;
@@ -23,58 +24,71 @@ grpo_scores_kernel(const float* __restrict__ rewards, const I* __restrict__ grou
     const float tot = red[0] + red[1] + red[2] + red[3];
     scores[blockIdx.x] = tot;
     if (stats) {
-      float* st = stats + 3 * static_cast<long long>(group[blockIdx.x]);
-      atomicAdd(st, tot);
-      atomicAdd(st + 1, tot * tot);
-      atomicAdd(st + 2, 1.f);
+      double* st = stats + 3 * static_cast<long long>(group[blockIdx.x]);
+      atomicAdd(st, static_cast<double>(tot));
+      atomicAdd(st + 1, static_cast<double>(tot) * tot);
+      atomicAdd(st + 2, 1.0);
     }
   }
 }
 
-__device__ __forceinline__ float grpo_block_sum(float v, float* red) {
+// Sums of a and b over the block.
+__device__ __forceinline__ void grpo_block_sum(double& a, int& b, double (&ra)[4], int (&rb)[4]) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+  b = __reduce_add_sync(0xffffffffu, b);
   __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  if ((threadIdx.x & 31) == 0) {
+    ra[threadIdx.x >> 5] = a;
+    rb[threadIdx.x >> 5] = b;
+  }
   __syncthreads();
-  return red[0] + red[1] + red[2] + red[3];
+  a = ra[0] + ra[1] + ra[2] + ra[3];
+  b = rb[0] + rb[1] + rb[2] + rb[3];
 }
 
 // adv[b,t] = (score - mean_g) / (std_g + eps) * mask[b,t]   (unbiased std; singleton group: mean 0, std 1). Without `stats` a row's
-// block finds the members of its group among the B scores itself: the mean first, then the squares around it (no cancellation), with
-// neither a zeroed scratch nor atomics. That scan is quadratic in B over the whole grid, so it is taken up to GRPO_SCAN_ROWS.
+// block finds the members of its group among the B scores itself: the mean first, then the squares around it, with neither a zeroed scratch
+// nor atomics. That scan is quadratic in B over the whole grid, so it is taken up to GRPO_SCAN_ROWS. Mean and variance are formed in double
+// on both ways: a group's scores can lie as close together as fp32 can tell (50 +- 0.01: with fp32 sums the advantages were off by 2e-4 with
+// the scan, and meaningless from the atomics).
 template <typename I>
 __global__ void __launch_bounds__(128)
-grpo_adv_kernel(const float* __restrict__ scores, const I* __restrict__ group, const float* __restrict__ stats,
+grpo_adv_kernel(const float* __restrict__ scores, const I* __restrict__ group, const double* __restrict__ stats,
                 const float* __restrict__ mask, int B, int L, float eps, int norm_by_std, float* __restrict__ adv) {
-  __shared__ float red[4];
+  __shared__ double red[4];
+  __shared__ int red_n[4];
   const int b = blockIdx.x;
   const I g = group[b];
-  float n = 0.f, sum = 0.f;
+  int n = 0;
+  double sum = 0.0;
   if (stats) {
-    n = stats[3 * static_cast<long long>(g) + 2];
+    n = static_cast<int>(stats[3 * static_cast<long long>(g) + 2]);
     sum = stats[3 * static_cast<long long>(g)];
   } else {
     for (int i = threadIdx.x; i < B; i += 128)
       if (group[i] == g) {
-        n += 1.f;
+        n += 1;
         sum += scores[i];
       }
-    n = grpo_block_sum(n, red);
-    sum = grpo_block_sum(sum, red);
+    grpo_block_sum(sum, n, red, red_n);
   }
-  float mean = 0.f, sd = 1.f;
-  if (n > 1.5f && stats) {
+  double mean = 0.0, sd = 1.0;
+  if (n > 1) {
     mean = sum / n;
-    sd = sqrtf(fmaxf((stats[3 * static_cast<long long>(g) + 1] - n * mean * mean) / (n - 1.f), 0.f));
-  } else if (n > 1.5f) {
-    mean = sum / n;
-    float sq = 0.f;
-    for (int i = threadIdx.x; i < B; i += 128)
-      if (group[i] == g) sq += (scores[i] - mean) * (scores[i] - mean);
-    sd = sqrtf(grpo_block_sum(sq, red) / (n - 1.f));
+    double sq = 0.0;
+    if (stats) {
+      sq = stats[3 * static_cast<long long>(g) + 1] - n * mean * mean;
+      if (sq < 0.0) sq = 0.0;  // (NaN stays)
+    } else {
+      int unused = 0;
+      for (int i = threadIdx.x; i < B; i += 128)
+        if (group[i] == g) sq += (scores[i] - mean) * (scores[i] - mean);
+      grpo_block_sum(sq, unused, red, red_n);
+    }
+    sd = sqrt(sq / (n - 1));
   }
-  const float a = norm_by_std ? (scores[b] - mean) / (sd + eps) : (scores[b] - mean);
+  const float a = static_cast<float>(norm_by_std ? (scores[b] - mean) / (sd + eps) : scores[b] - mean);
   const long long row = static_cast<long long>(b) * L;
   for (int t = threadIdx.x; t < L; t += 128) adv[row + t] = a * mask[row + t];
 }
@@ -220,12 +234,12 @@ extern "C" {
 constexpr int GRPO_SCAN_ROWS = 1024;
 int vb_grpo_needs_stats(int B) { return B > GRPO_SCAN_ROWS; }
 
-// group: int32 or int64 ids (group64); ids in [0, num_groups). stats: 3 * num_groups floats (zeroed here) when vb_grpo_needs_stats.
+// group: int32 or int64 ids (group64); ids in [0, num_groups). stats: 3 * num_groups doubles (zeroed here) when vb_grpo_needs_stats.
 int vb_grpo_advantage(const float* rewards, const float* mask, const void* group, int group64, int B, int L, int num_groups, float eps,
-                      int norm_by_std, float* scores, float* stats, float* adv, cudaStream_t s) {
+                      int norm_by_std, float* scores, double* stats, float* adv, cudaStream_t s) {
   if (B == 0) return 0;
   if (vb_grpo_needs_stats(B))
-    cudaMemsetAsync(stats, 0, sizeof(float) * 3 * num_groups, s);
+    cudaMemsetAsync(stats, 0, sizeof(double) * 3 * num_groups, s);
   else
     stats = nullptr;
   if (group64) {

@@ -677,11 +677,11 @@ std::tuple<Tensor, Tensor> grpo_advantage(const Tensor& rewards, const Tensor& m
   const int64_t B = rewards.size(0), L = rewards.size(1);
   Tensor adv = at::empty_like(rewards);
   Tensor scores = at::empty({B}, rewards.options());
-  Tensor stats = vb_grpo_needs_stats((int)B) ? at::empty({num_groups, 3}, rewards.options()) : Tensor();
+  Tensor stats = vb_grpo_needs_stats((int)B) ? at::empty({num_groups, 3}, rewards.options().dtype(at::kDouble)) : Tensor();
   count(2);
   CHECK_RC(vb_grpo_advantage(rewards.data_ptr<float>(), mask.data_ptr<float>(), group.data_ptr(), group.scalar_type() == at::kLong, (int)B,
                              (int)L, (int)num_groups, (float)eps, norm_by_std, scores.data_ptr<float>(),
-                             stats.defined() ? stats.data_ptr<float>() : nullptr, adv.data_ptr<float>(), cur_stream()),
+                             stats.defined() ? stats.data_ptr<double>() : nullptr, adv.data_ptr<float>(), cur_stream()),
            "vb_grpo_advantage");
   return {adv, scores};
 }

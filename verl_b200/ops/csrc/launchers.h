@@ -168,7 +168,7 @@ int vb_moe_publish_counts(const int* counts, const unsigned long long* table_ptr
 // advantage.cu
 int vb_grpo_needs_stats(int B);
 int vb_grpo_advantage(const float* rewards, const float* mask, const void* group, int group64, int B, int L, int num_groups, float eps,
-                      int norm_by_std, float* scores, float* stats, float* adv, cudaStream_t s);
+                      int norm_by_std, float* scores, double* stats, float* adv, cudaStream_t s);
 int vb_gae_blocks(int B);
 int vb_gae(const float* rewards, const float* values, const float* mask, int B, int L, float gamma, float lam, float* adv, float* ret,
            double* part, cudaStream_t s);
