@@ -287,6 +287,42 @@ def test_attention_of_prompts_and_their_continuations(ops, hd, nh, nkv, groups):
             assert float((got.double() - w).norm()) < 1.5e-2 * float(w.norm()) + small
 
 
+@pytest.mark.parametrize("hd,nh,nkv", [(128, 4, 4), (64, 4, 2)])
+@pytest.mark.parametrize("lens,parent", [([70, 40, 33, 130, 5], [-1, -1, 0, 1, 0]), ([9, 200, 130], [1, -1, 1]), ([40, 129, 64, 1], [3, -1, 3, -1]),
+                                         ([100, 50, 60], [-1, 0, 1])])
+def test_continuations_anywhere_in_the_stream(ops, hd, nh, nkv, lens, parent):
+    """Sequences that continue an earlier or a later one with others between, and one that continues a continuation (of which it sees only the
+    keys of its own parent). One head per KV head: the prompt's own CTA would store what others add."""
+    from verl_b200.ops import functional as F
+
+    cu = np.cumsum([0] + lens).tolist()
+    keys = [(list(range(cu[p], cu[p + 1])) if p >= 0 else []) + list(range(a, a + i + 1)) for a, n, p in zip(cu, lens, parent) for i in range(n)]
+    T = cu[-1]
+    g = torch.Generator(device=DEV).manual_seed(T)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g).bfloat16()
+    q, k, v, dout = rnd(T, nh, hd), rnd(T, nkv, hd), rnd(T, nkv, hd), rnd(T, nh, hd)
+    cu_t, par_t = torch.tensor(cu, dtype=torch.int32, device=DEV), torch.tensor(parent, dtype=torch.int32, device=DEV)
+    out, lse = F.attention_shared_prefix(q, k, v, cu_t, par_t)
+    ref = [t.double().requires_grad_(True) for t in (q, k, v)]
+    want = _attention64(*ref, keys, hd**-0.5)
+    assert rel(out, want.detach()) < 6e-3
+    want.backward(dout.double())
+    got = [torch.empty_like(t) for t in (q, k, v)]
+    for _ in range(3):
+        F.attention_bwd_into_(dout, q, k, v, out, lse, cu_t, max(lens), *got, parent=par_t)
+        for x, w in zip(got, ref):
+            assert rel(x, w.grad) < 1.5e-2  # dS is rounded to bf16 and its terms cancel
+
+
+def test_audit_names_a_parent_out_of_range():
+    from verl_b200.ops import audit
+    from verl_b200.ops import functional as F
+
+    x, cu = torch.zeros(4, 2, 64, device=DEV, dtype=torch.bfloat16), torch.tensor([0, 2, 4], dtype=torch.int32, device=DEV)
+    with audit.scope(), pytest.raises(audit.AuditError, match="parent"):
+        F.attention_shared_prefix(x, x, x, cu, torch.tensor([-1, 2], dtype=torch.int32, device=DEV))
+
+
 @pytest.mark.parametrize("preset,layers", [("qwen2.5-0.5b", 2), ("tiny-shared", 2)])
 def test_update_with_shared_prompts_equals_separate_rows(ops, preset, layers):
     from verl_b200.models import DecoderModel, FlatParams

@@ -134,8 +134,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   const int ntiles = (keylen + AB_BK - 1) / AB_BK;
   if (ntiles > p.max_tiles && blockIdx.z == 0 && threadIdx.x == 0) atomicExch(p.status, ST_BAD_ARGS);  // max_seqlen too small
   if (from_end >= ntiles || seqlen <= 0) return;  // shorter sequence
-  // dK / dV of this block are also written by CTAs of other heads or query sequences
-  const bool shared_keys = p.hsplit > 1 || cross || (p.parent != nullptr && ks + 1 < p.num_seqs && p.parent[ks + 1] == ks);
+  bool has_child = false;  // of the sequences that this thread looks at
+  if (p.parent != nullptr && !cross)
+    for (int s = threadIdx.x; s < p.num_seqs; s += AB_THREADS) has_child |= p.parent[s] == ks;
   const int k0 = (ntiles - 1 - from_end) * AB_BK;
 
   if (threadIdx.x == 0) {
@@ -158,7 +159,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     tmem_relinquish();
   }
   tc_fence_before();
-  __syncthreads();
+  // dK / dV of this block are also written by CTAs of other heads, or of sequences that continue this one, wherever they stand
+  const bool shared_keys = (__syncthreads_or(has_child) != 0) || p.hsplit > 1 || cross;
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
   const int i0 = cross ? 0 : k0 / AB_BQ;                        // first query block at or below the diagonal

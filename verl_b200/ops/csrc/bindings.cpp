@@ -210,8 +210,8 @@ const int* check_seqs(const Tensor& cu, const OptTensor& parent, const char* who
 }
 
 // Causal GQA attention over packed sequences. q [T, nh, hd], k/v [T, nkv, hd] (strided views), cu_seqlens int32 [B+1].
-// parent (int32 [B], -1: none): the sequence whose keys a sequence's queries see in front of their own; it must have no parent itself,
-// and its children follow it directly. Returns (out [T, nh, hd] bf16, lse [nh, T] fp32).
+// parent (int32 [B], -1: none): the sequence whose keys a sequence's queries see in front of their own (not those of the parent's parent).
+// Returns (out [T, nh, hd] bf16, lse [nh, T] fp32).
 std::tuple<Tensor, Tensor> attn_fwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_seqlens,
                                     double scale, const OptTensor& parent) {
   check_heads(q, "attn_fwd");

@@ -486,10 +486,11 @@ def native_attention(q: torch.Tensor) -> bool:
 
 
 def attention_shared_prefix(q, k, v, cu_seqlens, parent, scale: Optional[float] = None):
-    """Causal GQA attention over a packed stream whose sequences may continue another one: the queries of sequence ``s`` see every
-    key of sequence ``parent[s]`` (-1: none) and then their own, causally. A parent has no parent itself and its children follow it
-    directly (a prompt and the responses of its group). Native kernels only (``native_attention``). Returns (out, lse)."""
+    """Causal GQA attention over a packed stream whose sequences may continue another one (the responses of a group behind their prompt):
+    the queries of sequence ``s`` see every key of sequence ``parent[s]`` (-1: none; a parent's own parent is not seen) and then their
+    own, causally. Native kernels only (``native_attention``). Returns (out, lse)."""
     scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
+    audit.check_index("attention_shared_prefix", "parent", parent, cu_seqlens.numel() - 1, skip_negative=True)
     return _ops().attn_fwd(q, k, v, cu_seqlens, float(scale), parent)
 
 
@@ -500,6 +501,7 @@ def attention_bwd_into_(dout, q, k, v, out, lse, cu_seqlens, max_seqlen: int, dq
     only; ``max_seqlen``: the longest sequence of ``cu_seqlens``."""
     scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
     pos, cos_t, sin_t = rope if rope is not None else (None, None, None)
+    audit.check_index("attention_bwd_into_", "parent", parent, cu_seqlens.numel() - 1, skip_negative=True)
     if pos is not None:
         audit.check_index("attention_bwd_into_", "positions", pos, cos_t.shape[0])
         pos = pos.to(torch.int32).contiguous()
