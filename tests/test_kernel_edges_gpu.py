@@ -314,6 +314,37 @@ def test_continuations_anywhere_in_the_stream(ops, hd, nh, nkv, lens, parent):
             assert rel(x, w.grad) < 1.5e-2  # dS is rounded to bf16 and its terms cancel
 
 
+@pytest.mark.parametrize("where,dtype", [("cpu", torch.int32), ("cpu", torch.int64), (DEV, torch.int64)])
+def test_lengths_from_the_host(where, dtype):
+    """An update over a batch whose lengths lie on the host, as the plain attention ops take them, and both ops on a shared prompt."""
+    from verl_b200.models import DecoderModel, FlatParams, PackedBatch
+    from verl_b200.models.config import get_preset
+    from verl_b200.ops import functional as F
+
+    cfg = get_preset("qwen2.5-0.5b")
+    cfg.num_hidden_layers = 1
+    got = []
+    for kind in ("as packed", "moved"):
+        params = FlatParams(cfg, dtype=torch.bfloat16, device=DEV, with_main_grad=True)
+        params.init_weights(seed=3, std=0.05)
+        batch = PackedBatch.from_lengths(torch.arange(3, 53, device=DEV), [20, 30], device=DEV)
+        if kind == "moved":
+            batch.cu_seqlens = batch.cu_seqlens.to(where, dtype)
+        lp, _ = DecoderModel(cfg, params).forward_logprobs(batch, torch.arange(4, 54, device=DEV), 1.0)
+        lp.sum().backward()
+        got.append((lp.detach(), params.main_grad))
+    assert torch.equal(got[0][0], got[1][0]) and rel(got[1][1], got[0][1]) < 1e-3
+    x = torch.randn(50, 2, 64, device=DEV).bfloat16()
+    cu, parent = torch.tensor([0, 20, 50], dtype=torch.int32, device=DEV), torch.tensor([-1, 0], dtype=torch.int32, device=DEV)
+    res = []
+    for c, p in ((cu, parent), (cu.to(where, dtype), parent.to(where, dtype))):
+        out, lse = F.attention_shared_prefix(x, x, x, c, p)
+        grads = [torch.empty_like(x) for _ in range(3)]
+        F.attention_bwd_into_(x, x, x, x, out, lse, c, 30, *grads, parent=p)
+        res.append([out, *grads])
+    assert torch.equal(res[0][0], res[1][0]) and all(rel(a, b) < 1e-3 for a, b in zip(res[1], res[0]))
+
+
 def test_audit_names_a_parent_out_of_range():
     from verl_b200.ops import audit
     from verl_b200.ops import functional as F

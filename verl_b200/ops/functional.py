@@ -491,7 +491,7 @@ def attention_shared_prefix(q, k, v, cu_seqlens, parent, scale: Optional[float] 
     own, causally. Native kernels only (``native_attention``). Returns (out, lse)."""
     scale = scale if scale is not None else 1.0 / math.sqrt(q.shape[-1])
     audit.check_index("attention_shared_prefix", "parent", parent, cu_seqlens.numel() - 1, skip_negative=True)
-    return _ops().attn_fwd(q, k, v, cu_seqlens, float(scale), parent)
+    return _ops().attn_fwd(q, k, v, cu_seqlens.to(q.device, torch.int32), float(scale), parent.to(q.device, torch.int32))
 
 
 def attention_bwd_into_(dout, q, k, v, out, lse, cu_seqlens, max_seqlen: int, dq, dk, dv, parent=None, rope=None,
@@ -505,7 +505,10 @@ def attention_bwd_into_(dout, q, k, v, out, lse, cu_seqlens, max_seqlen: int, dq
     if pos is not None:
         audit.check_index("attention_bwd_into_", "positions", pos, cos_t.shape[0])
         pos = pos.to(torch.int32).contiguous()
-    _ops().attn_bwd_into_(dout, q, k, v, out, lse, cu_seqlens.to(torch.int32), int(max_seqlen), float(scale), parent, dq, dk, dv, pos, cos_t, sin_t)
+    if parent is not None:
+        parent = parent.to(q.device, torch.int32)
+    _ops().attn_bwd_into_(dout, q, k, v, out, lse, cu_seqlens.to(q.device, torch.int32), int(max_seqlen), float(scale), parent, dq, dk, dv, pos,
+                          cos_t, sin_t)
 
 
 def _attention_query_slice(q, k, v, cu_seqlens, q_start: int, scale: float):
