@@ -649,9 +649,10 @@ def test_qk_norm_backward_in_place(ops, T, nh, nkv, hd):
 
 # ------------------------------------------------------------------------------------------------ a group's heads over several CTAs
 @pytest.mark.parametrize("nh,nkv,hd,lens", [(64, 32, 64, [700, 600]), (7, 1, 64, [1, 64, 65, 300]), (48, 16, 128, [513, 97, 700, 640]),
-                                            (14, 2, 128, [31, 33, 129])])
+                                            (14, 2, 128, [31, 33, 129]), (32, 8, 64, [1500, 700]), (14, 2, 128, [400] * 6)])
 def test_attention_backward_over_shares_of_heads(ops, nh, nkv, hd, lens):
-    """One CTA for all heads of a group, two, and one per head; without parents, so that a single CTA stores dK and dV."""
+    """One CTA for all heads of a group, two, four (the last with fewer heads), and one per head; without parents, so that a single CTA stores
+    dK and dV."""
     from verl_b200.ops import functional as F
 
     T = sum(lens)

@@ -532,16 +532,34 @@ extern "C" int vb_attn_bwd(const void* q, const void* k, const void* v, const vo
   float* dk32 = dkv32_ws;
   float* dv32 = dkv32_ws + T * nkv * hd;
   cudaError_t e = cudaMemsetAsync(dq32_ws, 0, sizeof(float) * static_cast<size_t>(T) * nh * hd, stream);
-  // Heads of a group per CTA. The longest CTA has max_seqlen / 64 steps per head; an SM has about nkv * G * T * max_seqlen / 2 / (128 * 64)
-  // / SMs of them (sequences of about the longest length). The longest CTA is to have no more steps than an SM; every further share costs
-  // 1 to 3% in loads of K and V and additions of dK and dV.
-  const int G = nh / nkv;
-  const double longest = 2.0 * 128 * num_sms() / (static_cast<double>(nkv) * total_tokens);  // in SMs' shares, all heads in one CTA
-  int hsplit = static_cast<int>(longest < G ? ceil(longest) : G);
-  if (hsplit > G) hsplit = G;
-  if (hsplit < 1) hsplit = 1;
+  // Shares that a group's heads are dealt in: the number whose launch is estimated shortest. A CTA takes its steps and about three more
+  // (set-up, loads of K and V, dK and dV out: with sequences of 40 tokens that is most of it). A launch takes as long as its longest CTA, the
+  // first key block of the longest sequence, or as an SM's share of all CTAs and some of what comes last: a quarter of a last key block,
+  // or, with parents, most of a long CTA, because queries behind a prompt meet its last key blocks as often as its first. Only the longest
+  // sequence is known here, so total_tokens / max_seqlen sequences of that length stand for all, and a continuation for a CTA per key block.
+  // Best share, its time and that of one share, 28 / 4 heads of 128: 64 x 40 tokens 1 (78 us; 104 with four), 8 x 1000 1 (393; 411 with two),
+  // 5 x 1000 2 (267; 339), 3 x 1000 4 (168; 318), 1 x 3072 4 (327; 820), 1 x 200 7 (27; 90); two prompts with five continuations 2 (792; 825);
+  // 32 / 8 heads, three prompts of 900 with eight continuations of 50 1 (411; 519 with two). Within 6% of the best share over 33 shapes, heads
+  // of 64 among them.
+  const int G = nh / nkv, sms = num_sms();
+  const double qb = (max_seqlen + AB_BQ - 1) / AB_BQ, kb = (max_seqlen + AB_BK - 1) / AB_BK, extra = 3.0;
+  const double seqs = total_tokens > max_seqlen ? static_cast<double>(total_tokens) / max_seqlen : 1.0;
+  const double blocks = kb * (seqs + (parent != nullptr ? num_seqs : 0));
+  int hsplit = 1;
+  double shortest = 0.0;
+  for (int share = 1; share <= G; ++share) {
+    const int per = (G + share - 1) / share;
+    if ((G + per - 1) / per != share) continue;  // deals the heads as fewer shares do
+    const double longest = per * qb + extra;
+    const double mean = nkv * (seqs * G * kb * (qb - kb + 1) + share * blocks * extra) / sms;
+    const double all = mean + (parent != nullptr ? 0.75 * longest : 0.25 * (2 * per + extra));
+    const double est = longest > all ? longest : all;
+    if (share == 1 || est < shortest) {
+      shortest = est;
+      hsplit = share;
+    }
+  }
   const int heads_per = (G + hsplit - 1) / hsplit;
-  hsplit = (G + heads_per - 1) / heads_per;
   if (e == cudaSuccess && (parent != nullptr || hsplit > 1)) e = cudaMemsetAsync(dkv32_ws, 0, sizeof(float) * 2 * static_cast<size_t>(T) * nkv * hd, stream);
   if (e != cudaSuccess) return static_cast<int>(e);
   AttnBwdParams p{};
