@@ -429,8 +429,9 @@ class DecoderModel:
         self.keep_layers_fn: Optional[Callable[[int], int]] = None
         self.tp: Optional[TensorParallelShard] = None  # set by the rollout engine; forward-only
         # set by the rollout engine for dense models: its products of at most 64 tokens may take kernels that sum in another order. Scoring
-        # and updates stay on one family, so that their log-probs of a sequence agree, and so do mixture-of-experts models: a router
-        # turns a last bit of its input into another choice of experts, and log-probs of a short rollout then move by 10%
+        # and updates do not, so that their log-probs of a sequence agree, and neither do mixture-of-experts models: a router turns a last
+        # bit of its input into another choice of experts, and log-probs of a short rollout then move by 10%. (Their expert products run
+        # on tiles of 16 to 128 rows, see _moe_tile, and give the same bits on all of them.)
         self.decode_kernels = False
         self.fp8_weights: Optional[dict] = None         # data_ptr of a bf16 weight -> (e4m3 copy, block scales)
         self.offloader = None                           # ActivationOffloader: inputs of recomputed layers live on the host
