@@ -417,7 +417,8 @@ def _choices(T, k, E, seed, skew=False):
 
 @pytest.mark.parametrize("tile", [16, 32, 64, 128])
 @pytest.mark.parametrize("T,k,E,skew", [(1, 1, 1, False), (3, 2, 5, True), (32, 8, 128, False), (257, 4, 60, True), (2049, 8, 128, False),
-                                        (40, 2, 1024, False)])
+                                        (40, 2, 1024, False), (8192, 1, 3, False), (8193, 1, 1, False), (1025, 8, 1024, False), (1366, 6, 64, True),
+                                        (40000, 4, 1023, False), (30000, 8, 128, True)])
 def test_expert_plan_is_the_stable_sort_by_expert(ops, tile, T, k, E, skew):
     idx = _choices(T, k, E, T + E, skew)
     counts = torch.bincount(idx.reshape(-1), minlength=E).int()
@@ -438,6 +439,17 @@ def test_expert_plan_is_the_stable_sort_by_expert(ops, tile, T, k, E, skew):
         used = int(num)
         assert torch.equal(te[:used].long(), torch.repeat_interleave(torch.arange(E, device=DEV), pad // tile))
         assert src.numel() % tile == 0 and used <= te.numel()
+
+
+@pytest.mark.parametrize("n", [64, 20000])
+def test_expert_plan_of_foreign_counts_stays_in_range(ops, n):
+    """Choices without an expert, and counts that are not the list's: every row and every slot is one of the buffers' own."""
+    g = torch.Generator().manual_seed(n)
+    idx = torch.randint(-2, 11, (n // 2, 2), generator=g).to(DEV)
+    for counts in (torch.zeros(9), torch.full((9,), n // 9), torch.arange(9) * n):
+        slot, src, seg, te, num = ops.moe_plan(idx, counts.int().to(DEV), 16)
+        assert int(slot.min()) >= 0 and int(slot.max()) < src.numel() and int(src.min()) >= -1 and int(src.max()) < n // 2
+        assert int(te.min()) >= 0 and int(te.max()) < 9 and 0 <= int(num) <= te.numel()
 
 
 @pytest.mark.parametrize("tile", [16, 32, 64, 128])

@@ -1038,9 +1038,11 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor> moe_plan(const Tensor& expert
     num.zero_();
     return {slot, src, seg, tile_expert, num};
   }
-  count(1);
-  CHECK_RC(vb_moe_plan(experts.data_ptr(), experts.scalar_type() == at::kLong, counts.data_ptr<int>(), (int)n, (int)k, (int)E, (int)tile, (int)cap,
-                       slot.data_ptr<int>(), src.data_ptr<int>(), seg.data_ptr<int>(), tile_expert.data_ptr<int>(), num.data_ptr<int>(), cur_stream()),
+  const int blocks = vb_moe_plan_blocks((int)n);
+  Tensor hist = blocks > 0 ? at::empty({blocks, E}, opt) : Tensor();
+  count(blocks > 0 ? 2 : 1);
+  CHECK_RC(vb_moe_plan(experts.data_ptr(), experts.scalar_type() == at::kLong, counts.data_ptr<int>(), blocks > 0 ? hist.data_ptr<int>() : nullptr,
+                       (int)n, (int)k, (int)E, (int)tile, (int)cap, slot.data_ptr<int>(), src.data_ptr<int>(), seg.data_ptr<int>(), tile_expert.data_ptr<int>(), num.data_ptr<int>(), cur_stream()),
            "vb_moe_plan");
   return {slot, src, seg, tile_expert, num};
 }

@@ -154,7 +154,8 @@ int vb_moe_route_topk(const void* logits, long long ld, int T, int E, int k, int
 int vb_moe_gather_rows(const void* src, long long lds, const int* map, const float* scale, void* dst, long long ldd, int rows, int H,
                        const int* num_mtiles, int tile_rows, cudaStream_t s);
 int vb_moe_swiglu(const void* gu, void* out, int rows, int I, const int* num_mtiles, int tile_rows, cudaStream_t s);
-int vb_moe_plan(const void* experts, int wide, const int* counts, int n, int k, int E, int tile, int cap, int* slot, int* src, int* seg,
+int vb_moe_plan_blocks(int n);
+int vb_moe_plan(const void* experts, int wide, const int* counts, int* hist, int n, int k, int E, int tile, int cap, int* slot, int* src, int* seg,
                 int* tile_expert, int* num_mtiles, cudaStream_t s);
 int vb_moe_combine(const void* y, long long ldy, const int* slot, const float* w, void* out, long long ldo, int T, int H, int k,
                    cudaStream_t s);

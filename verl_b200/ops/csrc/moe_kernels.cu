@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 namespace vb {
+int num_sms();
 
 // One warp per token. logits [T, E] (bf16), E <= 1024. Writes the k largest softmax probabilities
 // (optionally renormalised to sum 1), their expert ids, and bumps the per-expert histogram.
@@ -118,10 +119,10 @@ moe_swiglu_kernel(const __nv_bfloat16* __restrict__ gu, __nv_bfloat16* __restric
 // Expert-grouped row layout: every expert's rows start at a multiple of `tile` rows, in the order of the flat list of choices.
 //   seg[e] first row of expert e (seg[E]: rows in use), tile_expert[i] expert of tile i, num_mtiles tiles in use,
 //   slot[i] row of choice i, src[row] token of the row, -1 for padding.
-// One block per expert: every block forms the prefix of the padded counts by itself, its warps count the expert's choices in their
-// share of the list and then write them in list order, so the layout does not depend on the schedule. The list is read twice from L2
-// instead of being sorted: one launch where the sort, the scans and the scatters took about twenty (250 us per layer for 45,000 choices,
-// 80 us for 256).
+// Short lists (moe_plan_kernel): one block per expert. Every block forms the prefix of the padded counts by itself, its warps count the
+// expert's choices in their share of the list and then write them in list order, so the layout does not depend on the schedule. The list is
+// read twice per expert from L2 instead of being sorted: one launch where the sort, the scans and the scatters took about twenty (80 us per
+// layer for 256 choices). Time grows with experts x choices; long lists take the two launches below.
 template <typename IT>
 __global__ void __launch_bounds__(256)
 moe_plan_kernel(const IT* __restrict__ experts, const int* __restrict__ counts, int n, int k, int E, int tile, int cap, int* __restrict__ slot,
@@ -203,6 +204,117 @@ moe_plan_kernel(const IT* __restrict__ experts, const int* __restrict__ counts, 
       }
       at += __popc(bal[u]);
     }
+  }
+}
+
+// The same layout for long lists: every block takes a piece of the list. The first launch counts a piece's choices per expert, the second
+// places them: behind the earlier pieces' (their counts are summed up again by every block), the block's warps one behind the other, and
+// within 32 choices by the rank among the lanes with the same expert. The list is read three times in all, whatever the number of experts:
+// 65536 x 8 choices of 128 / 1024 experts 32 / 67 us, where one launch takes 510 / 733 and the sort took about 300.
+template <typename IT>
+__global__ void __launch_bounds__(256)
+moe_plan_count_kernel(const IT* __restrict__ experts, int n, int per_block, int E, int* __restrict__ hist) {
+  extern __shared__ int s_plan[];  // [E]
+  for (int e = threadIdx.x; e < E; e += 256) s_plan[e] = 0;
+  __syncthreads();
+  const int lo = blockIdx.x * per_block, hi = min(n, lo + per_block);
+  for (int i = lo + threadIdx.x; i < hi; i += 256) {
+    const IT id = experts[i];
+    if (id >= 0 && id < E) atomicAdd(s_plan + static_cast<int>(id), 1);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += 256) hist[static_cast<long long>(blockIdx.x) * E + e] = s_plan[e];
+}
+
+template <typename IT>
+__global__ void __launch_bounds__(256)
+moe_plan_place_kernel(const IT* __restrict__ experts, const int* __restrict__ counts, const int* __restrict__ hist, int n, int per_block, int k,
+                      int E, int tile, int cap, int* __restrict__ slot, int* __restrict__ src, int* __restrict__ seg,
+                      int* __restrict__ tile_expert, int* __restrict__ num_mtiles) {
+  extern __shared__ int s_plan[];
+  int* first = s_plan;          // [E + 1] first row of every expert
+  int* at = s_plan + E + 1;     // [8][E] next row of a warp's choices
+  __shared__ int s_warp[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, blk = blockIdx.x, blocks = gridDim.x;
+  // prefix of the padded counts: thread t holds experts 4t .. 4t + 3
+  int pad[4], sum = 0;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int x = threadIdx.x * 4 + u;
+    pad[u] = x < E ? (max(counts[x], 0) + tile - 1) / tile * tile : 0;
+    sum += pad[u];
+  }
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += v;
+  }
+  if (lane == 31) s_warp[warp] = incl;
+  for (int i = threadIdx.x; i < 8 * E; i += 256) at[i] = 0;
+  __syncthreads();
+  int row = incl - sum;
+  for (int w = 0; w < warp; ++w) row += s_warp[w];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int x = threadIdx.x * 4 + u;
+    if (x <= E) first[x] = row;
+    row += pad[u];
+  }
+  if (threadIdx.x == 255 && E == 1024) first[E] = row;
+  // choices per expert in every warp's share
+  const int per = per_block / 8;  // a multiple of 32
+  const int lo = min(n, blk * per_block + warp * per), hi = min(n, lo + per);
+  int* mine = at + warp * E;
+  for (int i = lo + lane; i < hi; i += 32) {
+    const IT id = experts[i];
+    if (id >= 0 && id < E) atomicAdd(mine + static_cast<int>(id), 1);
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += 256) {
+    int r = first[e];
+#pragma unroll 8
+    for (int c = 0; c < blk; ++c) r += hist[static_cast<long long>(c) * E + e];
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+      const int v = at[w * E + e];
+      at[w * E + e] = r;
+      r += v;
+    }
+  }
+  __syncthreads();
+  for (int i = lo; i < hi; i += 32) {
+    const int x = i + lane;
+    const IT raw = x < hi ? experts[x] : IT(-1);
+    const int id = raw >= 0 && raw < E ? static_cast<int>(raw) : -1;
+    const unsigned int same = __match_any_sync(0xffffffffu, id);
+    int pos = 0;
+    if (id >= 0) pos = mine[id] + __popc(same & ((1u << lane) - 1));
+    __syncwarp();
+    if (id >= 0 && lane == 31 - __clz(same)) mine[id] = pos + 1;
+    __syncwarp();
+    if (x < hi) {
+      // no such expert, or counts that do not belong to the list: nothing behind it may be read or written out of range
+      const bool ok = id >= 0 && pos < min(first[id + 1], cap);
+      slot[x] = ok ? pos : 0;
+      if (ok) src[pos] = x / k;
+    }
+  }
+  // padding rows and tiles: a warp per expert
+  for (int e = blk * 8 + warp; e < E; e += blocks * 8) {
+    int total = 0;
+    for (int c = lane; c < blocks; c += 32) total += hist[static_cast<long long>(c) * E + e];
+    total = __reduce_add_sync(0xffffffffu, total);
+    const int row0 = min(first[e], cap), row1 = min(first[e + 1], cap);
+    for (int i = row0 + min(total, row1 - row0) + lane; i < row1; i += 32) src[i] = -1;
+    for (int i = row0 / tile + lane; i < row1 / tile; i += 32) tile_expert[i] = e;
+  }
+  const int used = first[E];
+  for (int i = used + blk * 256 + threadIdx.x; i < cap; i += blocks * 256) src[i] = -1;
+  for (int i = used / tile + blk * 256 + threadIdx.x; i < cap / tile; i += blocks * 256) tile_expert[i] = E - 1;
+  if (blk == 0) {
+    for (int e = threadIdx.x; e <= E; e += 256) seg[e] = first[e];
+    if (threadIdx.x == 0) *num_mtiles = min(used, cap) / tile;
   }
 }
 
@@ -390,13 +502,41 @@ extern "C" int vb_moe_swiglu(const void* gu, void* out, int rows, int I, const i
   return static_cast<int>(cudaGetLastError());
 }
 
+// Up to here one launch is better: 8192 choices of 64 / 128 / 512 / 1024 experts 8 / 8.3 / 10.8 / 16.5 us against 8 / 9.0 / 15.4 / 24.8 with
+// two; 16384 choices 13 / 13.2 / 17.5 / 27.2 against 8.4 / 9.3 / 13.8 / 22.5.
+constexpr int PLAN_ONE_LAUNCH = 8192;
+// A block per SM, in pieces of at least 1024 choices: every block sums up the counts of all pieces before its own.
+static int plan_per_block(int n) {
+  const int even = (n + num_sms() - 1) / num_sms();
+  return even <= 1024 ? 1024 : (even + 255) / 256 * 256;
+}
+// Blocks of the two-launch form, 0 for one launch.
+extern "C" int vb_moe_plan_blocks(int n) {
+  if (n <= PLAN_ONE_LAUNCH) return 0;
+  return (n + plan_per_block(n) - 1) / plan_per_block(n);
+}
+
 // experts: [n] int64 (wide) or int32; n = tokens * k choices. E <= 1024, cap a multiple of tile that holds every segment.
-extern "C" int vb_moe_plan(const void* experts, int wide, const int* counts, int n, int k, int E, int tile, int cap, int* slot, int* src,
-                           int* seg, int* tile_expert, int* num_mtiles, cudaStream_t s) {
-  if (n <= 0 || k <= 0 || E <= 0 || E > 1024 || tile <= 0 || cap % tile) return -1;
-  if (wide) moe_plan_kernel<long long><<<E, 256, 0, s>>>(reinterpret_cast<const long long*>(experts), counts, n, k, E, tile, cap, slot, src, seg, tile_expert, num_mtiles);
-  else moe_plan_kernel<int><<<E, 256, 0, s>>>(reinterpret_cast<const int*>(experts), counts, n, k, E, tile, cap, slot, src, seg, tile_expert, num_mtiles);
+// hist: vb_moe_plan_blocks(n) * E integers.
+template <typename IT>
+static int moe_plan_launch(const IT* experts, const int* counts, int* hist, int n, int k, int E, int tile, int cap, int* slot, int* src, int* seg,
+                           int* tile_expert, int* num_mtiles, cudaStream_t s) {
+  const int blocks = vb_moe_plan_blocks(n);
+  if (blocks == 0) {
+    moe_plan_kernel<IT><<<E, 256, 0, s>>>(experts, counts, n, k, E, tile, cap, slot, src, seg, tile_expert, num_mtiles);
+  } else {
+    const int per = plan_per_block(n);
+    moe_plan_count_kernel<IT><<<blocks, 256, E * sizeof(int), s>>>(experts, n, per, E, hist);
+    moe_plan_place_kernel<IT><<<blocks, 256, (9 * E + 1) * sizeof(int), s>>>(experts, counts, hist, n, per, k, E, tile, cap, slot, src, seg,
+                                                                           tile_expert, num_mtiles);
+  }
   return static_cast<int>(cudaGetLastError());
+}
+extern "C" int vb_moe_plan(const void* experts, int wide, const int* counts, int* hist, int n, int k, int E, int tile, int cap, int* slot,
+                           int* src, int* seg, int* tile_expert, int* num_mtiles, cudaStream_t s) {
+  if (n <= 0 || k <= 0 || E <= 0 || E > 1024 || tile <= 0 || cap % tile) return -1;
+  return wide ? moe_plan_launch(reinterpret_cast<const long long*>(experts), counts, hist, n, k, E, tile, cap, slot, src, seg, tile_expert, num_mtiles, s)
+              : moe_plan_launch(reinterpret_cast<const int*>(experts), counts, hist, n, k, E, tile, cap, slot, src, seg, tile_expert, num_mtiles, s);
 }
 
 extern "C" int vb_moe_combine(const void* y, long long ldy, const int* slot, const float* w, void* out, long long ldo, int T, int H,
