@@ -404,6 +404,20 @@ def test_column_sums(ops, T, N, ld):
     assert (out - want).abs().max() < 1e-6 * (10 + T)
 
 
+@pytest.mark.parametrize("T,N", [(7900, 4608), (12000, 1152), (40000, 130)])
+def test_column_sums_lose_no_digits_over_many_rows(ops, T, N):
+    """Terms of one sign mostly, as a mean that does not cancel: eight chains of eight and three pairs in fp32 (averaged over the chunks of 64
+    rows), then one rounding (at most 2^-24, its root mean square below half of that)."""
+    from verl_b200.ops import functional as F
+
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x = (torch.randn(T, N, device=DEV, generator=g) * 0.01 + 0.02).bfloat16()
+    out = torch.zeros(N, device=DEV)
+    F.colsum_add_(x, out)
+    want = x.double().sum(0)
+    assert float(((out.double() - want) / want).square().mean().sqrt()) < 2.0**-25
+
+
 # ------------------------------------------------------------------------------------------------ expert products on tiles of tokens
 def _choices(T, k, E, seed, skew=False):
     """Distinct experts per token; with ``skew`` most tokens meet the first ones and some experts stay empty."""

@@ -402,41 +402,62 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict
 
 // ------------------------------------------------------------------------------------------ column sums
 // Gradient of a bias: sums over the rows of a bf16 matrix. A block sums COLSUM_ROWS rows of 512 columns (two neighbouring columns per
-// thread, 128 bytes per warp and row, eight rows in flight) into a plane of partial sums, a second launch folds the planes in order.
-// 7,900 x 4608 in 20 + 12 us; casting to fp32 first and reducing that took 42 + 69 us.
+// thread, 128 bytes per warp and row, eight rows in flight) into a plane of partial sums, a second launch folds the planes in order. A thread's
+// rows go to eight sums that are added pair by pair, and the planes are folded in double: one chain over the rows and one over the planes left
+// errors of 5e-8 to 9e-8 of the sum of magnitudes, where casting to fp32 and reducing that leaves 1.5e-8 to 2e-8; now 1e-8.
+// 7,900 x 4608 in 15 us, 16,000 x 5120 in 44 us; the cast and the reduction took 138 and 290.
 constexpr int COLSUM_ROWS = 64;
+__device__ __forceinline__ float colsum_pairs(const float (&s)[8]) { return ((s[0] + s[1]) + (s[2] + s[3])) + ((s[4] + s[5]) + (s[6] + s[7])); }
 __global__ void __launch_bounds__(256)
 colsum_part_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, int T, int N, float* __restrict__ part) {
   const int c = (blockIdx.x * 256 + threadIdx.x) * 2;
   if (c >= N) return;
   const int t0 = blockIdx.y * COLSUM_ROWS, t1 = min(T, t0 + COLSUM_ROWS);
-  float a = 0.f, b = 0.f;
+  float a[8], b[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) a[u] = b[u] = 0.f;
   const bool pair = c + 1 < N;
-  if (pair && ldx % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0) {
-#pragma unroll 8
-    for (int t = t0; t < t1; ++t) {
-      const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(x + t * ldx + c));
-      a += v.x;
-      b += v.y;
+  const bool vec = pair && ldx % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0;
+  int t = t0;
+  if (vec) {
+    for (; t + 8 <= t1; t += 8) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(x + (t + u) * ldx + c));
+        a[u] += v.x;
+        b[u] += v.y;
+      }
     }
-  } else {
-    for (int t = t0; t < t1; ++t) {
-      a += __bfloat162float(x[t * ldx + c]);
-      if (pair) b += __bfloat162float(x[t * ldx + c + 1]);
+  }
+  for (; t < t1; t += 8) {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      if (t + u < t1) {
+        a[u] += __bfloat162float(x[(t + u) * ldx + c]);
+        if (pair) b[u] += __bfloat162float(x[(t + u) * ldx + c + 1]);
+      }
     }
   }
   float* o = part + static_cast<long long>(blockIdx.y) * N + c;
-  o[0] = a;
-  if (pair) o[1] = b;
+  o[0] = colsum_pairs(a);
+  if (pair) o[1] = colsum_pairs(b);
 }
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
 colsum_fold_kernel(const float* __restrict__ part, int chunks, int N, float* __restrict__ out) {
-  const int c = blockIdx.x * 128 + threadIdx.x;
-  if (c >= N) return;
-  float s = 0.f;
+  __shared__ double fold[8][33];
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31), warp = threadIdx.x >> 5;
+  double s = 0.0;
+  if (c < N) {
 #pragma unroll 8
-  for (int k = 0; k < chunks; ++k) s += part[static_cast<long long>(k) * N + c];
-  out[c] += s;
+    for (int k = warp; k < chunks; k += 8) s += part[static_cast<long long>(k) * N + c];
+  }
+  fold[warp][threadIdx.x & 31] = s;
+  __syncthreads();
+  if (warp != 0 || c >= N) return;
+  s = 0.0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s += fold[k][threadIdx.x];
+  out[c] = static_cast<float>(out[c] + s);
 }
 
 // ------------------------------------------------------------------------------------------ SwiGLU
@@ -709,7 +730,7 @@ int vb_colsum_add(const void* x, long long ldx, int T, int N, float* part, float
   const int chunks = vb_colsum_chunks(T);
   if (chunks > 65535) return -4;
   colsum_part_kernel<<<dim3((N + 511) / 512, chunks), 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), ldx, T, N, part);
-  colsum_fold_kernel<<<(N + 127) / 128, 128, 0, s>>>(part, chunks, N, out);
+  colsum_fold_kernel<<<(N + 31) / 32, 256, 0, s>>>(part, chunks, N, out);
   return static_cast<int>(cudaGetLastError());
 }
 
