@@ -625,6 +625,24 @@ def test_weight_gradient_per_expert_accumulates(ops, M, N):
     assert int(ops.gemm_status()) == 0
 
 
+def test_grouped_products_on_every_device_of_the_process(ops):
+    for d in range(torch.cuda.device_count()):
+        g = torch.Generator().manual_seed(1)
+        seg = torch.tensor([0, 128, 256], dtype=torch.int32, device=f"cuda:{d}")
+        dy, x = torch.randint(-3, 4, (256, 96), generator=g).to(seg.device).bfloat16(), torch.randint(-3, 4, (256, 264), generator=g).to(seg.device).bfloat16()
+        out = torch.ones(2, 96, 264, device=seg.device)
+        ops.gemm_grouped_wgrad_(dy, x, out, seg, True)
+        for e in range(2):
+            part = slice(128 * e, 128 * e + 128)
+            assert torch.equal(out[e].cpu(), 1 + dy[part].float().cpu().T @ x[part].float().cpu())
+        w = torch.randint(-3, 4, (2, 24, 264), generator=g).to(seg.device).bfloat16()
+        te, num = torch.arange(16, dtype=torch.int32, device=seg.device) // 8, torch.tensor([16], dtype=torch.int32, device=seg.device)
+        y = ops.gemm_grouped_tiles(x, w, te, num, 16)
+        for e in range(2):
+            part = slice(128 * e, 128 * e + 128)
+            assert torch.equal(y[part].float().cpu(), (x[part].float().cpu() @ w[e].float().cpu().T).bfloat16().float())
+
+
 # ------------------------------------------------------------------------------------------------ norms
 @pytest.mark.parametrize("T,H", [(1, 8), (3, 248), (5, 264), (639, 264), (1183, 896), (1184, 1024), (640, 1032), (700, 2040), (1185, 2048),
                                  (641, 2056), (9, 3584), (700, 3584), (640, 4096), (640, 4104), (2, 8192), (1300, 3592)])

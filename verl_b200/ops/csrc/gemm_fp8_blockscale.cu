@@ -261,12 +261,9 @@ template <bool FP8, int R>
 static int launch_tile_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const TileGemmParams& p, cudaStream_t stream) {
   using L = TileGemm<FP8, R>;
   auto kern = tile_gemm_kernel<FP8, R>;
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  // on every launch: the attribute belongs to the current device, and a process may use several
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::TOTAL);
+  if (e != cudaSuccess) return static_cast<int>(e);
   const long long items = static_cast<long long>(p.mtiles) * p.ntiles;
   const int sms = num_sms();
   kern<<<static_cast<int>(items < sms ? items : sms), L::THREADS, L::TOTAL, stream>>>(tx, tw, p);

@@ -997,12 +997,9 @@ static int launch_acc(const CUtensorMap& ta, const CUtensorMap& tb, const GemmPa
   auto kern = gemm_bf16_acc_kernel<256, 4>;
   constexpr int smem = GemmSmem<256, 4>::TOTAL_ACC;
   static_assert(smem <= 232448, "shared memory of a CTA");
-  static bool configured = false;
-  if (!configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    configured = true;
-  }
+  // on every launch, as for the other grouped products: the attribute belongs to the current device, and a process may use several
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e != cudaSuccess) return static_cast<int>(e);
   kern<<<static_cast<int>(tiles < sms ? tiles : sms), GEMM_THREADS, smem, stream>>>(ta, tb, td, p);
   return static_cast<int>(cudaGetLastError());
 }
