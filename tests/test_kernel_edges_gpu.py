@@ -571,6 +571,10 @@ def test_few_tokens(ops, M, N, K):
         y = ops.gemm_few_tokens(x, w[:N], b, False).double()
         assert ((y - want).abs() <= want.abs() * 2.0**-8 + size[:, :N] * K * 2.0**-24 + 1e-30).all()
     gu = ops.gemm_few_tokens(x, w, None, False)
+    if M > 16:  # the gated form ends here
+        with pytest.raises(RuntimeError):
+            ops.gemm_few_tokens(x, w, None, True)
+        return
     act = ops.gemm_few_tokens(x, w, None, True)
     want = torch.nn.functional.silu(gu[:, :N].double()) * gu[:, N:].double()
     assert rel(act, want) < 4e-3  # 2^-9 for the result, 2^-9 where another order of the sums rounds a gate or an up value differently

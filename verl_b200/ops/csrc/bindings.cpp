@@ -79,8 +79,8 @@ bool gemm_row_ranges_(const Tensor& a, const Tensor& w, const OptTensor& bias, s
 Tensor gemm_few_tokens(const Tensor& x, const Tensor& w, const OptTensor& bias, bool swiglu) {
   CHECK_BF16(x);
   CHECK_BF16(w);
-  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.stride(1) == 1 && w.stride(1) == 1 && x.size(1) == w.size(1) && x.size(0) <= 64 &&
-              (!swiglu || (w.size(0) % 2 == 0 && !bias.has_value())), "gemm_few_tokens: x [M <= 64, K], w [N, K]");
+  TORCH_CHECK(x.dim() == 2 && w.dim() == 2 && x.stride(1) == 1 && w.stride(1) == 1 && x.size(1) == w.size(1) && x.size(0) <= (swiglu ? 16 : 64) &&
+              (!swiglu || (w.size(0) % 2 == 0 && !bias.has_value())), "gemm_few_tokens: x [M <= 64 (gated: 16), K], w [N, K]");
   const int64_t M = x.size(0), N = swiglu ? w.size(0) / 2 : w.size(0), K = x.size(1);
   if (bias.has_value()) TORCH_CHECK(bias->scalar_type() == at::kBFloat16 && bias->numel() == N && bias->is_contiguous());
   const c10::cuda::CUDAGuard guard(x.device());

@@ -20,6 +20,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "launchers.h"
 #include "tcgen05_common.cuh"
 
@@ -28,7 +30,7 @@ namespace cg = cooperative_groups;
 
 constexpr int FT_WARPS = 8, FT_THREADS = 32 * FT_WARPS;
 constexpr int FT_KB = 64;          // K per block
-constexpr int FT_MAX_TOKENS = 64;
+constexpr int FT_MAX_TOKENS = 64, FT_MAX_GATED = 16;
 
 struct FewTokensParams {
   const __nv_bfloat16* X;
@@ -170,12 +172,7 @@ template <int NT, int MT, bool SWIGLU, int U>
 static cudaError_t launch_few_tokens(const FewTokensParams& p, int tiles, int cl, cudaStream_t stream) {
   auto kern = few_tokens_kernel<NT, MT, SWIGLU, U>;
   constexpr int smem = FT_WARPS * 16 * MT * (8 * NT + 1) * 4;
-  static bool configured = false;
-  if (smem > 48 * 1024 && !configured) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static_assert(smem <= 48 * 1024, "shared memory without an attribute");
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(tiles) * cl);
   cfg.blockDim = dim3(FT_THREADS);
@@ -204,14 +201,14 @@ using namespace vb;
 //   tokens through its L1, which costs as much as the weights.
 extern "C" int vb_few_tokens_better(int M, int N, int K, int swiglu) {
   const long long bytes = 2LL * N * K * (swiglu ? 2 : 1);
-  if (swiglu) return M <= 8 || (M <= 16 && bytes <= (40LL << 20));
+  if (swiglu) return M <= 8 || (M <= FT_MAX_GATED && bytes <= (40LL << 20));
   return (M <= 32 && bytes <= (40LL << 20)) || (M <= FT_MAX_TOKENS && bytes <= (4LL << 20));
 }
 
-// swiglu: N is the width I of the activation, W has 2 I rows. Pointers 16-byte aligned (D: 4), ldx, ldw and K multiples of 8, ldd and N even.
+// swiglu: N is the width I of the activation, W has 2 I rows, M at most 16 (the rule above takes it no further). Pointers 16-byte aligned (D: 4), ldx, ldw and K multiples of 8, ldd and N even.
 extern "C" int vb_gemm_few_tokens(const void* X, const void* W, void* D, const void* bias, int M, int N, int K, long long ldx, long long ldw,
                                   long long ldd, int swiglu, cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || K <= 0 || M > FT_MAX_TOKENS) return -1;
+  if (M <= 0 || N <= 0 || K <= 0 || M > (swiglu ? FT_MAX_GATED : FT_MAX_TOKENS)) return -1;
   if ((K % 8) || (N % 2) || (ldx % 8) || (ldw % 8) || (ldd % 2)) return -1;
   if (((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(W)) & 15) || (reinterpret_cast<uintptr_t>(D) & 3)) return -2;
   FewTokensParams p{};
@@ -225,16 +222,16 @@ extern "C" int vb_gemm_few_tokens(const void* X, const void* W, void* D, const v
   // two CTAs per SM with two blocks per warp in flight, or three with one where that makes it a single wave (5120 x 2048, 32 tokens:
   // 320 CTAs, 12.4 us with two, 10.3 us with three); the gated product has two tiles per warp and takes three throughout
   const int ctas = tiles * cl, sms = num_sms();
-  const bool three = swiglu || (ctas > 2 * sms && ctas <= 3 * sms);
+  const bool three = (ctas > 2 * sms && ctas <= 3 * sms);
   cudaError_t e;
-#define VB_FT(NT)                                                                                                    \
-  e = swiglu  ? launch_few_tokens<NT, 2, true, 1>(p, tiles, cl, stream)                                              \
-      : three ? launch_few_tokens<NT, 1, false, 1>(p, tiles, cl, stream)                                             \
-              : launch_few_tokens<NT, 1, false, 2>(p, tiles, cl, stream)
-  if (M <= 8) VB_FT(1);
-  else if (M <= 16) VB_FT(2);
-  else if (M <= 32) VB_FT(4);
-  else VB_FT(8);
-#undef VB_FT
+  auto plain = [&](auto nt) {
+    constexpr int NT = decltype(nt)::value;
+    return three ? launch_few_tokens<NT, 1, false, 1>(p, tiles, cl, stream) : launch_few_tokens<NT, 1, false, 2>(p, tiles, cl, stream);
+  };
+  if (swiglu) e = M <= 8 ? launch_few_tokens<1, 2, true, 1>(p, tiles, cl, stream) : launch_few_tokens<2, 2, true, 1>(p, tiles, cl, stream);
+  else if (M <= 8) e = plain(std::integral_constant<int, 1>{});
+  else if (M <= 16) e = plain(std::integral_constant<int, 2>{});
+  else if (M <= 32) e = plain(std::integral_constant<int, 4>{});
+  else e = plain(std::integral_constant<int, 8>{});
   return static_cast<int>(e);
 }
