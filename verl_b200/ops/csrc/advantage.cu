@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 namespace vb {
+int num_sms();
 
 // scores[b] = sum_t rewards[b,t]; one block per row. With `stats` (zeroed by the caller) also stats[g] += {sum, sum of squares, count}, in
 // double: sums of fp32 scores and of their squares are then good for a variance far below the square of the mean.
@@ -109,7 +110,7 @@ __device__ __forceinline__ GaeMap gae_shfl_down(const GaeMap& m, int o) {
 }
 
 constexpr int GAE_PER = 4;           // consecutive tokens per thread
-constexpr int GAE_MAX_BLOCKS = 148 * 8;
+constexpr int GAE_BLOCKS_PER_SM = 8;
 
 // A block takes whole rows and walks a row from its end in tiles of blockDim * 4 tokens: every thread composes the maps of its four
 // tokens, a scan over the block gives the state behind them, and the four tokens are then stepped through. 512 x 1024 tokens: 267 us with
@@ -193,7 +194,7 @@ gae_kernel(const float* __restrict__ rewards, const float* __restrict__ values, 
 }
 
 // x <- (x - mean) * rsqrt(var + 1e-8), unbiased variance over the unmasked tokens. Every block folds the partial sums of the scan
-// (at most 1184 x 3) itself, in one order: no memset, no atomics, the same bits every time.
+// (at most eight per SM) itself, in one order: no memset, no atomics, the same bits every time.
 __global__ void __launch_bounds__(256)
 whiten_kernel(float* __restrict__ x, long long n, const double* __restrict__ part, int nparts) {
   __shared__ double red[8][3];
@@ -256,7 +257,7 @@ int vb_grpo_advantage(const float* rewards, const float* mask, const void* group
 
 // Blocks of the scan = rows of `part` (3 doubles each). A row's tiles follow one another, so rows are what fills the machine; a block
 // is as wide as the row needs, up to 256 threads (1024 tokens per tile).
-int vb_gae_blocks(int B) { return B < GAE_MAX_BLOCKS ? B : GAE_MAX_BLOCKS; }
+int vb_gae_blocks(int B) { return B < GAE_BLOCKS_PER_SM * num_sms() ? B : GAE_BLOCKS_PER_SM * num_sms(); }
 
 // Whitening of the advantages over the whole batch (statistics over unmasked tokens, result not re-masked) is applied when `part` is
 // given.
@@ -268,8 +269,9 @@ int vb_gae(const float* rewards, const float* values, const float* mask, int B, 
   gae_kernel<<<vb_gae_blocks(B), threads, 0, s>>>(rewards, values, mask, B, L, gamma, lam, adv, ret, part);
   if (part) {
     const long long n = static_cast<long long>(B) * L;
-    const long long want_blocks = (n + 1023) / 1024;
-    whiten_kernel<<<static_cast<int>(want_blocks < 148 * 4 ? want_blocks : 148 * 4), 256, 0, s>>>(adv, n, part, vb_gae_blocks(B));
+    // a block per 1024 tokens, four per SM at most: every block folds the partial sums
+    const long long want_blocks = (n + 1023) / 1024, most = 4LL * num_sms();
+    whiten_kernel<<<static_cast<int>(want_blocks < most ? want_blocks : most), 256, 0, s>>>(adv, n, part, vb_gae_blocks(B));
   }
   return static_cast<int>(cudaGetLastError());
 }

@@ -216,9 +216,10 @@ extern "C" int vb_gemm_few_tokens(const void* X, const void* W, void* D, const v
   p.bias = reinterpret_cast<const __nv_bfloat16*>(bias); p.D = reinterpret_cast<__nv_bfloat16*>(D);
   p.ldx = ldx; p.ldw = ldw; p.ldd = ldd; p.M = M; p.N = N; p.K = K;
   const int tiles = (N + 15) / 16, nb = (K + FT_KB - 1) / FT_KB;
-  // split K over a cluster while SMs are without a CTA and every warp keeps a block
+  // split K over a cluster while every warp keeps a block and there are fewer than one and a half CTAs per SM: 896 x 4864 at 64 tokens 20.0 ->
+  // 11.9 us with the split; up to two per SM the second CTA's exchange costs more than its loads hide (4608 x 3584 at 32 tokens 11.8 -> 18.2 us)
   int cl = 1;
-  while (cl < 8 && tiles * cl < 222 && nb >= 2 * cl * FT_WARPS) cl *= 2;
+  while (cl < 8 && 2 * tiles * cl < 3 * num_sms() && nb >= 2 * cl * FT_WARPS) cl *= 2;
   // two CTAs per SM with two blocks per warp in flight, or three with one where that makes it a single wave (5120 x 2048, 32 tokens:
   // 320 CTAs, 12.4 us with two, 10.3 us with three); the gated product has two tiles per warp and takes three throughout
   const int ctas = tiles * cl, sms = num_sms();

@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 namespace vb {
+int num_sms();
 
 __device__ __forceinline__ float wsum(float v) {
 #pragma unroll
@@ -742,11 +743,12 @@ int vb_sample(const void* logits, long long ld, int B, int V, int valid_vocab, f
               long long step, long long* tokens, float* logprobs, cudaStream_t s) {
   if (B == 0) return 0;
   if (valid_vocab <= 0 || valid_vocab > V) valid_vocab = V;
-  // 16-byte loads where every row starts on a 16-byte boundary. CTAs per row: as many as have a full turn of logits, up to the portable
-  // cluster size, no more than about two waves of the chip need (148 SMs x 4 CTAs).
+  // 16-byte loads where every row starts on a 16-byte boundary. CTAs per row: doubled up to the portable cluster size while every CTA has a
+  // full turn of logits and the launch less than 16 CTAs per SM. (An SM holds six: at most 32 per SM come out of it, so that many rows still
+  // end together, and 320 rows of 152064 get eight CTAs each.)
   const bool vec = reinterpret_cast<uintptr_t>(logits) % 16 == 0 && ld % 8 == 0;
   int parts = 1;
-  while (parts < 8 && parts * SAMPLE_THREADS * 8 < valid_vocab && static_cast<long long>(B) * parts < 148 * 16) parts *= 2;
+  while (parts < 8 && parts * SAMPLE_THREADS * 8 < valid_vocab && static_cast<long long>(B) * parts < 16LL * num_sms()) parts *= 2;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(B) * parts);
   cfg.blockDim = dim3(SAMPLE_THREADS);
