@@ -39,6 +39,7 @@
 // that case 470 -> 295 us, two prompts with five continuations each (7,900 tokens, 28 / 4 heads of 128) 984 -> 800, 5 x 3072 1862 -> 1614,
 // 8192 2491 -> 1983 us. A step of 64 queries still takes 2.5 us of which the tensor pipe works 1.1: S^T / dP^T of the next step, the
 // softmax and the products of this one follow each other, and TMEM (512 columns at head_dim 128) has no room for a second S^T / dP^T.
+// dQ, and dK / dV where several CTAs add to them, are summed in an order that varies from run to run; full determinism takes the autograd form.
 //
 // With `parent` (see attention_fwd_tcgen05.cu) a key block of a prompt has queries in several sequences. They are dealt to one CTA per
 // (key block, query sequence): blockIdx.y = s is sequence s against its own keys, num_seqs + s is sequence s against those of parent[s],

@@ -565,7 +565,8 @@ __device__ __forceinline__ void adamw_one(float& p, float g, float& m, float& v,
   p -= (a.lr / a.bc1) * (m / denom);
 }
 // 30 bytes an element. VEC: 4 elements a thread in 16-byte accesses (every pointer 16-byte aligned, the bf16 copy 8; the remainder of n
-// goes to the last threads one by one): 2^28 elements in 1.18 ms (6.8 TB/s) instead of 1386 us with 4-byte accesses (5.8 TB/s).
+// goes to the last threads one by one): 2^28 elements back to back 1163 us (6.9 TB/s, a little above a plain copy's 6.5) instead of 1337 us with
+// 4-byte accesses (6.0 TB/s).
 template <bool VEC>
 __global__ void __launch_bounds__(256)
 adamw_kernel(float* __restrict__ master, float* __restrict__ grad, float* __restrict__ m, float* __restrict__ v,

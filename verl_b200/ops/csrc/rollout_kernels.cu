@@ -143,7 +143,7 @@ qk_norm_rope_kernel(__nv_bfloat16* __restrict__ qkv, long long ld, const int* __
 #pragma unroll
   for (int j = 0; j < 8; j += 2) {
     const float2 c = *reinterpret_cast<const float2*>(cos_t + tab + j), sn = *reinterpret_cast<const float2*>(sin_t + tab + j);
-    // a c - b s with the second product rounded, b c + a s with the first one: what the rotation kernel's expressions compile to
+    // a c - b s with the second product rounded, b c + a s with the first one: the bits of the separate kernels, to which a test holds it
     reinterpret_cast<__nv_bfloat162*>(&out)[j >> 1] =
         low ? __floats2bfloat162_rn(__fmaf_rn(f[j], c.x, -__fmul_rn(o[j], sn.x)), __fmaf_rn(f[j + 1], c.y, -__fmul_rn(o[j + 1], sn.y)))
             : __floats2bfloat162_rn(__fmaf_rn(o[j], sn.x, __fmul_rn(f[j], c.x)), __fmaf_rn(o[j + 1], sn.y, __fmul_rn(f[j + 1], c.y)));

@@ -19,16 +19,17 @@ __all__ = ["enable_full_determinism", "pad_packed_inputs", "prepare_micro_batche
 
 
 def enable_full_determinism(seed: int) -> None:
-    """Seeds every generator and switches the libraries to their deterministic code paths. The native kernels have no
-    atomically-accumulated outputs on the default training path (wgrad accumulates in a fixed K order, the MoE combine and
-    the fused collectives sum in rank order), so this is sufficient for run-to-run identical losses."""
+    """Seeds every generator and switches the libraries to their deterministic code paths. Two native training kernels sum in an order
+    that varies, the attention backward (dQ, and dK / dV where several thread blocks add to them) and the embedding's gradient: an
+    autograd form and an ordered one take their place. Weight gradients accumulate in a fixed K order (one addition per element and
+    call), the MoE combine and the fused collectives sum in rank order, so losses are identical from run to run."""
     random.seed(seed)
     np.random.seed(seed)
     torch.manual_seed(seed)
     if torch.cuda.is_available():
         torch.cuda.manual_seed_all(seed)
     os.environ.setdefault("CUBLAS_WORKSPACE_CONFIG", ":4096:8")
-    os.environ["VERL_B200_NATIVE_ATTN_BWD"] = "0"  # the tcgen05 attention backward reduces dQ with fp32 atomics
+    os.environ["VERL_B200_NATIVE_ATTN_BWD"] = "0"  # the tcgen05 attention backward adds in a varying order
     from ...ops import functional as _F
 
     _F._ATTN_IMPL["bwd"] = None                    # also when the kernels were selected before this call
